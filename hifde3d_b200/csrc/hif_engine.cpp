@@ -368,6 +368,9 @@ struct Arena {
   };
   Mark mark() const { return Mark{cur, chunks.empty() ? 0 : chunks[cur].used}; }
   void rewind(const Mark& m) {
+    size_t u = 0;  // the temporaries count towards what consolidate() asks for
+    for (const Chunk& c : chunks) u += c.used;
+    hw_cycle = std::max(hw_cycle, u);
     for (size_t q = m.cur + 1; q < chunks.size(); ++q) chunks[q].used = 0;
     if (!chunks.empty()) chunks[m.cur].used = m.used;
     cur = m.cur;
@@ -2543,82 +2546,41 @@ class Engine {
       }
     }
     int* d_ord = orders.empty() ? nullptr : tmp.add(upload(orders, stream));
-    // Tall faces are first reduced to their triangular factor R0 (n x n) by an
-    // unpivoted blocked Householder QR; the pivoted QR of R0 makes the same
-    // pivot choices and yields the same R as that of M in exact arithmetic
-    // (both depend on M only through M^T M = R0^T R0).
-    std::vector<double*> idM(nf);
-    std::vector<int> idm(nf);
-    for (int f = 0; f < nf; ++f) {
-      idM[f] = dM + o_M[f];
-      idm[f] = rows_l[f].size();
-    }
-    // mixed precision: tall faces go to the pivoted Cholesky ID instead (no
-    // compression; replayed pivot orders keep the QR path). The Gram matrix
-    // M^T M resolves a column's remaining norm only down to about sqrt(u) ||M||
-    // = 1.5e-8 ||M||, so the rank test R_ii <= eps R_00 needs eps well above
-    // that: below kGramMinEps the faces take the FP64 pivoted QR as in FP64 mode.
+    // mixed precision: tall faces go to the pivoted Cholesky ID instead (replayed
+    // pivot orders keep the QR path). The Gram matrix M^T M resolves a column's
+    // remaining norm only down to about sqrt(u) ||M|| = 1.5e-8 ||M||, so the rank
+    // test R_ii <= eps R_00 needs eps well above that: below kGramMinEps the
+    // faces take the FP64 pivoted QR as in FP64 mode.
     const bool chol = precision == HIF_PRECISION_MIXED && d_ord == nullptr && eps >= kGramMinEps;
-    if (!chol) compress_faces(blocks, rows_l, dM, o_M, idM, idm, tmp);
-    mark("skel row compression", level);
     std::vector<IdDesc> idd(nf);
     for (int f = 0; f < nf; ++f) {
       IdDesc& d = idd[f];
-      d.M = idM[f];
+      d.M = dM + o_M[f];
       d.order = d_ord ? d_ord + o_ord[f] : nullptr;
       d.jpvt = d_jp + o_i[f];
       d.rdiag = d_rd + o_i[f];
       d.keep = d_keep + o_i[f];
       d.rank = d_rank + f;
       d.W = dWs + o_W[f];
-      d.m = idm[f];
+      d.m = rows_l[f].size();
       d.n = blocks[f].global.size();
     }
-    // small faces: one CTA each (k_id); compressed faces: grouped ID, several
-    // CTAs per face for the largest ones
-    std::vector<IdDesc> small_id, chol_id;
-    std::vector<IdGroupDesc> g1, gbig;
-    int small_n = 0, g1_m = 0, g1_n = 0, big_m = 0, big_n = 0;
+    // small faces: one CTA each (k_id); tall wide ones: the pivoted QR by phases
+    std::vector<IdDesc> small_id, chol_id, wide_id;
+    std::vector<int> wide_f;
+    int small_n = 0;
     for (int f = 0; f < nf; ++f) {
-      const bool compressed = idM[f] != dM + o_M[f];
       const int n = idd[f].n;
       if (chol && n > gram_min_n && idd[f].m > n) {
         chol_id.push_back(idd[f]);
-        continue;
-      }
-      if (!compressed) {
+      } else if (!chol && n > kCompressMinN && idd[f].m > n) {
+        wide_id.push_back(idd[f]);
+        wide_f.push_back(f);
+      } else {
         small_id.push_back(idd[f]);
         small_n = std::max(small_n, n);
-        continue;
-      }
-      IdGroupDesc gd{};
-      gd.id = idd[f];
-      (n >= kGroupMinN ? gbig : g1).push_back(gd);
-      if (n >= kGroupMinN) {
-        big_m = std::max(big_m, idd[f].m);
-        big_n = std::max(big_n, n);
-      } else {
-        g1_m = std::max(g1_m, idd[f].m);
-        g1_n = std::max(g1_n, n);
       }
     }
-    const int group = gbig.empty() ? 1 : std::max(1, std::min(16, 148 / (int)gbig.size()));
-    auto scratch_for = [&](std::vector<IdGroupDesc>& v, int grp) {
-      long long nd = 0, ni = 0;
-      for (const IdGroupDesc& g : v) nd += 2LL * g.id.n + grp + 2;
-      ni = 64LL * v.size();
-      double* dsc = tmp.add(dalloc<double>(nd, stream));
-      int* isc = tmp.add(dalloc<int>(ni, stream));
-      HIF_CK(cudaMemsetAsync(isc, 0, ni * sizeof(int), stream));
-      long long od = 0;
-      for (size_t q = 0; q < v.size(); ++q) {
-        v[q].norms = dsc + od;
-        v[q].cand = dsc + od + 2LL * v[q].id.n;
-        v[q].tau = dsc + od + 2LL * v[q].id.n + grp;
-        od += 2LL * v[q].id.n + grp + 2;
-        v[q].sync = isc + 64 * q;
-      }
-    };
     double idfl = 0;
     for (const IdDesc& d : idd) idfl += 4.0 * d.m * d.n * d.n - 4.0 / 3.0 * d.n * d.n * (double)d.n;
     if (!small_id.empty()) {
@@ -2631,20 +2593,18 @@ class Engine {
       idfl = 0;
     }
     if (!chol_id.empty()) id_cholesky(chol_id, tmp);
-    for (int pass = 0; pass < 2; ++pass) {
-      std::vector<IdGroupDesc>& v = pass == 0 ? g1 : gbig;
-      if (v.empty()) continue;
-      const int grp = pass == 0 ? 1 : group;
-      scratch_for(v, grp);
-      IdGroupDesc* dg = tmp.add(upload(v, stream));
-      cudaError_t le = cudaSuccess;
-      timed(HIF_KCLASS_ID, idfl, 0, [&] {
-        le = launch_id_group(dg, (int)v.size(), grp, eps, d_status, stream,
-                             pass == 0 ? g1_m : big_m, pass == 0 ? g1_n : big_n);
-      });
-      idfl = 0;
-      if (le != cudaSuccess)
-        throw Error{HIF_ERR_CUDA, std::string("grouped ID launch: ") + cudaGetErrorString(le)};
+    // by phases, unless the order is prescribed or the grouped QR was asked for:
+    // n = 128 FP64, the three wide levels 758 ms column by column, 325 ms by
+    // phases; n = 32, 12 faces of 225 columns, 11.0 ms against 4.6 ms
+    if (!wide_id.empty() && (d_ord || group_asked)) {
+      id_householder(wide_id, tmp);
+    } else if (!wide_id.empty() && !id_phases(wide_id, tmp)) {
+      // a face the phases do not take: the wide faces are assembled again and all
+      // of them decomposed column by column
+      std::vector<GatherTarget> tw;
+      for (int f : wide_f) tw.push_back(tg[f]);
+      gather(tw, cells, d_own, d_sd, d_dof, tmp);
+      id_householder(wide_id, tmp);
     }
     HIF_CK(cudaGetLastError());
     // pivots, kept flags and |R_ii| read back into pinned staging: the copies
@@ -2926,26 +2886,300 @@ class Engine {
     sync();
     timed(HIF_KCLASS_ID, 0, 0, [&] { launch_pchol_finish(dpd, nd, max_n, stream); });
     HIF_CK(cudaGetLastError());
-    // W := R11^{-1} R12, diagonal blocks from the bottom, products above them
+    std::vector<TriSolve> ts;
+    for (int q = 0; q < nd; ++q) ts.push_back(TriSolve{pd[q].G, v[q].W, info[2 * q], v[q].n});
+    solve_w(ts, tmp);
+  }
+
+  // Column-pivoted QR of wide tall faces by phases (see PqrDesc). Per phase: the
+  // Gram matrices of what is left, pivoted Cholesky panels on them, one read-back of
+  // the pivot counts (they set the shapes of the phase's products), then the
+  // products. Returns false, with the faces' M overwritten, when a face is outside
+  // what the scheme holds for: |E| above kPqrMaxE (picked columns far worse
+  // conditioned than their pivots), kept columns that are not a prefix of the
+  // order, or more than kPqrMaxPhases phases (norms spread over hundreds of
+  // decades).
+  static constexpr int kPqrMaxPhases = 40;
+  bool id_phases(const std::vector<IdDesc>& v, BufList& tmp) {
+    Arena& work = *cur_work;
+    const Arena::Mark mk = work.mark();
+    const int nd = (int)v.size();
+    struct Face {
+      long long g = 0, s = 0, z = 0, q = 0, i = 0;  // offsets of its buffers
+      int o = 0;                                     // columns already picked
+    };
+    std::vector<Face> fc(nd);
+    long long gsz = 0, ssz = 0, zsz = 0, qsz = 0, isz = 0;
+    int max_m = 0, max_n = 0;
+    for (int f = 0; f < nd; ++f) {
+      const IdDesc& d = v[f];
+      const long long cap = std::min(kPqrCap, d.n);
+      fc[f].g = gsz;
+      gsz += (long long)d.n * d.n;
+      fc[f].s = ssz;
+      ssz += d.m * cap;
+      fc[f].z = zsz;
+      zsz += cap * d.n;
+      fc[f].q = qsz;
+      qsz += cap * cap;
+      fc[f].i = isz;
+      isz += d.n;
+      max_m = std::max(max_m, d.m);
+      max_n = std::max(max_n, d.n);
+    }
+    double* G = work.alloc<double>(gsz);
+    double* Rr = work.alloc<double>(gsz);
+    double* S = work.alloc<double>(ssz);
+    double* Z = work.alloc<double>(zsz);
+    double* Rsel = work.alloc<double>(zsz);
+    double* R1 = work.alloc<double>(qsz);
+    double* R1i = work.alloc<double>(qsz);
+    double* d0 = work.alloc<double>(nd);
+    int* chosen = work.alloc<int>(isz);
+    int* piv = work.alloc<int>(isz);
+    int* perm = work.alloc<int>(isz);
+    int* info = work.alloc<int>(2LL * nd + 1);  // steps, done flag per face; *flag last
+    int* flag = info + 2LL * nd;
+    HIF_CK(cudaMemsetAsync(flag, 0, sizeof(int), stream));
+    int* h_perm = static_cast<int*>(stage.get(isz * sizeof(int)));
+    for (int f = 0; f < nd; ++f)
+      for (int j = 0; j < v[f].n; ++j) h_perm[fc[f].i + j] = j;
+    HIF_CK(cudaMemcpyAsync(perm, h_perm, isz * sizeof(int), cudaMemcpyHostToDevice, stream));
+    int* h_info = static_cast<int*>(stage.get((2LL * nd + 1) * sizeof(int)));
+    auto tm = [&](int cls, double fl, double by, auto&& f, int n) { timed(cls, fl, by, f, n); };
+    std::vector<int> act(nd);
+    for (int f = 0; f < nd; ++f) act[f] = f;
+    bool ok = true;
+    for (int phase = 0; !act.empty() && ok; ++phase) {
+      if (phase == kPqrMaxPhases) {
+        ok = false;
+        break;
+      }
+      BufList step;
+      const int na = (int)act.size();
+      std::vector<PcholDesc> pd(na);
+      std::vector<GemmDesc> gram;
+      std::vector<int> ids(na);
+      int max_w = 0;
+      for (int q = 0; q < na; ++q) {
+        const IdDesc& d = v[act[q]];
+        const Face& c = fc[act[q]];
+        const int w = d.n - c.o;
+        max_w = std::max(max_w, w);
+        PcholDesc& p = pd[q];
+        p.G = G + c.g;
+        p.R = Rsel + c.z;
+        p.chosen = chosen + c.i;
+        p.piv = piv + c.i;
+        p.info = info + 2 * q;
+        p.d0 = d0 + q;
+        p.id = d;
+        p.id.n = w;
+        GemmDesc g{};
+        g.C = p.G;
+        g.ldc = w;
+        g.A = g.B = d.M + (long long)c.o * d.m;
+        g.lda = g.ldb = d.m;
+        g.m = g.n = w;
+        g.k = d.m;
+        g.transA = 1;
+        g.alpha = 1.0;
+        g.lower = 1;
+        gram.push_back(g);
+        ids[q] = q;
+      }
+      HIF_CK(cudaMemsetAsync(info, 0, 2LL * na * sizeof(int), stream));
+      gemm_batch(gram, step, stream, HIF_KCLASS_QR, tm, 128);
+      PcholDesc* dpd = step.add(upload(pd, stream));
+      for (int i0 = 0; i0 < std::min(max_w, kPqrCap); i0 += kPcholNB) {
+        std::vector<int> on;
+        std::vector<GemmDesc> upd;
+        for (int q = 0; q < na; ++q) {
+          const int w = pd[q].id.n;
+          if (w <= i0) continue;
+          on.push_back(q);
+          if (w <= i0 + kPcholNB || i0 + kPcholNB >= kPqrCap) continue;
+          GemmDesc g{};
+          g.C = pd[q].G;
+          g.ldc = w;
+          g.A = g.B = pd[q].R + (long long)i0 * w;
+          g.lda = g.ldb = w;
+          g.transB = 1;
+          g.m = g.n = w;
+          g.k = kPcholNB;
+          g.alpha = -1.0;
+          g.beta = 1.0;
+          g.lower = 1;
+          g.skip = pd[q].info + 1;
+          upd.push_back(g);
+        }
+        int* da = step.add(upload(on, stream));
+        timed(HIF_KCLASS_ID, 0, 0, [&] {
+          launch_pchol_panel(dpd, da, (int)on.size(), i0, kPcholNB, kPqrDrop, max_w, d_status,
+                             stream);
+        });
+        HIF_CK(cudaGetLastError());
+        gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm, 128);
+      }
+      HIF_CK(cudaMemcpyAsync(h_info, info, 2LL * na * sizeof(int), cudaMemcpyDeviceToHost, stream));
+      HIF_CK(cudaMemcpyAsync(h_info + 2LL * nd, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+      sync();
+      if (h_info[2LL * nd]) {
+        ok = false;
+        step.release(stream);
+        break;
+      }
+      std::vector<PqrDesc> qd;
+      std::vector<GemmDesc> gq, gz, gu;
+      std::vector<int> next;
+      int mk_ = 0, mc = 0, mm = 0;
+      for (int q = 0; q < na; ++q) {
+        const IdDesc& d = v[act[q]];
+        Face& c = fc[act[q]];
+        const int k = h_info[2 * q], w = d.n - c.o;
+        if (k == 0) {
+          // nothing of the face is left: rows of zeros, the columns in their order
+          HIF_CK(cudaMemsetAsync(Rr + c.g + (long long)c.o * d.n, 0,
+                                 (size_t)w * d.n * sizeof(double), stream));
+          c.o = d.n;
+          continue;
+        }
+        PqrDesc p{};
+        p.T = d.M;
+        p.S = S + c.s;
+        p.R1 = R1 + c.q;
+        p.R1inv = R1i + c.q;
+        p.Z = Z + c.z;
+        p.Rr = Rr + c.g;
+        p.perm = perm + c.i;
+        p.Rsel = pd[q].R;
+        p.piv = pd[q].piv;
+        p.m = d.m;
+        p.n = d.n;
+        p.o = c.o;
+        p.k = k;
+        qd.push_back(p);
+        mk_ = std::max(mk_, k);
+        mc = std::max(mc, w);
+        mm = std::max(mm, d.m);
+        double* To = d.M + (long long)c.o * d.m;
+        GemmDesc a{};  // Q1 = S R1^{-1}, over the picked columns' place in T
+        a.C = To;
+        a.ldc = d.m;
+        a.A = p.S;
+        a.lda = d.m;
+        a.B = p.R1inv;
+        a.ldb = k;
+        a.m = d.m;
+        a.n = k;
+        a.k = k;
+        a.alpha = 1.0;
+        gq.push_back(a);
+        GemmDesc z{};  // Z = Q1^T [Q1 | T]
+        z.C = p.Z;
+        z.ldc = k;
+        z.A = z.B = To;
+        z.lda = z.ldb = d.m;
+        z.transA = 1;
+        z.m = k;
+        z.n = w;
+        z.k = d.m;
+        z.alpha = 1.0;
+        gz.push_back(z);
+        if (w > k) {
+          GemmDesc u{};  // T -= Q1 D
+          u.C = To + (long long)k * d.m;
+          u.ldc = d.m;
+          u.A = To;
+          u.lda = d.m;
+          u.B = p.Z + (long long)k * k;
+          u.ldb = k;
+          u.m = d.m;
+          u.n = w - k;
+          u.k = k;
+          u.alpha = -1.0;
+          u.beta = 1.0;
+          gu.push_back(u);
+          next.push_back(act[q]);
+        }
+        c.o += k;
+      }
+      if (!qd.empty()) {
+        PqrDesc* dq = step.add(upload(qd, stream));
+        const int nq = (int)qd.size();
+        timed(HIF_KCLASS_QR, 0, 0, [&] {
+          launch_pqr_extract(dq, nq, mm, stream);
+          launch_pqr_trinv(dq, nq, mk_, stream);
+        }, 2);
+        HIF_CK(cudaGetLastError());
+        gemm_batch(gq, step, stream, HIF_KCLASS_QR, tm);
+        gemm_batch(gz, step, stream, HIF_KCLASS_QR, tm);
+        timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mc, flag, stream); }, 1);
+        HIF_CK(cudaGetLastError());
+        gemm_batch(gu, step, stream, HIF_KCLASS_QR, tm);
+      }
+      act.swap(next);
+      step.release(stream);
+    }
+    if (ok) {
+      std::vector<PqrOut> po(nd);
+      for (int f = 0; f < nd; ++f)
+        po[f] = PqrOut{Rr + fc[f].g, perm + fc[f].i, G + fc[f].g, v[f]};
+      PqrOut* dpo = tmp.add(upload(po, stream));
+      timed(HIF_KCLASS_ID, 0, 0, [&] {
+        launch_pqr_finish(dpo, nd, eps, max_n, flag, d_status, stream);
+      });
+      HIF_CK(cudaGetLastError());
+      // ranks of consecutive faces lie side by side: one copy per run of them
+      int* h_rank = static_cast<int*>(stage.get((nd + 1) * sizeof(int)));
+      for (int f = 0; f < nd;) {
+        int e = f + 1;
+        while (e < nd && v[e].rank == v[e - 1].rank + 1) ++e;
+        HIF_CK(cudaMemcpyAsync(h_rank + f, v[f].rank, (e - f) * sizeof(int),
+                               cudaMemcpyDeviceToHost, stream));
+        f = e;
+      }
+      HIF_CK(cudaMemcpyAsync(h_rank + nd, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+      sync();
+      ok = h_rank[nd] == 0;
+      if (ok) {
+        std::vector<TriSolve> ts;
+        for (int f = 0; f < nd; ++f) ts.push_back(TriSolve{G + fc[f].g, v[f].W, h_rank[f], v[f].n});
+        solve_w(ts, tmp);
+      }
+    }
+    work.rewind(mk);
+    return ok;
+  }
+
+  // W := R11^{-1} R12 of every face (R11 k x k, ld k; W k x (n - k), ld k): diagonal
+  // blocks from the bottom, products above them.
+  struct TriSolve {
+    const double* R11;
+    double* W;
+    int k, n;
+  };
+  void solve_w(const std::vector<TriSolve>& v, BufList& tmp) {
+    auto tm = [&](int cls, double fl, double by, auto&& f, int n) { timed(cls, fl, by, f, n); };
     int kmax = 0;
-    for (int q = 0; q < nd; ++q) kmax = std::max(kmax, info[2 * q]);
+    for (const TriSolve& t : v) kmax = std::max(kmax, t.k);
     for (int b = 0; b * kTrsmNB < kmax; ++b) {
       std::vector<TrsmBlockDesc> tb;
       std::vector<GemmDesc> up;
       int maxc = 0;
-      for (int q = 0; q < nd; ++q) {
-        const int k = info[2 * q], nc = pd[q].id.n - k;
+      for (const TriSolve& t : v) {
+        const int k = t.k, nc = t.n - k;
         const int a1 = k - b * kTrsmNB, a0 = std::max(0, a1 - kTrsmNB);
         if (a1 <= 0 || nc <= 0) continue;
-        tb.push_back(TrsmBlockDesc{pd[q].G, pd[q].id.W, k, nc, a0, a1});
+        tb.push_back(TrsmBlockDesc{t.R11, t.W, k, nc, a0, a1});
         maxc = std::max(maxc, nc);
         if (a0 > 0) {
           GemmDesc g{};
-          g.C = pd[q].id.W;
+          g.C = t.W;
           g.ldc = k;
-          g.A = pd[q].G + (long long)a0 * k;
+          g.A = t.R11 + (long long)a0 * k;
           g.lda = k;
-          g.B = pd[q].id.W + a0;
+          g.B = t.W + a0;
           g.ldb = k;
           g.m = a0;
           g.n = nc;
@@ -2965,34 +3199,80 @@ class Engine {
     }
   }
 
-  // Blocked Householder row compression of the faces with more than
-  // kCompressMinN columns: on return idM[f] / idm[f] point at R0 (n x n, ld n).
-  // Two levels of blocking: kQrNB2-column outer panels, each factored by
-  // kQrNB-column sub-panels that update only the rest of the outer panel; the
-  // columns right of the outer panel get one compact-WY update with all of its
-  // kQrNB2 reflectors (T from V^T V).
-  static constexpr int kCompressMinN = 64;
-  int kGroupMinN = 512;  // faces this wide get a CTA group (HIF_OPT_ID_GROUP_MIN_N)
-  void compress_faces(const std::vector<BlockInfo>& blocks,
-                      const std::vector<std::vector<int>>& rows_l, double* dM,
-                      const std::vector<long long>& o_M, std::vector<double*>& idM,
-                      std::vector<int>& idm, BufList& tmp) {
-    std::vector<int> list;
-    long long vsz = 0, wsz = 0, rsz = 0;
-    int maxn = 0;
-    for (size_t f = 0; f < blocks.size(); ++f) {
-      const int n = blocks[f].global.size(), m = rows_l[f].size();
-      if (n > kCompressMinN && m > n) {
-        list.push_back(f);
-        vsz += (long long)m * kQrNB2;
-        wsz += (long long)kQrNB2 * n;
-        rsz += (long long)n * n;
-        maxn = std::max(maxn, n);
+  // Column-by-column pivoted QR of wide tall faces, for replayed pivot orders, for
+  // faces the phases do not take and where HIF_OPT_ID_GROUP_MIN_N was set: row compression to R0 (n x n), whose pivoted
+  // QR makes the same pivot choices and yields the same R as that of M in exact
+  // arithmetic (both depend on M only through M^T M = R0^T R0); several CTAs per
+  // face for the widest.
+  void id_householder(std::vector<IdDesc>& v, BufList& tmp) {
+    compress_faces(v, tmp);
+    mark("skel row compression", -1);
+    std::vector<IdGroupDesc> g1, gbig;
+    int g1_m = 0, g1_n = 0, big_m = 0, big_n = 0;
+    for (const IdDesc& d : v) {
+      IdGroupDesc gd{};
+      gd.id = d;
+      (d.n >= kGroupMinN ? gbig : g1).push_back(gd);
+      if (d.n >= kGroupMinN) {
+        big_m = std::max(big_m, d.m);
+        big_n = std::max(big_n, d.n);
+      } else {
+        g1_m = std::max(g1_m, d.m);
+        g1_n = std::max(g1_n, d.n);
       }
     }
-    if (list.empty()) return;
+    const int group = gbig.empty() ? 1 : std::max(1, std::min(16, 148 / (int)gbig.size()));
+    auto scratch_for = [&](std::vector<IdGroupDesc>& w, int grp) {
+      long long nd = 0, ni = 0;
+      for (const IdGroupDesc& g : w) nd += 2LL * g.id.n + grp + 2;
+      ni = 64LL * w.size();
+      double* dsc = tmp.add(dalloc<double>(nd, stream));
+      int* isc = tmp.add(dalloc<int>(ni, stream));
+      HIF_CK(cudaMemsetAsync(isc, 0, ni * sizeof(int), stream));
+      long long od = 0;
+      for (size_t q = 0; q < w.size(); ++q) {
+        w[q].norms = dsc + od;
+        w[q].cand = dsc + od + 2LL * w[q].id.n;
+        w[q].tau = dsc + od + 2LL * w[q].id.n + grp;
+        od += 2LL * w[q].id.n + grp + 2;
+        w[q].sync = isc + 64 * q;
+      }
+    };
+    for (int pass = 0; pass < 2; ++pass) {
+      std::vector<IdGroupDesc>& w = pass == 0 ? g1 : gbig;
+      if (w.empty()) continue;
+      const int grp = pass == 0 ? 1 : group;
+      scratch_for(w, grp);
+      IdGroupDesc* dg = tmp.add(upload(w, stream));
+      cudaError_t le = cudaSuccess;
+      timed(HIF_KCLASS_ID, 0, 0, [&] {
+        le = launch_id_group(dg, (int)w.size(), grp, eps, d_status, stream,
+                             pass == 0 ? g1_m : big_m, pass == 0 ? g1_n : big_n);
+      });
+      if (le != cudaSuccess)
+        throw Error{HIF_ERR_CUDA, std::string("grouped ID launch: ") + cudaGetErrorString(le)};
+    }
+  }
+
+  // Blocked Householder row compression: on return a face's M / m point at R0
+  // (n x n, ld n). Two levels of blocking: kQrNB2-column outer panels, each
+  // factored by kQrNB-column sub-panels that update only the rest of the outer
+  // panel; the columns right of the outer panel get one compact-WY update with all
+  // of its kQrNB2 reflectors (T from V^T V).
+  static constexpr int kCompressMinN = 64;  // wider faces (and m > n) are "wide"
+  int kGroupMinN = 512;  // faces this wide get a CTA group (HIF_OPT_ID_GROUP_MIN_N)
+  bool group_asked = false;  // that option was set: wide faces column by column
+  void compress_faces(std::vector<IdDesc>& v, BufList& tmp) {
+    long long vsz = 0, wsz = 0, rsz = 0;
+    int maxn = 0;
+    for (const IdDesc& d : v) {
+      vsz += (long long)d.m * kQrNB2;
+      wsz += (long long)kQrNB2 * d.n;
+      rsz += (long long)d.n * d.n;
+      maxn = std::max(maxn, d.n);
+    }
     Arena& work = *cur_work;
-    const size_t nl = list.size();
+    const size_t nl = v.size();
     double* V = work.alloc<double>(vsz);
     double* Tm = work.alloc<double>(nl * kQrNB * kQrNB);
     double* T2 = work.alloc<double>(nl * kQrNB2 * kQrNB2);
@@ -3005,9 +3285,8 @@ class Engine {
     std::vector<long long> o_w, o_r;
     long long ov = 0, ow = 0, orr = 0;
     for (size_t q = 0; q < nl; ++q) {
-      const int f = list[q];
-      const int n = blocks[f].global.size(), m = rows_l[f].size();
-      qd.push_back(QrDesc{dM + o_M[f], V + ov, Tm + (long long)q * kQrNB * kQrNB,
+      const int n = v[q].n, m = v[q].m;
+      qd.push_back(QrDesc{v[q].M, V + ov, Tm + (long long)q * kQrNB * kQrNB,
                           tau + (long long)q * kQrNB2, m, n});
       o_w.push_back(ow);
       o_r.push_back(orr);
@@ -3160,10 +3439,10 @@ class Engine {
     }
     std::vector<TriuDesc> td;
     for (size_t q = 0; q < qd.size(); ++q) {
-      const int f = list[q], n = qd[q].n;
+      const int n = qd[q].n;
       td.push_back(TriuDesc{qd[q].M, R0 + o_r[q], qd[q].m, n, n});
-      idM[f] = R0 + o_r[q];
-      idm[f] = n;
+      v[q].M = R0 + o_r[q];
+      v[q].m = n;
     }
     TriuDesc* dtd = tmp.add(upload(td, stream));
     timed(HIF_KCLASS_QR, 0, 0, [&] { launch_triu(dtd, (int)td.size(), stream); });
@@ -4335,6 +4614,7 @@ int hif_set_option(hif_handle h, int option, long long value) {
     case HIF_OPT_ID_GROUP_MIN_N:
       if (value < 2) return HIF_ERR_ARG;
       h->e->kGroupMinN = (int)value;
+      h->e->group_asked = true;
       return HIF_OK;
     case HIF_OPT_PROFILE:
       return guarded([&] {

@@ -3114,6 +3114,275 @@ void launch_trsm_block(const TrsmBlockDesc* d_desc, int nd, int max_cols, cudaSt
 }
 
 // ===========================================================================
+// Column-pivoted QR of tall faces by phases (see PqrDesc). The flops are in the
+// batched products (Gram, Q1, Q1^T T, T -= Q1 D); these kernels move columns and
+// do the k x k work around them, bound by their traffic or by launch latency.
+// At n = 128 the three wide levels' decompositions took 758 ms as row compression
+// plus a column-by-column pivoted QR (each step reading and writing the whole
+// trailing face).
+// ===========================================================================
+
+// Thread = row of a 256-row chunk, so every column access is coalesced and a row's
+// picked entries are saved before the displaced columns overwrite them.
+__global__ void __launch_bounds__(256) k_pqr_extract(const PqrDesc* __restrict__ descs) {
+  const PqrDesc d = descs[blockIdx.y];
+  const int k = d.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if ((int)blockIdx.x * 256 >= d.m) return;
+  __shared__ int piv[kPqrCap], sel[kPqrCap], from[kPqrCap], to[kPqrCap], wsum[2][8];
+  if (tid < kPqrCap) sel[tid] = 0;
+  __syncthreads();
+  int p = -1;
+  if (tid < k) {
+    p = d.piv[tid];
+    piv[tid] = p;
+    if (p < k) sel[p] = 1;
+  }
+  __syncthreads();
+  // unpicked positions below k (ascending) go to the picked positions beyond k
+  const bool isf = tid < k && !sel[tid], ist = tid < k && p >= k;
+  const unsigned bf = __ballot_sync(0xffffffffu, isf), bt = __ballot_sync(0xffffffffu, ist);
+  if (lane == 0) {
+    wsum[0][warp] = __popc(bf);
+    wsum[1][warp] = __popc(bt);
+  }
+  __syncthreads();
+  int of = 0, ot = 0, nmove = 0;
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) {
+      of += wsum[0][w];
+      ot += wsum[1][w];
+    }
+    nmove += wsum[0][w];
+  }
+  const unsigned below = (1u << lane) - 1u;
+  if (isf) from[of + __popc(bf & below)] = tid;
+  if (ist) to[ot + __popc(bt & below)] = p;
+  __syncthreads();
+  // eight columns' loads in flight before their stores
+  const int r = blockIdx.x * 256 + tid;
+  if (r < d.m) {
+    double* T = d.T + (long long)d.o * d.m + r;
+    double* S = d.S + r;
+    for (int i0 = 0; i0 < k; i0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = (i0 + u < k) ? T[(long long)piv[i0 + u] * d.m] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i0 + u < k) S[(long long)(i0 + u) * d.m] = v[u];
+    }
+    // sources lie below k, destinations beyond: no overlap
+    for (int q0 = 0; q0 < nmove; q0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = (q0 + u < nmove) ? T[(long long)from[q0 + u] * d.m] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (q0 + u < nmove) T[(long long)to[q0 + u] * d.m] = v[u];
+    }
+  }
+  if (blockIdx.x == 0) {
+    int* perm = d.perm + d.o;
+    int mine = 0, moved = 0;
+    if (tid < k) mine = perm[piv[tid]];
+    if (tid < nmove) moved = perm[from[tid]];
+    __syncthreads();
+    if (tid < k) perm[tid] = mine;
+    if (tid < nmove) perm[to[tid]] = moved;
+    const int w = d.n - d.o;
+    for (int e = tid; e < k * k; e += 256) {
+      const int a = e % k, b = e / k;
+      d.R1[e] = (b >= a) ? d.Rsel[(long long)a * w + piv[b]] : 0.0;
+    }
+  }
+}
+
+void launch_pqr_extract(const PqrDesc* d_desc, int nd, int max_m, cudaStream_t s) {
+  if (nd <= 0) return;
+  k_pqr_extract<<<dim3((max_m + 255) / 256, nd), 256, 0, s>>>(d_desc);
+}
+
+// R1^{-1} by 32-wide block columns, a CTA each (they are independent): block row i
+// of column j is R_ii^{-1} (I_ij - sum_{l > i} R_il X_lj), from the diagonal up.
+constexpr int kPqrTi = 32;
+__global__ void __launch_bounds__(256) k_pqr_trinv(const PqrDesc* __restrict__ descs) {
+  const PqrDesc d = descs[blockIdx.y];
+  const int k = d.k, j0 = blockIdx.x * kPqrTi, tid = threadIdx.x;
+  if (j0 >= k) return;
+  const int nc = min(kPqrTi, k - j0), rows = j0 + nc;
+  extern __shared__ double ti_sm[];
+  double* X = ti_sm;                                  // [c][row], rows <= kPqrCap
+  double* Rt = X + kPqrTi * (kPqrCap + 1);            // 32 x 33
+  double* Y = Rt + kPqrTi * (kPqrTi + 1);             // 32 x 33: [c][row]
+  const int tx = tid & 31, ty = tid >> 5;             // row, column group of 4
+  for (int i0 = j0; i0 >= 0; i0 -= kPqrTi) {
+    const int nr = min(kPqrTi, k - i0);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* Ri = d.R1 + i0 + tx;
+    for (int l = i0 + kPqrTi; l < rows; ++l) {
+      const double rv = (tx < nr) ? Ri[(long long)l * k] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fma(rv, X[(ty * 4 + q) * (kPqrCap + 1) + l], acc[q]);
+    }
+    for (int e = tid; e < kPqrTi * kPqrTi; e += 256) {
+      const int a = e % kPqrTi, b = e / kPqrTi;
+      const double v = (a < nr && b < nr) ? d.R1[(i0 + a) + (long long)(i0 + b) * k]
+                                          : (a == b ? 1.0 : 0.0);
+      Rt[b * (kPqrTi + 1) + a] = (a == b) ? 1.0 / v : v;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = ty * 4 + q;
+      Y[c * (kPqrTi + 1) + tx] =
+          (tx < nr) ? ((i0 == j0 && tx == c) ? 1.0 : 0.0) - acc[q] : 0.0;
+    }
+    __syncthreads();
+    if (tid < nc) {
+      double y[kPqrTi];
+#pragma unroll
+      for (int a = 0; a < kPqrTi; ++a) y[a] = Y[tid * (kPqrTi + 1) + a];
+#pragma unroll
+      for (int a = kPqrTi - 1; a >= 0; --a) {
+        y[a] *= Rt[a * (kPqrTi + 1) + a];
+#pragma unroll
+        for (int t = 0; t < kPqrTi; ++t)
+          if (t < a) y[t] = fma(-Rt[a * (kPqrTi + 1) + t], y[a], y[t]);
+      }
+#pragma unroll
+      for (int a = 0; a < kPqrTi; ++a)
+        if (a < nr) X[tid * (kPqrCap + 1) + i0 + a] = y[a];
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < k * nc; e += 256) {
+    const int a = e % k, c = e / k;
+    d.R1inv[a + (long long)(j0 + c) * k] = (a < rows) ? X[c * (kPqrCap + 1) + a] : 0.0;
+  }
+}
+
+void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s) {
+  if (nd <= 0) return;
+  const int smem = (kPqrTi * (kPqrCap + 1) + 2 * kPqrTi * (kPqrTi + 1)) * (int)sizeof(double);
+  ensure_smem((const void*)k_pqr_trinv, smem);
+  k_pqr_trinv<<<dim3((max_k + kPqrTi - 1) / kPqrTi, nd), 256, smem, s>>>(d_desc);
+}
+
+// A CTA per 32 columns of [R1 | Q1^T T]: with C the columns in shared memory and E
+// read once per CTA, row a needs sum_{l<a}, l = a and sum_{l>a} of E(a, l) C(l).
+constexpr int kPqrFc = 32;
+__global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ descs,
+                                                 int* __restrict__ flag) {
+  const PqrDesc d = descs[blockIdx.y];
+  const int k = d.k, cols = d.n - d.o, c0 = blockIdx.x * kPqrFc, tid = threadIdx.x;
+  if (c0 >= cols) return;
+  const int nc = min(kPqrFc, cols - c0);
+  extern __shared__ double fx_sm[];  // [c][row], ld k | 1
+  const int ld = k | 1;
+  for (int e = tid; e < k * nc; e += 256) {
+    const int a = e % k, c = e / k, j = c0 + c;
+    fx_sm[a + c * ld] = (j < k) ? d.R1[a + (long long)j * k] : d.Z[a + (long long)j * k];
+  }
+  __syncthreads();
+  const int tx = tid & 31, ty = tid >> 5;  // row within 32, group of 4 columns
+  bool bad = false;
+  for (int a0 = 0; a0 < k; a0 += 32) {
+    const int a = a0 + tx;
+    if (a >= k) continue;
+    double lo[4] = {}, up[4] = {};
+    const double* Ea = d.Z + a;  // row a of Q1^T Q1 (symmetric)
+    auto add = [&](double (&acc)[4], int l) {
+      const double e = Ea[(long long)l * k];
+      bad |= !(fabs(e) <= kPqrMaxE);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fma(e, fx_sm[l + (ty * 4 + q) * ld], acc[q]);
+    };
+#pragma unroll 4
+    for (int l = 0; l < a0; ++l) add(lo, l);
+    const int a1 = min(k, a0 + 32);
+    for (int l = a0; l < a1; ++l) {
+      if (l < a) add(lo, l);
+      else if (l > a) add(up, l);
+    }
+#pragma unroll 4
+    for (int l = a1; l < k; ++l) add(up, l);
+    const double ed = Ea[(long long)a * k] - 1.0;
+    bad |= !(fabs(ed) <= kPqrMaxE);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = ty * 4 + q, j = c0 + c;
+      if (c >= nc) continue;
+      const double v = fx_sm[a + c * ld];
+      double* row = d.Rr + (long long)(d.o + a) * d.n;
+      const int col = d.perm[d.o + j];
+      if (j < k) {
+        // column j of R11 = (I + U) R1 (zero below the diagonal)
+        row[col] = (j >= a) ? v + 0.5 * ed * v + up[q] : 0.0;
+      } else {
+        row[col] = v - (lo[q] + 0.5 * ed * v);
+        d.Z[a + (long long)j * k] = v - (lo[q] + ed * v + up[q]);
+      }
+    }
+  }
+  if (bad) atomicOr(flag, 1);
+}
+
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_cols, int* flag, cudaStream_t s) {
+  if (nd <= 0) return;
+  const int smem = kPqrFc * (kPqrCap + 1) * (int)sizeof(double);
+  ensure_smem((const void*)k_pqr_fix, smem);
+  k_pqr_fix<<<dim3((max_cols + kPqrFc - 1) / kPqrFc, nd), 256, smem, s>>>(d_desc, flag);
+}
+
+__global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ outs, double eps,
+                                                    int* __restrict__ flag,
+                                                    int* __restrict__ status) {
+  const PqrOut o = outs[blockIdx.x];
+  const int n = o.id.n, tid = threadIdx.x, nthr = blockDim.x;
+  extern __shared__ int pn_sm[];  // perm
+  __shared__ int s_k, s_last;
+  if (tid == 0) s_k = s_last = 0;
+  for (int i = tid; i < n; i += nthr) pn_sm[i] = o.perm[i];
+  __syncthreads();
+  const double r00 = fabs(o.Rr[pn_sm[0]]), tol = r00 * eps;
+  for (int i = tid; i < n; i += nthr) {
+    const double v = o.Rr[(long long)i * n + pn_sm[i]];
+    const int kp = fabs(v) > tol;
+    if (blockIdx.y == 0) {
+      o.id.jpvt[i] = pn_sm[i];
+      o.id.rdiag[i] = v;
+      o.id.keep[i] = kp;
+    }
+    if (kp) {
+      atomicAdd(&s_k, 1);
+      atomicMax(&s_last, i + 1);
+    }
+  }
+  __syncthreads();
+  const int k = s_k;
+  if (tid == 0 && blockIdx.y == 0) {
+    *o.id.rank = k;
+    if (s_last != k) atomicOr(flag, 2);
+    if (r00 == 0.0) atomicOr(status, kStatusIdZero);
+  }
+  // rows of R by position: R11 (ld k, upper) and R12, split over the face's CTAs
+  for (long long e = tid + (long long)blockIdx.y * nthr; e < (long long)k * n;
+       e += (long long)nthr * gridDim.y) {
+    const int a = (int)(e / n), i = (int)(e % n);
+    const double v = (i >= a) ? o.Rr[(long long)a * n + pn_sm[i]] : 0.0;
+    if (i < k) o.R11[a + (long long)i * k] = v;
+    else o.id.W[a + (long long)(i - k) * k] = v;
+  }
+}
+
+void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* flag, int* status,
+                       cudaStream_t s) {
+  if (nd <= 0) return;
+  const size_t smem = (size_t)max_n * sizeof(int);
+  if (smem > 48 * 1024) ensure_smem((const void*)k_pqr_finish, smem);
+  k_pqr_finish<<<dim3(nd, nd < 148 ? 16 : 2), 512, smem, s>>>(d_out, eps, flag, status);
+}
+
+// ===========================================================================
 // Source membership (one CTA per cell / face)
 // ===========================================================================
 __global__ void k_member_cells(const int* __restrict__ skel, const long long* __restrict__ off,

@@ -126,6 +126,49 @@ struct TrsmBlockDesc {
 };
 void launch_trsm_block(const TrsmBlockDesc* d_desc, int nd, int max_cols, cudaStream_t s);
 
+// ---- Column-pivoted QR of a tall face by phases (FP64 interpolative
+// decomposition). T holds the columns not yet chosen, less their components along
+// the chosen ones. A phase picks pivots by pivoted Cholesky of G = T^T T until the
+// largest remaining norm has fallen by kPqrDrop (at most kPqrCap pivots), then
+// orthogonalises the picked columns S twice: Q1 = S R1^{-1} with R1 from the
+// Cholesky rows, E = Q1^T Q1 - I, Q = Q1 (I + E)^{-1/2} to second order in E; R's
+// rows are R11 = (I + U) R1 and B = (I - U^T) Q1^T T, U the upper triangle of E
+// with half its diagonal, and T -= Q1 (I - E) Q1^T T. G is formed again from the
+// updated T, so a pivot's norm is never resolved below kPqrDrop of the phase's
+// largest: its relative error stays near u / kPqrDrop^2, where the usual norm
+// downdating of a pivoted QR lets it reach sqrt(u).
+constexpr int kPqrCap = 256;        // pivots of one phase, at most
+constexpr double kPqrDrop = 1e-3;   // end of a phase: remaining norm / first norm
+constexpr double kPqrMaxE = 1e-6;   // largest |E| accepted (E^2 is dropped)
+struct PqrDesc {
+  double* T;      // m x n, ld m; columns o.. are active, o + k.. remain after this phase
+  double* S;      // m x kPqrCap, ld m: the picked columns
+  double* R1;     // k x k, ld k, upper
+  double* R1inv;  // k x k, ld k, upper
+  double* Z;      // k x (n - o), ld k: [Q1^T Q1 | Q1^T T]; the second part ends as (I - E) Q1^T T
+  double* Rr;     // n x n row-major: row i of R by column of the face
+  int* perm;      // n: column of the face at each position of T
+  const double* Rsel;  // the phase's Cholesky rows (row-major, n - o wide)
+  const int* piv;      // the phase's pivots as positions relative to o
+  int m, n, o, k;
+};
+// Picked columns to S, the columns they displace into the holes, perm, R1.
+void launch_pqr_extract(const PqrDesc* d_desc, int nd, int max_m, cudaStream_t s);
+void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s);
+// R11 and B into Rr, (I - E) Q1^T T over Z; *flag |= 1 where |E| exceeds kPqrMaxE.
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_cols, int* flag, cudaStream_t s);
+// After the last phase: jpvt, rdiag, keep, rank; R11 (k x k, ld k) into G and R12
+// into W for the triangular solve. *flag |= 2 where the kept columns are not a
+// prefix of the pivot order.
+struct PqrOut {
+  const double* Rr;
+  const int* perm;
+  double* R11;
+  IdDesc id;
+};
+void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* flag, int* status,
+                       cudaStream_t s);
+
 // Source membership of the DOFs (the 6 x NC^3 arrays read by k_gather), built
 // on the device. Cells: skeleton DOF t of cell b (cell_ids[b] >= 0) gets
 // (source, t) in slot pair 0 (on the cell's low face along some axis) or 1.

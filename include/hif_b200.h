@@ -191,7 +191,11 @@ enum hif_option {
                                 2: per-phase host and device times, no synchronisation */
   HIF_OPT_MEM_BUDGET_MB = 3, /* refuse factorizations whose device memory exceeds this */
   HIF_OPT_PROFILE = 4,       /* time every launch with CUDA events (resets the counters) */
-  HIF_OPT_ID_GROUP_MIN_N = 5, /* faces with at least this many columns get a CTA group (default 512) */
+  HIF_OPT_ID_GROUP_MIN_N = 5, /* column-by-column pivoted QR of the faces wider than 64 columns:
+                                 faces with at least this many columns get a CTA group (default
+                                 512). Setting it selects that QR for these faces; otherwise
+                                 they are decomposed by phases (the same pivots and R up to
+                                 rounding; R's diagonal is positive there) */
   HIF_OPT_PRECISION = 6,      /* HIF_PRECISION_FP64 (default) or HIF_PRECISION_MIXED */
   HIF_OPT_AUTOTUNE = 7,       /* 1: tune online: the tile shape of the batched FP64
                                  products per batch signature, and in mixed precision on
