@@ -474,14 +474,14 @@ struct Sources {
   BufList bufs;                // device memory holding the blocks
 };
 
-// One batched GEMM launch; 128x128 tiles when most of the work sits in
-// problems at least that large (or when forced: in-place panel products rely on
-// a single output tile along the aliased dimension), else 64x64. Problems with
+// One batched GEMM launch: 64x64 tiles (as fast as larger ones on large problems
+// and less padding on the rest), or 128x128 when forced (in-place panel products
+// rely on a single output tile along the aliased dimension). Problems with
 // a reduction much longer than their output dimensions are split along k into
 // partial products and summed in a fixed order.
 // Online tile-shape tuner for the batched FP64 products (HIF_OPT_AUTOTUNE).
 // A batch is keyed by its class and the log2 buckets of its work and mean
-// shape; until both candidate tiles (64 x 64 FFMA, 128 x 128 DMMA) have run
+// shape; until both candidate tiles (64 x 64, 128 x 128) have run
 // once for a key, the next untried one runs with events around it; after that
 // the faster is kept. Events are read when the factorization synchronises.
 struct GemmTuner {
@@ -639,15 +639,9 @@ void gemm_batch(const std::vector<GemmDesc>& gin, BufList& tmp, cudaStream_t str
     red.push_back(SplitKDesc{x.C, P + po, x.ldc, x.m, x.n, sp.S, x.alpha, x.beta});
     po += (long long)sp.S * x.m * x.n;
   }
-  double big = 0, all = 0;
-  for (const GemmDesc& x : g) {
-    const double w = (double)x.m * x.n;
-    all += w;
-    if (x.m >= 96 && x.n >= 96) big += w;
-  }
-  bool lower = false;  // lower-triangle products are tiled by 128 x 128
+  bool lower = false;
   for (const GemmDesc& x : g) lower = lower || x.lower;
-  int tile = force_tile ? force_tile : ((lower || big >= 0.5 * all) ? 128 : 64);
+  int tile = force_tile ? force_tile : 64;
   GemmTuner::Pending tp{0, -1, nullptr, nullptr};
   if (t_tuner && !force_tile && !lower && !g.empty()) {
     double sm = 0, sn = 0, sk = 0;
@@ -922,7 +916,7 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
         u.k = nbk;
         u.alpha = -1.0;
         u.beta = 1.0;
-        u.lower = 1;
+        u.lower = 2;
         gu.push_back(u);
       }
       cdg.push_back(CopyDesc{Dv, d.a22inv + k0 + (long long)k0 * r, nbk, r, nbk, nbk});
@@ -940,7 +934,7 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
     }
     gemm_batch(gp, step, stream, HIF_KCLASS_SWEEP_PANEL, timed);
     // rank-128 updates: FP64 (from int8 slices they are bound by their C traffic)
-    gemm_batch(gu, step, stream, HIF_KCLASS_GEMM, timed, 128);
+    gemm_batch(gu, step, stream, HIF_KCLASS_GEMM, timed);
     {
       CopyDesc* dc = step.add(upload(cdg, stream));
       int* doc = step.add(upload(ocd, stream));
@@ -1073,7 +1067,7 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
   else gemm_batch(gy, tmp, stream, HIF_KCLASS_GEMM, timed);
   if (ar.schur > 0) gemm_batch_int8(gs, tmp, stream, timed, ar.schur, d_status);
   else if (ar.schur == 0) gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM_MIXED, timed, 128, d_status);
-  else gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM, timed, 128);
+  else gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM, timed);
   std::vector<TCopyDesc> tm;
   std::vector<int> otm(1, 0);
   for (const SweepDesc& d : large) {
@@ -1398,7 +1392,7 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
   else gemm_batch(gx, tmp, stream, HIF_KCLASS_GEMM, timed);
   if (ar.schur > 0) gemm_batch_int8(gs, tmp, stream, timed, ar.schur, d_status);
   else if (ar.schur == 0) gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM_MIXED, timed, 128, d_status);
-  else gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM, timed, sym ? 128 : 0);
+  else gemm_batch(gs, tmp, stream, HIF_KCLASS_GEMM, timed);
   if (sym) {
     std::vector<TCopyDesc> tm;
     std::vector<int> otm(1, 0);
@@ -1706,7 +1700,7 @@ class Engine {
         std::vector<long long> goff(1, 0), eoff(1, 0);
         std::vector<int> toff(1, 0);
         long long ox = 0, oy = 0;
-        const int tile = nrhs >= 48 ? 128 : 64;
+        const int tile = 64;
         for (const GemvDesc& g : l.hdesc) {
           const int len = g.trans ? g.m : g.n, rows = g.trans ? g.n : g.m;
           gd.push_back(ApplyGatherDesc{g.in_idx, xin + ox, len});
@@ -2833,7 +2827,7 @@ class Engine {
       g.transA = 1;
       g.alpha = 1.0;
       g.beta = 0.0;
-      g.lower = 1;  // G is symmetric: the panels read its lower triangle only
+      g.lower = 2;  // G is symmetric: the panels read its lower triangle only
       gram.push_back(g);
     }
     auto tm = [&](int cls, double fl, double by, auto&& f, int n) { timed(cls, fl, by, f, n); };
@@ -2841,7 +2835,7 @@ class Engine {
     // slices the product's error, about k 2^-56 max|M|^2, is below an FP64
     // product's k u |M|^2 bound, so the pivots and rank see FP64 accuracy
     if (gram_slices > 0) gemm_batch_int8(gram, tmp, stream, tm, gram_slices, d_status);
-    else gemm_batch(gram, tmp, stream, HIF_KCLASS_QR, tm, 128);
+    else gemm_batch(gram, tmp, stream, HIF_KCLASS_QR, tm);
     PcholDesc* dpd = tmp.add(upload(pd, stream));
     // a fixed sequence of panels without host synchronisation: a face whose
     // rank is known skips its later panels and updates on the device
@@ -2866,7 +2860,7 @@ class Engine {
         g.k = kPcholNB;
         g.alpha = -1.0;
         g.beta = 1.0;
-        g.lower = 1;
+        g.lower = 2;
         g.skip = pd[q].info + 1;
         upd.push_back(g);
       }
@@ -2877,7 +2871,7 @@ class Engine {
                            stream);
       });
       HIF_CK(cudaGetLastError());
-      gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm, 128);
+      gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm);
       HIF_CK(cudaGetLastError());
       step.release(stream);
     }
@@ -2959,7 +2953,6 @@ class Engine {
       const int na = (int)act.size();
       std::vector<PcholDesc> pd(na);
       std::vector<GemmDesc> gram;
-      std::vector<int> ids(na);
       int max_w = 0;
       for (int q = 0; q < na; ++q) {
         const IdDesc& d = v[act[q]];
@@ -2984,12 +2977,11 @@ class Engine {
         g.k = d.m;
         g.transA = 1;
         g.alpha = 1.0;
-        g.lower = 1;
+        g.lower = 2;
         gram.push_back(g);
-        ids[q] = q;
       }
       HIF_CK(cudaMemsetAsync(info, 0, 2LL * na * sizeof(int), stream));
-      gemm_batch(gram, step, stream, HIF_KCLASS_QR, tm, 128);
+      gemm_batch(gram, step, stream, HIF_KCLASS_QR, tm);
       PcholDesc* dpd = step.add(upload(pd, stream));
       for (int i0 = 0; i0 < std::min(max_w, kPqrCap); i0 += kPcholNB) {
         std::vector<int> on;
@@ -3009,7 +3001,7 @@ class Engine {
           g.k = kPcholNB;
           g.alpha = -1.0;
           g.beta = 1.0;
-          g.lower = 1;
+          g.lower = 2;
           g.skip = pd[q].info + 1;
           upd.push_back(g);
         }
@@ -3019,7 +3011,7 @@ class Engine {
                              stream);
         });
         HIF_CK(cudaGetLastError());
-        gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm, 128);
+        gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm);
       }
       HIF_CK(cudaMemcpyAsync(h_info, info, 2LL * na * sizeof(int), cudaMemcpyDeviceToHost, stream));
       HIF_CK(cudaMemcpyAsync(h_info + 2LL * nd, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -3745,7 +3737,7 @@ class Engine {
     }
     std::vector<GemmDesc> v(1, g);
     gemm_batch(v, tmp, stream, HIF_KCLASS_GEMM,
-               [&](int, double, double, auto&& f, int = 1) { f(); }, 128);
+               [&](int, double, double, auto&& f, int = 1) { f(); });
     HIF_CK(cudaGetLastError());
     sync();
     HIF_CK(cudaMemcpy(out, C, (size_t)r * ncol * 8, cudaMemcpyDeviceToHost));

@@ -236,141 +236,28 @@ void launch_gather(const GatherTarget* d_tg, const int* d_tile_off, int ntg, int
 }
 
 // ===========================================================================
-// Batched FP64 GEMM: 64x64x16 tiles, 256 threads, 4x4 outputs per thread.
-// Thread (tx, ty) owns rows tx + 16 a and columns ty + 16 b so that the
-// epilogue stores are coalesced along the (column-major) rows.
+// Batched FP64 GEMM on the FP64 tensor cores (DMMA, mma.sync m8n8k4), 64 x 64 x 16
+// tiles by 4 warps (32 x 32 each), four CTAs per SM; and 128 x 128 x 16 tiles by 16
+// warps, for products that need one tile along a dimension (in-place panels) and as
+// the tuner's other candidate. Operands go through a cp.async pipeline (8-byte
+// copies: sub-matrix views are only 8-byte aligned; out-of-range elements are
+// zero-filled by the copy).
+//
+// Bound: the DMMA pipe. What kept it idle was the work between two stages' products:
+// recomputing every copy's address and bounds (~15 instructions a copy) right after
+// the barrier, with all 16 warps of one CTA at the same point. So a thread's copies
+// are one pointer plus constant strides, the next stage's copies are issued a quarter
+// after each k-step of 4, and four independent CTAs fill each other's barriers,
+// fragment loads and epilogues. 8000 x 8000 (odd sizes), TF/s before -> after, at
+// k = 2050: 23.8 -> 31.4, transposed A with beta = 1: 23.2 -> 31.1, k = 128 with
+// beta = 1: 18.2 -> 28.0 (cuBLAS, aligned: 34.6 at k = 2050); the 128 x 128 form 30.8,
+// 30.3 and 22.1. Stage rows are padded to 4 mod 16 doubles: a fragment load (8 rows x
+// 4 k) then touches each bank pair once per half warp.
 // ===========================================================================
-constexpr int kBM = 64, kBN = 64, kBK = 16;
-
 int dgemm_tiles(int m, int n, int tile) {
   if (m <= 0 || n <= 0) return 0;
   return ((m + tile - 1) / tile) * ((n + tile - 1) / tile);
 }
-
-__global__ void __launch_bounds__(256) k_dgemm(const GemmDesc* __restrict__ descs,
-                                               const int* __restrict__ tile_off, int nd) {
-  const int di = find_desc(tile_off, nd, blockIdx.x);
-  const GemmDesc g = descs[di];
-  const int local = blockIdx.x - tile_off[di];
-  const int tiles_m = (g.m + kBM - 1) / kBM;
-  if (g.skip && *g.skip) return;
-  const int m0 = (local % tiles_m) * kBM, n0 = (local / tiles_m) * kBN;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-
-  __shared__ double As[2][kBK][kBM + 1];
-  __shared__ double Bs[2][kBK][kBN + 1];
-
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-
-  double ra[4], rb[4];
-  auto load_a = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      int mm, kk;
-      if (g.transA == 0) { mm = e % kBM; kk = e / kBM; } else { mm = e / kBK; kk = e % kBK; }
-      const int gm = m0 + mm, gk = k0 + kk;
-      double v = 0.0;
-      if (gm < g.m && gk < g.k)
-        v = (g.transA == 0) ? g.A[gm + (long long)gk * g.lda] : g.A[gk + (long long)gm * g.lda];
-      ra[q] = v;
-    }
-  };
-  auto load_b = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      int nn, kk;
-      if (g.transB == 0) { kk = e % kBK; nn = e / kBK; } else { nn = e % kBN; kk = e / kBN; }
-      const int gn = n0 + nn, gk = k0 + kk;
-      double v = 0.0;
-      if (gn < g.n && gk < g.k)
-        v = (g.transB == 0) ? g.B[gk + (long long)gn * g.ldb] : g.B[gn + (long long)gk * g.ldb];
-      rb[q] = v;
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      int mm, kk;
-      if (g.transA == 0) { mm = e % kBM; kk = e / kBM; } else { mm = e / kBK; kk = e % kBK; }
-      As[buf][kk][mm] = ra[q];
-      int nn, kb;
-      if (g.transB == 0) { kb = e % kBK; nn = e / kBK; } else { nn = e % kBN; kb = e / kBN; }
-      Bs[buf][kb][nn] = rb[q];
-    }
-  };
-
-  const int kend = g.a_lower ? min(g.k, m0 + kBM) : g.k;
-  const int kbeg = g.b_lower ? min(kend, n0) : 0;  // n0: a multiple of kBK
-  const int nk = (kend - kbeg + kBK - 1) / kBK;
-  if (nk > 0) {
-    load_a(kbeg);
-    load_b(kbeg);
-    store(0);
-  }
-  __syncthreads();
-  for (int t = 0; t < nk; ++t) {
-    const int buf = t & 1;
-    if (t + 1 < nk) {
-      load_a(kbeg + (t + 1) * kBK);
-      load_b(kbeg + (t + 1) * kBK);
-    }
-#pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      double av[4], bv[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[buf][kk][tx + 16 * a];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = Bs[buf][kk][ty + 16 * b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
-    }
-    if (t + 1 < nk) store(buf ^ 1);
-    __syncthreads();
-  }
-  // with beta != 0 every C entry is loaded before the first store, so that the
-  // 16 loads are in flight together
-  double cv[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b)
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int gm = m0 + tx + 16 * a, gn = n0 + ty + 16 * b;
-      cv[a][b] = (g.beta != 0.0 && gm < g.m && gn < g.n) ? g.C[gm + (long long)gn * g.ldc] : 0.0;
-    }
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int gn = n0 + ty + 16 * b;
-    if (gn >= g.n) continue;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int gm = m0 + tx + 16 * a;
-      if (gm >= g.m) continue;
-      const double v = g.alpha * acc[a][b];
-      g.C[gm + (long long)gn * g.ldc] = (g.beta == 0.0) ? v : fma(g.beta, cv[a][b], v);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// 128 x 128 x 16 tiles, 256 threads, 8 x 8 outputs per thread, operands staged
-// through a 3-stage cp.async pipeline (8-byte copies: sub-matrix views are
-// only 8-byte aligned; out-of-range elements are zero-filled by the copy).
-// ---------------------------------------------------------------------------
-constexpr int kLBM = 128, kLBN = 128, kLBK = 16, kLStages = 3;
-constexpr int kLAStride = kLBM + 2;  // doubles per k-row of the A stage
-constexpr int kLBStride = kLBN + 2;
-constexpr int kLSmem = kLStages * kLBK * (kLAStride + kLBStride) * (int)sizeof(double);
-// with beta != 0 the C tile is prefetched into shared memory with the first stages
-constexpr int kLSmemC = kLSmem + kLBM * kLBN * (int)sizeof(double);
 
 __device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool valid) {
   const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem);
@@ -384,56 +271,82 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-__global__ void __launch_bounds__(512, 1) k_dgemm128(const GemmDesc* __restrict__ descs,
-                                                     const int* __restrict__ tile_off, int nd) {
+constexpr int kGBK = 16;  // k per stage
+template <int BM, int BN, int ST>
+constexpr int dgemm_smem() {
+  return ST * kGBK * (BM + 4 + BN + 4) * (int)sizeof(double);
+}
+
+// Warp tile 32 x 32 = 4 x 4 MMA tiles. Fragments (PTX ISA, m8n8k4 .f64): with
+// g = lane / 4, t = lane % 4, A holds (row g, k t), B holds (k t, col g), C holds
+// (row g, cols 2t and 2t + 1).
+template <int BM, int BN, int ST, int MINB>
+__global__ void __launch_bounds__(BM * BN / 32, MINB)
+    k_dgemm(const GemmDesc* __restrict__ descs, const int* __restrict__ tile_off, int nd) {
+  constexpr int T = BM * BN / 32;  // threads
+  constexpr int SA = BM + 4, SB = BN + 4;
+  constexpr int QA = BM * kGBK / T, QB = BN * kGBK / T;  // copies of a thread per stage
+  constexpr int KS = kGBK / 4;
+  static_assert(T % BM == 0 && T % BN == 0 && T % kGBK == 0 && QA % KS == 0 && QB % KS == 0,
+                "a thread's copies differ by constant strides, an equal share per k-step");
   extern __shared__ double lsm[];
-  double* As = lsm;                                  // [stage][k][kLAStride]
-  double* Bs = lsm + kLStages * kLBK * kLAStride;    // [stage][k][kLBStride]
+  double* As = lsm;                   // [stage][k][SA]
+  double* Bs = lsm + ST * kGBK * SA;  // [stage][k][SB]
   const int di = find_desc(tile_off, nd, blockIdx.x);
   const GemmDesc g = descs[di];
   const int local = blockIdx.x - tile_off[di];
-  const int tiles_m = (g.m + kLBM - 1) / kLBM;
-  if (g.lower && local % tiles_m < local / tiles_m) return;
+  const int tiles_m = (g.m + BM - 1) / BM;
+  const int m0 = (local % tiles_m) * BM, n0 = (local / tiles_m) * BN;
+  // lower: 1 skips the 128 x 128 blocks above the diagonal, 2 the tiles above it
+  if (g.lower == 1 && m0 / 128 < n0 / 128) return;
+  if (g.lower == 2 && m0 < n0) return;
   if (g.skip && *g.skip) return;
-  const int m0 = (local % tiles_m) * kLBM, n0 = (local / tiles_m) * kLBN;
+  const int kend = g.a_lower ? min(g.k, m0 + BM) : g.k;
+  const int kbeg = g.b_lower ? min(kend, n0) : 0;  // n0: a multiple of kGBK
+  const int nk = (kend - kbeg + kGBK - 1) / kGBK;
   const int tid = threadIdx.x;
-
-  auto issue = [&](int stage, int k0) {
-    double* as = As + stage * kLBK * kLAStride;
-    double* bs = Bs + stage * kLBK * kLBStride;
+  const bool ta = g.transA != 0, tb = g.transB != 0;
+  // copy q of a thread: A row amm (+ q T / BK if transposed), k akk (+ q T / BM if not)
+  const int amm = ta ? tid / kGBK : tid % BM, akk = ta ? tid % kGBK : tid / BM;
+  const int bnn = tb ? tid % BN : tid / kGBK, bkk = tb ? tid / BN : tid % kGBK;
+  const long long astep = (long long)(ta ? T / kGBK : T / BM) * g.lda;
+  const long long bstep = (long long)(tb ? T / BN : T / kGBK) * g.ldb;
+  const long long aadv = ta ? kGBK : (long long)kGBK * g.lda;
+  const long long badv = tb ? (long long)kGBK * g.ldb : kGBK;
+  const int ak = kbeg + akk, bk = kbeg + bkk;
+  const double* ap = ta ? g.A + ak + (long long)(m0 + amm) * g.lda
+                        : g.A + (m0 + amm) + (long long)ak * g.lda;
+  const double* bp = tb ? g.B + (n0 + bnn) + (long long)bk * g.ldb
+                        : g.B + bk + (long long)(n0 + bnn) * g.ldb;
+  const int as0 = akk * SA + amm, bs0 = bkk * SB + bnn;
+  const int asq = ta ? T / kGBK : (T / BM) * SA, bsq = tb ? (T / BN) * SB : T / kGBK;
+  unsigned amask = 0, bmask = 0;  // copies whose row / column is in range
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 512 * q;
-      int mm, kk;
-      if (g.transA == 0) { mm = e % kLBM; kk = e / kLBM; } else { mm = e / kLBK; kk = e % kLBK; }
-      const int gm = m0 + mm, gk = k0 + kk;
-      const bool ok = gm < g.m && gk < g.k;
-      const double* src = ok ? ((g.transA == 0) ? g.A + gm + (long long)gk * g.lda
-                                                : g.A + gk + (long long)gm * g.lda)
-                             : g.A;
-      cp_async8(as + kk * kLAStride + mm, src, ok);
-    }
+  for (int q = 0; q < QA; ++q)
+    if (m0 + amm + (ta ? (T / kGBK) * q : 0) < g.m) amask |= 1u << q;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 512 * q;
-      int nn, kk;
-      if (g.transB == 0) { kk = e % kLBK; nn = e / kLBK; } else { nn = e % kLBN; kk = e / kLBN; }
-      const int gn = n0 + nn, gk = k0 + kk;
-      const bool ok = gn < g.n && gk < g.k;
-      const double* src = ok ? ((g.transB == 0) ? g.B + gk + (long long)gn * g.ldb
-                                                : g.B + gn + (long long)gk * g.ldb)
-                             : g.B;
-      cp_async8(bs + kk * kLBStride + nn, src, ok);
-    }
+  for (int q = 0; q < QB; ++q)
+    if (n0 + bnn + (tb ? 0 : (T / kGBK) * q) < g.n) bmask |= 1u << q;
+  // copies [q0, q1) of the stage whose first k is k0; ap / bp point at that stage
+  auto issue = [&](int stage, int k0, int part, int parts) {
+    double* as = As + stage * kGBK * SA + as0;
+    double* bs = Bs + stage * kGBK * SB + bs0;
+#pragma unroll
+    for (int q = 0; q < QA; ++q)
+      if (q >= QA / parts * part && q < QA / parts * (part + 1)) {
+        const bool ok = (amask >> q & 1) && k0 + akk + (ta ? 0 : (T / BM) * q) < kend;
+        cp_async8(as + q * asq, ok ? ap + q * astep : g.A, ok);
+      }
+#pragma unroll
+    for (int q = 0; q < QB; ++q)
+      if (q >= QB / parts * part && q < QB / parts * (part + 1)) {
+        const bool ok = (bmask >> q & 1) && k0 + bkk + (tb ? (T / BN) * q : 0) < kend;
+        cp_async8(bs + q * bsq, ok ? bp + q * bstep : g.B, ok);
+      }
   };
 
-  // FP64 tensor cores: mma.sync m8n8k4 (DMMA). 16 warps as 4 (m) x 4 (n), warp
-  // tile 32 x 32 = 4 x 4 MMA tiles (four warps per SM sub-partition keep the
-  // DMMA pipe fed across the fixed issue spacing of one warp). Fragments (PTX
-  // ISA, m8n8k4 .f64): with g = lane / 4, t = lane % 4, A holds (row g, k t),
-  // B holds (k t, col g), C holds (row g, cols 2t and 2t + 1).
   const int lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
+  const int wm = (warp % (BM / 32)) * 32, wn = (warp / (BM / 32)) * 32;
   const int gq = lane >> 2, tq = lane & 3;
   double acc[4][4][2];
 #pragma unroll
@@ -441,38 +354,28 @@ __global__ void __launch_bounds__(512, 1) k_dgemm128(const GemmDesc* __restrict_
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 
-  double* Cs = lsm + kLStages * kLBK * (kLAStride + kLBStride);  // [col][row], 128 x 128
-  const bool prefetch_c = g.beta != 0.0;
-  if (prefetch_c) {
-    for (int e = tid; e < kLBM * kLBN; e += 512) {
-      const int i = e % kLBM, j = e / kLBM;
-      const bool ok = (m0 + i) < g.m && (n0 + j) < g.n;
-      cp_async8(Cs + e, ok ? g.C + (m0 + i) + (long long)(n0 + j) * g.ldc : g.C, ok);
-    }
-  }
-  const int kend = g.a_lower ? min(g.k, m0 + kLBM) : g.k;
-  const int kbeg = g.b_lower ? min(kend, n0) : 0;  // n0: a multiple of kLBK
-  const int nk = (kend - kbeg + kLBK - 1) / kLBK;
 #pragma unroll
-  for (int st = 0; st < kLStages - 1; ++st) {
-    if (st < nk) issue(st, kbeg + st * kLBK);
-    cp_async_commit();  // the first group also carries the C tile
+  for (int st = 0; st < ST - 1; ++st) {
+    if (st < nk) {
+      issue(st, kbeg + st * kGBK, 0, 1);
+      ap += aadv;
+      bp += badv;
+    }
+    cp_async_commit();
   }
   for (int t = 0; t < nk; ++t) {
-    cp_async_wait<kLStages - 2>();
+    cp_async_wait<ST - 2>();
     __syncthreads();
-    const int nt = t + kLStages - 1;
-    if (nt < nk) issue(nt % kLStages, kbeg + nt * kLBK);
-    cp_async_commit();
-    const double* as = As + (t % kLStages) * kLBK * kLAStride;
-    const double* bs = Bs + (t % kLStages) * kLBK * kLBStride;
+    const int nt = t + ST - 1;
+    const double* as = As + (t % ST) * kGBK * SA + tq * SA + wm + gq;
+    const double* bs = Bs + (t % ST) * kGBK * SB + tq * SB + wn + gq;
 #pragma unroll
-    for (int k4 = 0; k4 < kLBK; k4 += 4) {
+    for (int k4 = 0; k4 < KS; ++k4) {
       double af[4], bf[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) af[a] = as[(k4 + tq) * kLAStride + wm + a * 8 + gq];
+      for (int a = 0; a < 4; ++a) af[a] = as[k4 * 4 * SA + a * 8];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bf[b] = bs[(k4 + tq) * kLBStride + wn + b * 8 + gq];
+      for (int b = 0; b < 4; ++b) bf[b] = bs[k4 * 4 * SB + b * 8];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -481,24 +384,34 @@ __global__ void __launch_bounds__(512, 1) k_dgemm128(const GemmDesc* __restrict_
               "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
               : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
               : "d"(af[a]), "d"(bf[b]));
+      if (nt < nk) issue(nt % ST, kbeg + nt * kGBK, k4, KS);
     }
+    cp_async_commit();
+    ap += aadv;
+    bp += badv;
   }
   cp_async_wait<0>();
-  __syncthreads();
+  // with beta != 0 a column group's C entries are loaded before its first store, so
+  // that the loads are in flight together
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int gm = m0 + wm + a * 8 + gq;
-    if (gm >= g.m) continue;
+  for (int b = 0; b < 4; ++b) {
+    double cv[4][2];
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        const int cl = wn + b * 8 + tq * 2 + c;
-        const int gn = n0 + cl;
-        if (gn >= g.n) continue;
-        double* cp = g.C + gm + (long long)gn * g.ldc;
+        const int gm = m0 + wm + a * 8 + gq, gn = n0 + wn + b * 8 + tq * 2 + c;
+        cv[a][c] =
+            (g.beta != 0.0 && gm < g.m && gn < g.n) ? g.C[gm + (long long)gn * g.ldc] : 0.0;
+      }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int gm = m0 + wm + a * 8 + gq, gn = n0 + wn + b * 8 + tq * 2 + c;
+        if (gm >= g.m || gn >= g.n) continue;
         const double v = g.alpha * acc[a][b][c];
-        *cp = prefetch_c ? fma(g.beta, Cs[cl * kLBM + wm + a * 8 + gq], v) : v;
+        g.C[gm + (long long)gn * g.ldc] = (g.beta == 0.0) ? v : fma(g.beta, cv[a][c], v);
       }
   }
 }
@@ -507,10 +420,13 @@ void launch_dgemm(const GemmDesc* d_desc, const int* d_tile_off, int nd, int tot
                   cudaStream_t s, int tile) {
   if (total_tiles <= 0) return;
   if (tile == 128) {
-    ensure_smem((const void*)k_dgemm128, kLSmemC);
-    k_dgemm128<<<total_tiles, 512, kLSmemC, s>>>(d_desc, d_tile_off, nd);
+    constexpr int smem = dgemm_smem<128, 128, 4>();
+    ensure_smem((const void*)k_dgemm<128, 128, 4, 1>, smem);
+    k_dgemm<128, 128, 4, 1><<<total_tiles, 512, smem, s>>>(d_desc, d_tile_off, nd);
   } else {
-    k_dgemm<<<total_tiles, 256, 0, s>>>(d_desc, d_tile_off, nd);
+    constexpr int smem = dgemm_smem<64, 64, 3>();
+    ensure_smem((const void*)k_dgemm<64, 64, 3, 4>, smem);
+    k_dgemm<64, 64, 3, 4><<<total_tiles, 128, smem, s>>>(d_desc, d_tile_off, nd);
   }
 }
 

@@ -63,7 +63,7 @@ struct GemmDesc {
   int m, n, k;
   int transA, transB;
   double alpha, beta;
-  int lower;  // 128 x 128 tiles only: skip the tiles above the diagonal (row tile < column tile)
+  int lower;  // skip what lies above the diagonal: 1 the 128 x 128 blocks, 2 the kernel's tiles
   const int* skip;  // optional: the product is skipped when *skip != 0 (read on the device)
   int a_lower;  // op(A) is lower triangular (m = k): a row tile reads no k past its last row
   int b_lower;  // op(B) is lower triangular (k = n): a column tile reads no k before its first column
@@ -261,8 +261,8 @@ void launch_gather(const GatherTarget* d_tg, const int* d_tile_off, int ntg, int
                    const double* d_band, long long ncell3, int NC, cudaStream_t s);
 int gather_tiles(int m, int n);
 
-// tile: 64 (64x64x16, 4x4 per thread) or 128 (128x128x16, 8x8 per thread,
-// 3-stage cp.async pipeline); tile offsets must be built with the same tile.
+// tile: 64 (64x64x16, 4 warps) or 128 (128x128x16, 16 warps); tile offsets must be
+// built with the same tile.
 void launch_dgemm(const GemmDesc* d_desc, const int* d_tile_off, int nd, int total_tiles,
                   cudaStream_t s, int tile = 64);
 int dgemm_tiles(int m, int n, int tile = 64);
