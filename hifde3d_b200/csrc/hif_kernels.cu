@@ -1397,115 +1397,297 @@ void launch_sweep_small(const SweepDesc* d_desc, int nd, int max_n, int* d_statu
 // Step for pivot block K = [k0, k1) of A22: Dinv = B[K, K]^{-1} (k_sweep_diag);
 // the row / column panels and the rank-128 update are batched GEMMs issued by
 // the host; B[K, K] = Dinv (k_sweep_setdiag).
-// Register-resident Gauss-Jordan inverse of the pivot block: thread (tx, ty)
-// of a 16 x 32 grid holds the 4 x 8 sub-block rows 4 ty.., columns 8 tx.. in
-// registers. At step k the owners of the old row k and column k publish them
-// to shared memory (two buffers, alternating, so one barrier per step orders
-// both the reads of step k and the writes of step k + 2); every thread then
-// updates its 32 entries with the same operations as the in-place sweep:
-// row k * (1 / p), column k * (-1 / p), the rest a - a_ik (a_kj / p).
-__global__ void __launch_bounds__(512) k_sweep_diag(const SweepDesc* __restrict__ descs,
-                                                    const int* __restrict__ active, int k0,
-                                                    double* __restrict__ dinv,
-                                                    int* __restrict__ status, int sym) {
+// The pivot block of both eliminations, 128 x 128, by 16-wide block steps: one CTA
+// per block, and on the critical path of the top levels, where one or a few blocks
+// remain, so it is built for latency. 16 worker warps hold the block as DMMA
+// accumulators (32 x 32 a warp); step K reads the panels of block K from the owners
+// through shared memory and updates everything by one rank-16 product:
+//   Gauss-Jordan: with D = block KK, R = D^{-1} (row panel), rows K := R, columns
+//     K := -C D^{-1}, the rest A - C R: with the K rows and columns of the
+//     accumulators zeroed, R[:, K] = D^{-1} and C[K, :] = -I it is A - C R throughout;
+//   Cholesky: l = chol(D), x = l^{-1}; L_iK = A_iK x^T below, the finished part of
+//     L^{-1} left of K gets X_K = x X_K; R = [X_K | x | L_jK^T], rows K := R and rows
+//     below K := A - L_iK R. The lower triangle only; L goes straight to B.
+// The serial part, the 16 x 16 inverse (or factor and inverse), is a 17th warp's: the
+// owner of the next diagonal block updates that block first and hands it over, so the
+// inverse runs beside the rest of the update (4096 DMMA cycles a step; 128^3
+// multiply-adds take 32.8 k). Before, the inverse was one pivot and one barrier at a
+// time over registers: 200 us a block, the factor 32-wide by one warp, 150 us.
+constexpr int kPbW = 16;                  // block step
+constexpr int kPbLd = kSweepNB + 4;       // panel rows: 4 mod 16 doubles, conflict-free fragments
+constexpr int kPbSt = kSweepNB + 1;       // staging
+constexpr int kPbD = kPbW + 1;
+constexpr int kPbThreads = 17 * 32;
+constexpr int kPbSmem =
+    (kSweepNB * kPbSt + 4 * kPbW * kPbLd + 4 * kPbW * kPbD) * (int)sizeof(double);
+
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 16 x 16 inverse (CHOL: the inverse of the Cholesky factor, the factor itself to
+// Ls[k][i]) by one warp: lane = (row i, half h), columns 8h .. 8h + 7 in registers.
+template <bool CHOL>
+__device__ __forceinline__ void pivot16(const double* Dn, double* Di, double* Ls, int live,
+                                        int& bad) {
+  const int lane = threadIdx.x & 31, i = lane & 15, h = lane >> 4;
+  double a[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) a[c] = Dn[i * kPbD + 8 * h + c];
+#pragma unroll
+  for (int k = 0; k < kPbW; ++k) {
+    const int kh = k >> 3, kc = k & 7;
+    const double p = __shfl_sync(0xffffffffu, a[kc], k + 16 * kh);
+    const double cik = __shfl_sync(0xffffffffu, a[kc], i + 16 * kh);
+    double rj[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) rj[c] = __shfl_sync(0xffffffffu, a[c], k + 16 * h);
+    if (CHOL) {
+      if (k < live && (!(p > 1e-300) || !isfinite(p))) bad = 1;
+      const double q = fabs(p) > 1e-300 ? fabs(p) : 1.0;
+      const double rk = rsqrt(q), li = cik * rk;
+      if (h == 0) Ls[k * kPbD + i] = i > k ? li : (i == k ? q * rk : 0.0);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const double r = (8 * h + c == k) ? rk : rj[c] * rk;
+        const double old = (8 * h + c == k) ? 0.0 : a[c];
+        if (i == k) a[c] = r;
+        else if (i > k) a[c] = fma(-li, r, old);
+      }
+    } else {
+      if (k < live && (!(fabs(p) > 1e-300) || !isfinite(p))) bad = 1;
+      const double ip = 1.0 / p;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const double r = (8 * h + c == k) ? ip : rj[c] * ip;
+        const double old = (8 * h + c == k) ? 0.0 : a[c];
+        a[c] = (i == k) ? r : fma(-cik, r, old);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) Di[i * kPbD + 8 * h + c] = (CHOL && 8 * h + c > i) ? 0.0 : a[c];
+}
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// sym (always with CHOL): the block is taken from its lower triangle (mirrored), so
+// that the inverse of a symmetric elimination stays consistent when the input carries
+// an asymmetric rounding error.
+template <bool CHOL>
+__global__ void __launch_bounds__(kPbThreads, 1)
+    k_pivot_block(const SweepDesc* __restrict__ descs, const int* __restrict__ active, int k0,
+                  double* __restrict__ dinv, int* __restrict__ status, int sym) {
+  constexpr int NBLK = kSweepNB / kPbW;
   const int di = active[blockIdx.x];
   const SweepDesc d = descs[di];
   const int nb = min(kSweepNB, d.r - k0);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  __shared__ double rowk[2][kSweepNB], colk[2][kSweepNB];
-  extern __shared__ double dg_sm[];  // kSweepNB x kSweepNB staging (coalesced load / store)
-  // sym: the block is taken from its lower triangle (mirrored), so that the
-  // inverse of a symmetric elimination stays consistent when the input carries
-  // an asymmetric rounding error
-  for (int e = threadIdx.x; e < kSweepNB * kSweepNB; e += blockDim.x) {
-    const int i = e & (kSweepNB - 1), j = e / kSweepNB;
-    const int ii = (sym && i < j) ? j : i, jj = (sym && i < j) ? i : j;
-    dg_sm[e] = (i < nb && j < nb) ? d.B[(k0 + ii) + (long long)(k0 + jj) * d.n] : 0.0;
+  extern __shared__ double pb_sm[];
+  double* St = pb_sm;                      // [col][row], staging
+  double* Rowp = St + kSweepNB * kPbSt;    // [k][col]: rows K
+  double* Colp = Rowp + kPbW * kPbLd;      // [k][row]: columns K (Gauss-Jordan: -C, I at K, even K)
+  double* Rn = Colp + kPbW * kPbLd;        // [k][col]: R
+  double* An = Rn + kPbW * kPbLd;          // [k][row]: Cholesky's -L_iK, I at K; else Colp of odd K
+  double* Dn = An + kPbW * kPbLd;          // the next diagonal block
+  double* Di = Dn + kPbW * kPbD;           // its inverse
+  double* Ls = Di + kPbW * kPbD;           // 2 x its Cholesky factor, [k][row]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  {
+    const double* Bk = d.B + k0 + (long long)k0 * d.n;
+#pragma unroll 8
+    for (int e = tid; e < kSweepNB * kSweepNB; e += kPbThreads) {
+      const int i = e & (kSweepNB - 1), j = e / kSweepNB;
+      const int ii = (sym && i < j) ? j : i, jj = (sym && i < j) ? i : j;
+      // past nb: the identity, which the elimination leaves alone
+      St[i + j * kPbSt] =
+          (i < nb && j < nb) ? Bk[ii + (long long)jj * d.n] : (i == j ? 1.0 : 0.0);
+    }
   }
   __syncthreads();
-  double a[4][8];
+  if (warp == 16) {
+    // the 16 x 16 pivots
+    int bad = 0;
+    for (int e = lane; e < kPbW * kPbW; e += 32)
+      Dn[(e & 15) * kPbD + (e >> 4)] = St[(e & 15) + (e >> 4) * kPbSt];
+    __syncwarp();
+    pivot16<CHOL>(Dn, Di, Ls, nb, bad);
+    for (int kb = 0; kb < NBLK; ++kb) {
+      bar_sync(1, kPbThreads);
+      if (kb + 1 == NBLK) break;
+      bar_sync(3, 64);
+      pivot16<CHOL>(Dn, Di, Ls + ((kb + 1) & 1) * kPbW * kPbD, nb - (kb + 1) * kPbW, bad);
+    }
+    if (bad) atomicOr(status, kStatusTinyPivot);
+  } else {
+    const int wr = warp & 3, wc = warp >> 2, wm = wr * 32, wn = wc * 32;
+    double acc[4][4][2];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) a[r][c] = dg_sm[(4 * ty + r) + (8 * tx + c) * kSweepNB];
-  int bad = 0;
-  for (int k = 0; k < nb; ++k) {
-    const int buf = k & 1;
-    if (ty == (k >> 2)) {
-      const int kr = k & 3;
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        double v = a[0][c];
+        for (int c = 0; c < 2; ++c)
+          acc[a][b][c] = St[(wm + a * 8 + gq) + (wn + b * 8 + tq * 2 + c) * kPbSt];
+    auto step = [&](auto par_, int kb) {
+      constexpr int P = decltype(par_)::value;  // kb & 1: the K rows are MMA tiles 2P, 2P + 1
+      const int K = kb * kPbW;
+      // Gauss-Jordan reads the column panel through the update, so it alternates with
+      // the buffer that holds -L_iK in the Cholesky form
+      double* Cp = (!CHOL && P) ? An : Colp;
+      if (wr == kb >> 1 && (!CHOL || wc <= wr)) {
 #pragma unroll
-        for (int r = 1; r < 4; ++r)
-          if (r == kr) v = a[r][c];
-        rowk[buf][8 * tx + c] = v;
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+              Rowp[(a * 8 + gq) * kPbLd + wn + b * 8 + tq * 2 + c] = acc[2 * P + a][b][c];
       }
-    }
-    if (tx == (k >> 3)) {
-      const int kc = k & 7;
+      if (wc == kb >> 1 && (!CHOL || wc <= wr)) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        double v = a[r][0];
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int c = 1; c < 8; ++c)
-          if (c == kc) v = a[r][c];
-        colk[buf][4 * ty + r] = v;
+          for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const int i = wm + a * 8 + gq, k = b * 8 + tq * 2 + c;
+              const double v = acc[a][2 * P + b][c];
+              Cp[k * kPbLd + i] =
+                  CHOL ? v : ((unsigned)(i - K) < kPbW ? (i - K == k ? 1.0 : 0.0) : -v);
+            }
       }
-    }
-    __syncthreads();
-    const double p = rowk[buf][k];
-    if (threadIdx.x == 0 && (!(fabs(p) > 1e-300) || !isfinite(p))) bad = 1;
-    const double ip = 1.0 / p;
-    double rj[8];
+      // rows and columns K are replaced (Cholesky keeps columns K of the rows above)
+      if (wr == kb >> 1) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) rj[c] = rowk[buf][8 * tx + c] * ip;
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const double cir = colk[buf][4 * ty + r];
+          for (int b = 0; b < 4; ++b) acc[2 * P + a][b][0] = acc[2 * P + a][b][1] = 0.0;
+      }
+      if (wc == kb >> 1) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) a[r][c] = fma(-cir, rj[c], a[r][c]);
-    }
-    // row k, column k and the pivot replace what the general update wrote there
-    if (ty == (k >> 2)) {
-      const int kr = k & 3;
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (r == kr) {
+          for (int b = 0; b < 2; ++b)
+            if (!CHOL || wm + a * 8 >= K) acc[a][2 * P + b][0] = acc[a][2 * P + b][1] = 0.0;
+      }
+      bar_sync(1, kPbThreads);
+      // R, 8 columns a warp
+      {
+        const int j0 = warp * 8;
+        const bool own = (unsigned)(j0 - K) < kPbW;
+        const double* src = (CHOL && j0 > K) ? Cp : Rowp;
+        double r[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        if (own) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) a[r][c] = rj[c];
+          for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+              r[a][c] = Di[(a * 8 + gq) * kPbD + (j0 - K) + tq * 2 + c];
+        } else {
+#pragma unroll
+          for (int k4 = 0; k4 < kPbW; k4 += 4) {
+            const double b = src[(k4 + tq) * kPbLd + j0 + gq];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) dmma(r[a], Di[(a * 8 + gq) * kPbD + k4 + tq], b);
+          }
         }
-    }
-    if (tx == (k >> 3)) {
-      const int kc = k & 7;
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (c == kc) {
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-            a[r][c] = (4 * ty + r == k) ? ip : colk[buf][4 * ty + r] * -ip;
+          for (int c = 0; c < 2; ++c) {
+            const int k = a * 8 + gq, j = j0 + tq * 2 + c;
+            Rn[k * kPbLd + j] = r[a][c];
+            if (CHOL) An[k * kPbLd + j] = own ? (j - K == k ? 1.0 : 0.0) : (j > K ? -r[a][c] : 0.0);
+          }
+      }
+      bar_sync(2, 512);
+      // A += An R, the quadrant that holds the next diagonal block first
+      const double* Aop = CHOL ? An : Cp;
+      const bool run = !CHOL || (wc <= wr && wm + 32 > K);
+      if (run) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int qa = (q & 1) ? P : 1 - P, qb = (q & 2) ? P : 1 - P;
+#pragma unroll
+          for (int k4 = 0; k4 < kPbW; k4 += 4) {
+            double af[2], bf[2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+              af[a] = Aop[(k4 + tq) * kPbLd + wm + (2 * qa + a) * 8 + gq];
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+              bf[b] = Rn[(k4 + tq) * kPbLd + wn + (2 * qb + b) * 8 + gq];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) dmma(acc[2 * qa + a][2 * qb + b], af[a], bf[b]);
+          }
+          if (q == 0 && kb + 1 < NBLK && wr == wc && wr == (kb + 1) >> 1) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                  Dn[(a * 8 + gq) * kPbD + b * 8 + tq * 2 + c] =
+                      acc[2 * qa + a][2 * qb + b][c];
+            bar_arrive(3, 64);
+          }
         }
+      }
+      if (CHOL) {
+        // columns K of L: zeros above, l, L_iK
+        const double* L = Ls + (kb & 1) * kPbW * kPbD;
+        for (int e = tid; e < kPbW * kSweepNB; e += 512) {
+          const int i = e & (kSweepNB - 1), k = e / kSweepNB, r = i - K;
+          if (i < nb && K + k < nb)
+            d.B[(k0 + i) + (long long)(k0 + K + k) * d.n] =
+                r < 0 ? 0.0 : (r < kPbW ? L[k * kPbD + r] : Rn[k * kPbLd + i]);
+        }
+      }
+    };
+    for (int kb = 0; kb < NBLK; kb += 2) {
+      step(std::integral_constant<int, 0>{}, kb);
+      step(std::integral_constant<int, 1>{}, kb + 1);
     }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          St[(wm + a * 8 + gq) + (wn + b * 8 + tq * 2 + c) * kPbSt] = acc[a][b][c];
   }
-  if (bad) atomicOr(status, kStatusTinyPivot);
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) dg_sm[(4 * ty + r) + (8 * tx + c) * kSweepNB] = a[r][c];
   __syncthreads();
   double* out = dinv + (long long)di * kSweepNB * kSweepNB;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+  for (int e = tid; e < nb * nb; e += kPbThreads) {
     const int i = e % nb, j = e / nb;
-    out[e] = dg_sm[i + j * kSweepNB];
+    out[e] = (CHOL && i < j) ? 0.0 : St[i + j * kPbSt];
   }
 }
 
 void launch_sweep_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
                        double* d_dinv, int* d_status, cudaStream_t s, int sym) {
   if (nact <= 0) return;
-  const int smem = kSweepNB * kSweepNB * (int)sizeof(double);
-  ensure_smem((const void*)k_sweep_diag, smem);
-  k_sweep_diag<<<nact, 512, smem, s>>>(d_desc, d_active, k0, d_dinv, d_status, sym);
+  ensure_smem((const void*)k_pivot_block<false>, kPbSmem);
+  k_pivot_block<false><<<nact, kPbThreads, kPbSmem, s>>>(d_desc, d_active, k0, d_dinv, d_status,
+                                                         sym);
+}
+
+void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
+                      double* d_dinv, int* d_status, cudaStream_t s) {
+  if (nact <= 0) return;
+  ensure_smem((const void*)k_pivot_block<true>, kPbSmem);
+  k_pivot_block<true><<<nact, kPbThreads, kPbSmem, s>>>(d_desc, d_active, k0, d_dinv, d_status,
+                                                        1);
 }
 
 __global__ void k_sweep_setdiag(const SweepDesc* __restrict__ descs,
@@ -1618,240 +1800,6 @@ void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status
   const size_t smem = (size_t)max_n * max_n * sizeof(double);
   ensure_smem((const void*)k_chol_small, kSmallSweepN * kSmallSweepN * sizeof(double));
   k_chol_small<<<nd, 256, smem, s>>>(d_desc, d_status);
-}
-
-// Pivot block of the blocked Cholesky: L_KK = chol(D) over B[K, K] (zeros
-// above the diagonal) and L_KK^{-1} into dinv, with D (128 x 128, lower
-// triangle read, padded with the identity past nb) in shared memory. This
-// kernel is on the critical path of the top levels, where one or a few blocks
-// remain, so it is built for latency: the only serial work is the pivot chain
-// of each 32-wide panel.
-//   for each panel p: warp 0 factors the 32 x 32 diagonal block with its rows
-//   in registers (pivot and multipliers passed by shuffles; one reciprocal
-//   square root per pivot, kept for the rest); the rows below are solved
-//   against it by forward substitution, a thread per row; the trailing lower
-//   triangle is updated with each thread holding a 16-strided micro-tile of
-//   the outputs in registers (rows tx + 16a, columns ty + 16b), so that a
-//   warp's loads are 16 consecutive doubles or broadcasts;
-//   then the four 32 x 32 diagonal inverses, one warp each, and L^{-1} in
-//   place, block row ib by block row: for every block column jb < ib at once,
-//   Tb = L(ib, jb:ib) X(jb:ib, jb), then X(ib, jb) = -X_ib Tb.
-constexpr int kCdP = 32;             // panel width
-constexpr int kCdXs = kCdP + 1;      // padded stride of the diagonal inverses
-constexpr int kCdThreads = 256;
-constexpr size_t kCholDiagSmem =
-    (size_t)(kSweepNB * kSweepNB + 4 * kCdP * kCdXs + 3 * kCdP * kCdXs + kSweepNB + 2 * kCdP) *
-    sizeof(double);
-static_assert(kSweepNB == 4 * kCdP && kCdThreads == 256, "16 x 16 thread grid over 32-row panels");
-
-__global__ void __launch_bounds__(kCdThreads) k_chol_diag(const SweepDesc* __restrict__ descs,
-                                                          const int* __restrict__ active, int k0,
-                                                          double* __restrict__ dinv,
-                                                          int* __restrict__ status) {
-  const int di = active[blockIdx.x];
-  const SweepDesc d = descs[di];
-  const int nb = min(kSweepNB, d.r - k0);
-  constexpr int T = kSweepNB;  // tile edge; column-major S[i + j T]
-  extern __shared__ double cd_sm[];
-  double* S = cd_sm;
-  double* Xd = S + T * T;              // 4 diagonal inverses, [p][c][i] = X_pp(i, c)
-  double* Tb = Xd + 4 * kCdP * kCdXs;  // 3 products of the inverse, [jb][c][k]
-  double* rd = Tb + 3 * kCdP * kCdXs;  // 1 / L(i, i)
-  double* colk = rd + T;               // 2 x 32: the current pivot column, double-buffered
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tx = tid & 15, ty = tid >> 4;
-  // the lower triangle only (the only one read), in whole columns; 16 loads
-  // of a thread in flight at once
-  {
-    const double* Bk = d.B + k0 + (long long)k0 * d.n;
-#pragma unroll 1
-    for (int base = 0; base < T * T; base += kCdThreads * 16) {
-      double v[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int e = base + u * kCdThreads + tid, i = e % T, j = e / T;
-        v[u] = (i < nb && j < nb) ? (i >= j ? Bk[i + (long long)j * d.n] : 0.0)
-                                  : (i == j ? 1.0 : 0.0);
-      }
-#pragma unroll
-      for (int u = 0; u < 16; ++u) S[base + u * kCdThreads + tid] = v[u];
-    }
-  }
-  __syncthreads();
-  int bad = 0;
-  for (int p = 0; p < T / kCdP; ++p) {
-    const int o = p * kCdP;
-    if (warp == 0) {
-      // Cholesky of the 32 x 32 diagonal block: lane = row, a[j] = D(lane, j)
-      double a[kCdP];
-#pragma unroll
-      for (int j = 0; j < kCdP; ++j) a[j] = S[(o + lane) + (o + j) * T];
-      double rmine = 1.0;  // 1 / L(lane, lane)
-#pragma unroll
-      for (int k = 0; k < kCdP; ++k) {
-        const double pv = __shfl_sync(0xffffffffu, a[k], k);
-        if (lane == 0 && o + k < nb && (!(pv > 1e-300) || !isfinite(pv))) bad = 1;
-        const double q = fabs(pv) > 1e-300 ? fabs(pv) : 1.0;
-        const double rk = rsqrt(q);
-        if (lane > k) a[k] *= rk;
-        if (lane == k) {
-          a[k] = q * rk;
-          rmine = rk;
-        }
-        // D(lane, j) -= L(lane, k) L(j, k), k < j <= lane; the column L(:, k) is
-        // passed through shared memory (one store per lane, broadcast loads)
-        // rather than by a pair of shuffles per entry; the buffer alternates
-        // with k, so one warp barrier per pivot suffices
-        double* ck = colk + (k & 1) * kCdP;
-        ck[lane] = a[k];
-        __syncwarp();
-#pragma unroll
-        for (int j = 1; j < kCdP; ++j) {
-          if (j > k) {  // fixed trip count: a[] stays in registers
-            const double ljk = ck[j];
-            if (lane >= j) a[j] = fma(-a[k], ljk, a[j]);
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kCdP; ++j) S[(o + lane) + (o + j) * T] = a[j];
-      rd[o + lane] = rmine;
-    }
-    __syncthreads();
-    const int r0 = o + kCdP, nrow = T - r0;
-    if (nrow > 0) {
-      // panel rows below, a thread per row: L(i, c) = (A(i, c) - sum_{k<c} L(i, k) L(c, k)) / L(c, c)
-      if (tid < nrow) {
-        const int i = r0 + tid;
-        double l[kCdP];
-#pragma unroll
-        for (int c = 0; c < kCdP; ++c) l[c] = S[i + (o + c) * T];
-#pragma unroll
-        for (int c = 0; c < kCdP; ++c) {
-          double acc = l[c];
-#pragma unroll
-          for (int k = 0; k < kCdP - 1; ++k)
-            if (k < c) acc = fma(-l[k], S[(o + c) + (o + k) * T], acc);
-          l[c] = acc * rd[o + c];
-        }
-#pragma unroll
-        for (int c = 0; c < kCdP; ++c) S[i + (o + c) * T] = l[c];
-      }
-      __syncthreads();
-      // trailing lower triangle: A(i, j) -= sum_k L(i, k) L(j, k)
-      const int na = nrow / 16;  // 6, 4 or 2 row strides
-      double t[6][6];
-#pragma unroll
-      for (int a = 0; a < 6; ++a)
-#pragma unroll
-        for (int b = 0; b < 6; ++b)
-          t[a][b] = (a < na && b < na) ? S[(r0 + tx + 16 * a) + (r0 + ty + 16 * b) * T] : 0.0;
-#pragma unroll 2
-      for (int k = 0; k < kCdP; ++k) {
-        double li[6], lj[6];
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-          li[a] = a < na ? S[(r0 + tx + 16 * a) + (o + k) * T] : 0.0;
-          lj[a] = a < na ? S[(r0 + ty + 16 * a) + (o + k) * T] : 0.0;
-        }
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-          for (int b = 0; b < 6; ++b)
-            if (a < na && b < na) t[a][b] = fma(-li[a], lj[b], t[a][b]);
-      }
-#pragma unroll
-      for (int a = 0; a < 6; ++a)
-#pragma unroll
-        for (int b = 0; b < 6; ++b)
-          if (a < na && b < na && tx + 16 * a >= ty + 16 * b)
-            S[(r0 + tx + 16 * a) + (r0 + ty + 16 * b) * T] = t[a][b];
-      __syncthreads();
-    }
-  }
-  if (bad) atomicOr(status, kStatusTinyPivot);
-  // L over B[K, K]: warp per column
-  for (int j = warp; j < nb; j += kCdThreads / 32)
-    for (int i = lane; i < nb; i += 32)
-      d.B[(k0 + i) + (long long)(k0 + j) * d.n] = (i >= j) ? S[i + j * T] : 0.0;
-  // the diagonal inverses, warp p for block p, lane = column c:
-  // X(c, c) = 1 / l_cc, X(i, c) = -(sum_{k=c}^{i-1} l_ik X(k, c)) / l_ii, zero above
-  if (warp < T / kCdP) {
-    const int o = warp * kCdP, c = lane;
-    double x[kCdP];
-#pragma unroll
-    for (int i = 0; i < kCdP; ++i) {
-      double acc = 0.0;
-#pragma unroll
-      for (int k = 0; k < kCdP - 1; ++k)
-        if (k < i) acc = fma(S[(o + i) + (o + k) * T], x[k], acc);
-      x[i] = i == c ? rd[o + i] : (i > c ? -acc * rd[o + i] : 0.0);
-    }
-    double* X = Xd + warp * kCdP * kCdXs;
-#pragma unroll
-    for (int i = 0; i < kCdP; ++i) X[c * kCdXs + i] = x[i];
-  }
-  __syncthreads();
-  // L^{-1} in place: the diagonal blocks first (X_jj, zeros above)
-  for (int e = tid; e < 4 * kCdP * kCdP; e += blockDim.x) {
-    const int jb = e / (kCdP * kCdP), r = e % (kCdP * kCdP), i = r % kCdP, c = r / kCdP;
-    S[(jb * kCdP + i) + (jb * kCdP + c) * T] = Xd[jb * kCdP * kCdXs + c * kCdXs + i];
-  }
-  __syncthreads();
-  for (int ib = 1; ib < T / kCdP; ++ib) {
-    const int oi = ib * kCdP;
-    // Tb[jb](i, c) = sum_{k in [jb 32, oi)} L(oi + i, k) X(k, jb 32 + c)
-    for (int jb = 0; jb < ib; ++jb) {
-      const int oj = jb * kCdP;
-      double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll 4
-      for (int k = oj; k < oi; ++k) {
-        const double l0 = S[(oi + tx) + k * T], l1 = S[(oi + tx + 16) + k * T];
-        const double x0 = S[k + (oj + ty) * T], x1 = S[k + (oj + ty + 16) * T];
-        acc[0][0] = fma(l0, x0, acc[0][0]);
-        acc[0][1] = fma(l0, x1, acc[0][1]);
-        acc[1][0] = fma(l1, x0, acc[1][0]);
-        acc[1][1] = fma(l1, x1, acc[1][1]);
-      }
-      double* Tj = Tb + jb * kCdP * kCdXs;
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) Tj[(ty + 16 * b) * kCdXs + tx + 16 * a] = acc[a][b];
-    }
-    __syncthreads();
-    // X(ib, jb) = -X_ib Tb[jb]
-    const double* Xi = Xd + ib * kCdP * kCdXs;
-    for (int jb = 0; jb < ib; ++jb) {
-      const int oj = jb * kCdP;
-      const double* Tj = Tb + jb * kCdP * kCdXs;
-      double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll 4
-      for (int k = 0; k < kCdP; ++k) {
-        const double x0 = Xi[k * kCdXs + tx], x1 = Xi[k * kCdXs + tx + 16];
-        const double t0 = Tj[ty * kCdXs + k], t1 = Tj[(ty + 16) * kCdXs + k];
-        acc[0][0] = fma(x0, t0, acc[0][0]);
-        acc[0][1] = fma(x0, t1, acc[0][1]);
-        acc[1][0] = fma(x1, t0, acc[1][0]);
-        acc[1][1] = fma(x1, t1, acc[1][1]);
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) S[(oi + tx + 16 * a) + (oj + ty + 16 * b) * T] = -acc[a][b];
-    }
-    __syncthreads();
-  }
-  double* out = dinv + (long long)di * kSweepNB * kSweepNB;
-  for (int j = warp; j < nb; j += kCdThreads / 32)
-    for (int i = lane; i < nb; i += 32) out[i + j * nb] = (i >= j) ? S[i + j * T] : 0.0;
-}
-
-void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
-                      double* d_dinv, int* d_status, cudaStream_t s) {
-  if (nact <= 0) return;
-  ensure_smem((const void*)k_chol_diag, kCholDiagSmem);
-  k_chol_diag<<<nact, kCdThreads, kCholDiagSmem, s>>>(d_desc, d_active, k0, d_dinv, d_status);
 }
 
 // ===========================================================================
