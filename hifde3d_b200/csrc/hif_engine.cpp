@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <functional>
 #include <chrono>
 #include <climits>
@@ -444,13 +445,16 @@ struct ApplyLaunch {
   GemvDesc* d_desc = nullptr;
   int nd = 0;
   int in_vec = 0, out_vec = 0;  // 0 = ua, 1 = ub, 2 = uc (Cholesky phases' L^{-1} u_r)
-  // GEMV layout (launch_gemv_fast) and its unit table; the serving loop binds
-  // the descriptors to a request's vectors and reuses the table
-  int layout = 0;
-  int2* d_tab = nullptr;
-  int units = 0;
-  GemvFastSeg* d_seg = nullptr;  // one segment: this launch's descriptors and table
-  int* d_segoff = nullptr;
+  // Layout (launch_gemv), unit table and the launch's one segment, for one vector [0]
+  // and for several [1] (built on the first such apply). The serving loop binds the
+  // descriptors to a request's vectors and reuses the tables.
+  struct Form {
+    GemvLayout lay;
+    int4* d_tab = nullptr;
+    int units = 0;
+    GemvFastSeg* d_seg = nullptr;
+    int* d_segoff = nullptr;
+  } form[2];
   int* d_dof = nullptr;
   int* d_off = nullptr;
   int* d_slot = nullptr;
@@ -461,7 +465,7 @@ struct ApplyLaunch {
 struct ApplyPlan {
   std::vector<ApplyLaunch> launches;
   BufList bufs;
-  long long contrib_slots = 0;
+  bool multi = false;  // the several-vector tables are built
 };
 
 // Live Schur complement blocks feeding the next phase.
@@ -1642,131 +1646,6 @@ class Engine {
   void drop_graphs() {
     for (auto& kv : apply_graphs) cudaGraphExecDestroy(kv.second);
     apply_graphs.clear();
-    for (auto& kv : gemm_plans) kv.second.bufs.release(stream);
-    gemm_plans.clear();
-  }
-
-  // ---- apply for many right-hand sides: every GEMV launch of a plan as gather /
-  // GEMM / emit, so each factor matrix is read once per apply instead of once
-  // per 4 right-hand sides. Built per (direction, RHS count) from the plan's
-  // descriptors; launches only, so the sweep is still captured in a graph.
-  static constexpr int kGemmApplyMinRhs = 16;
-  struct GemmStage {
-    size_t launch = 0;  // plan launch (reduce-scatter launches are run as they are)
-    ApplyGatherDesc* d_gather = nullptr;
-    long long* d_goff = nullptr;
-    int ng = 0;
-    long long gtotal = 0;
-    GemmDesc* d_gemm = nullptr;
-    int* d_toff = nullptr;
-    int tiles = 0, tile = 64;
-    ApplyEmitDesc* d_emit = nullptr;
-    long long* d_eoff = nullptr;
-    long long etotal = 0;
-    double flops = 0;
-  };
-  struct GemmPlan {
-    std::vector<GemmStage> stages;
-    BufList bufs;
-  };
-  std::map<std::pair<int, int>, GemmPlan> gemm_plans;
-
-  GemmPlan& gemm_plan(ApplyPlan& plan, int inverse, int nrhs) {
-    const std::pair<int, int> key(inverse, nrhs);
-    auto it = gemm_plans.find(key);
-    if (it != gemm_plans.end()) return it->second;
-    GemmPlan gp;
-    long long xmax = 1, ymax = 1;
-    for (const ApplyLaunch& l : plan.launches) {
-      if (l.type != 0) continue;
-      long long xs = 0, ys = 0;
-      for (const GemvDesc& g : l.hdesc) {
-        xs += (long long)(g.trans ? g.m : g.n) * nrhs;
-        ys += (long long)(g.trans ? g.n : g.m) * nrhs;
-      }
-      xmax = std::max(xmax, xs);
-      ymax = std::max(ymax, ys);
-    }
-    double* xin = gp.bufs.add(dalloc<double>(xmax, stream));
-    double* yout = gp.bufs.add(dalloc<double>(ymax, stream));
-    for (size_t q = 0; q < plan.launches.size(); ++q) {
-      const ApplyLaunch& l = plan.launches[q];
-      GemmStage st;
-      st.launch = q;
-      if (l.type == 0) {
-        std::vector<ApplyGatherDesc> gd;
-        std::vector<ApplyEmitDesc> ed;
-        std::vector<GemmDesc> gm;
-        std::vector<long long> goff(1, 0), eoff(1, 0);
-        std::vector<int> toff(1, 0);
-        long long ox = 0, oy = 0;
-        const int tile = 64;
-        for (const GemvDesc& g : l.hdesc) {
-          const int len = g.trans ? g.m : g.n, rows = g.trans ? g.n : g.m;
-          gd.push_back(ApplyGatherDesc{g.in_idx, xin + ox, len});
-          goff.push_back(goff.back() + (long long)len * nrhs);
-          GemmDesc m{};
-          m.C = yout + oy;
-          m.ldc = rows;
-          m.A = g.M;
-          m.lda = g.ld;
-          m.transA = g.trans;
-          m.B = xin + ox;
-          m.ldb = len;
-          m.m = rows;
-          m.n = nrhs;
-          m.k = len;
-          m.alpha = 1.0;
-          m.beta = 0.0;
-          gm.push_back(m);
-          toff.push_back(toff.back() + dgemm_tiles(rows, nrhs, tile));
-          ed.push_back(ApplyEmitDesc{yout + oy, g.out_idx, g.contrib, rows, g.mode, g.alpha});
-          eoff.push_back(eoff.back() + (long long)rows * nrhs);
-          st.flops += 2.0 * rows * len * nrhs;
-          ox += (long long)len * nrhs;
-          oy += (long long)rows * nrhs;
-        }
-        st.d_gather = gp.bufs.add(upload(gd, stream));
-        st.d_goff = gp.bufs.add(upload(goff, stream));
-        st.ng = (int)gd.size();
-        st.gtotal = goff.back();
-        st.d_gemm = gp.bufs.add(upload(gm, stream));
-        st.d_toff = gp.bufs.add(upload(toff, stream));
-        st.tiles = toff.back();
-        st.tile = tile;
-        st.d_emit = gp.bufs.add(upload(ed, stream));
-        st.d_eoff = gp.bufs.add(upload(eoff, stream));
-        st.etotal = eoff.back();
-      }
-      gp.stages.push_back(st);
-    }
-    return gemm_plans.emplace(key, std::move(gp)).first->second;
-  }
-
-  void run_gemm_plan(ApplyPlan& plan, GemmPlan& gp, int nrhs) {
-    double* vec[3] = {d_ua, d_ub, d_uc};
-    for (GemmStage& st : gp.stages) {
-      ApplyLaunch& l = plan.launches[st.launch];
-      if (l.type == 0) {
-        timed(HIF_KCLASS_VECTOR, 0, 0, [&] {
-          launch_apply_gather(st.d_gather, st.d_goff, st.ng, st.gtotal, vec[l.in_vec], n3,
-                              stream);
-        });
-        timed(HIF_KCLASS_GEMV, st.flops, l.bytes, [&] {
-          launch_dgemm(st.d_gemm, st.d_toff, st.ng, st.tiles, stream, st.tile);
-        });
-        timed(HIF_KCLASS_VECTOR, 0, 0, [&] {
-          launch_apply_emit(st.d_emit, st.d_eoff, st.ng, st.etotal, vec[l.out_vec], n3,
-                            contrib_ld, stream);
-        });
-      } else {
-        timed(HIF_KCLASS_VECTOR, 0, 0, [&] {
-          launch_reduce_scatter(l.d_dof, l.d_off, l.d_slot, d_contrib, l.ndof, contrib_ld,
-                                l.alpha, vec[l.out_vec], nrhs, n3, stream);
-        });
-      }
-      HIF_CK(cudaGetLastError());
-    }
   }
 
   void release_plans() {
@@ -1777,6 +1656,7 @@ class Engine {
     plan_fwd.bufs.release(stream);
     plan_inv.launches.clear();
     plan_fwd.launches.clear();
+    plan_inv.multi = plan_fwd.multi = false;
     plans_built = false;
   }
 
@@ -3677,7 +3557,7 @@ class Engine {
       g.tri = tri;
       g.alpha = alpha;
       g.mode = mode;
-      g.contrib = (mode == 1) ? d_contrib + st.o_skel[b] : nullptr;
+      g.cslot = (mode == 1) ? st.o_skel[b] : 0;
       mbytes += 8.0 * g.m * g.n;
       dd.push_back(g);
     }
@@ -3689,26 +3569,61 @@ class Engine {
     l.in_vec = in_vec;
     l.out_vec = out_vec;
     l.d_desc = plan.bufs.add(upload(dd, stream));
-    int big = 0;
-    for (const GemvDesc& g : dd) big = std::max(big, std::max(g.m, g.n));
-    if (big <= kGemvSmallMax) {
-      l.layout = kGemvSmall;
-      l.units = (int)dd.size();
-    } else {
-      l.layout = kGemvTiles;
-      std::vector<int2> tab;
-      for (size_t q = 0; q < dd.size(); ++q) {
-        const int nt = gemv_tile_count(dd[q].m, dd[q].n, trans);
-        for (int t = 0; t < nt; ++t) tab.push_back(make_int2((int)q, t));
-      }
-      l.units = (int)tab.size();
-      l.d_tab = plan.bufs.add(upload(tab, stream));
-    }
-    l.d_seg = plan.bufs.add(upload(std::vector<GemvFastSeg>{{l.d_desc, l.d_tab}}, stream));
-    l.d_segoff = plan.bufs.add(upload(std::vector<int>{0, l.units}, stream));
     l.hdesc = std::move(dd);
+    gemv_form(plan, l, 0, stream);
     l.key = my_key;
     plan.launches.push_back(std::move(l));
+  }
+
+  // Layout and unit table of a launch for one vector (multi 0) or several (1).
+  void gemv_form(ApplyPlan& plan, ApplyLaunch& l, int multi, cudaStream_t s) {
+    ApplyLaunch::Form& f = l.form[multi];
+    int big = 0, elems = 0;
+    for (const GemvDesc& g : l.hdesc) {
+      big = std::max(big, std::max(g.m, g.n));
+      elems = std::max(elems, g.m * g.n);
+    }
+    std::vector<int4> tab;
+    if (!multi && big <= kGemvSmallMax && elems <= kGemvSmallElems) {
+      f.lay.kind = kGemvSmall;
+      f.lay.elems = elems;
+      f.units = (int)l.hdesc.size();
+    } else {
+      const int w = multi ? 64 : 32;
+      long long tiles = 0, red = 0;
+      for (const GemvDesc& g : l.hdesc) {
+        const int out = g.trans ? g.n : g.m, len = g.trans ? g.m : g.n;
+        tiles += (out + w - 1) / w;
+        red = std::max<long long>(red, len);
+      }
+      // one vector: tiles of short reductions are taken several to a unit, about 96 KB
+      // of M each, as long as some 1500 units (three waves and more) remain
+      const long long most = multi ? 1 : std::max(1LL, tiles / 1500);
+      tab.reserve(tiles);
+      for (size_t q = 0; q < l.hdesc.size(); ++q) {
+        const GemvDesc& g = l.hdesc[q];
+        const int out = g.trans ? g.n : g.m, len = g.trans ? g.m : g.n, nt = (out + w - 1) / w;
+        const int per = (int)std::min<long long>(most, std::max(1, 98304 / (len * 32 * 8)));
+        for (int t = 0; t < nt; t += per)
+          tab.push_back(make_int4((int)q, t, std::min(per, nt - t), 0));
+      }
+      f.lay.kind = multi ? kGemvMulti : kGemvTiles;
+      f.units = (int)tab.size();
+      // few units: a cluster shares each, down to 128 entries of the reduction a CTA
+      while (f.lay.cluster < 8 && (long long)f.units * f.lay.cluster < 600 &&
+             red >= 256LL * f.lay.cluster)
+        f.lay.cluster *= 2;
+      f.d_tab = plan.bufs.add(upload(tab, s));
+    }
+    f.d_seg = plan.bufs.add(upload(std::vector<GemvFastSeg>{{l.d_desc, f.d_tab}}, s));
+    f.d_segoff = plan.bufs.add(upload(std::vector<int>{0, f.units}, s));
+  }
+  // The several-vector tables of a plan, on first use.
+  void ensure_multi(ApplyPlan& plan, cudaStream_t s) {
+    if (plan.multi) return;
+    for (ApplyLaunch& l : plan.launches)
+      if (l.type == 0) gemv_form(plan, l, 1, s);
+    plan.multi = true;
   }
 
   // A22 = L L^T, A22^{-1} = L^{-T} L^{-1} or X = L^{-T} Y (which 0 / 1 / 2) of
@@ -3880,19 +3795,15 @@ class Engine {
   }
 
   // Contribution buffer: max over phases of the skeleton slots, times the
-  // right-hand-side capacity; GEMV descriptors point into it directly.
+  // right-hand-side capacity.
   long long contrib_ld = 1;
   int contrib_cap = 0;
 
-  void build_plans(int nrhs_cap) {
+  void build_plans() {
     release_plans();
     long long max_slots = 1;
     for (const StepData& st : steps) max_slots = std::max(max_slots, st.n_skel);
     contrib_ld = max_slots;
-    dfree(d_contrib, stream);
-    d_contrib = dalloc<double>(max_slots * nrhs_cap, stream);
-    contrib_cap = nrhs_cap;
-    plan_inv.contrib_slots = plan_fwd.contrib_slots = max_slots;
     // index steps by (level, kind)
     std::vector<const StepData*> sch(L, nullptr), skl(L, nullptr);
     for (const StepData& st : steps) (st.skel ? skl : sch)[st.level] = &st;
@@ -4031,7 +3942,13 @@ class Engine {
   }
 
   void ensure_workspace(int nrhs) {
-    if (!plans_built || contrib_cap < nrhs) build_plans(std::max(nrhs, contrib_cap));
+    if (!plans_built) build_plans();
+    if (contrib_cap < nrhs || !d_contrib) {
+      drop_graphs();
+      dfree(d_contrib, stream);
+      d_contrib = dalloc<double>(contrib_ld * nrhs, stream);
+      contrib_cap = nrhs;
+    }
     if (ws_nrhs >= nrhs && d_ua) return;
     drop_graphs();
     dfree(d_ua, stream);
@@ -4047,15 +3964,16 @@ class Engine {
     double* vec[3] = {d_ua, d_ub, d_uc};
     for (ApplyLaunch& l : plan.launches) {
       if (l.type == 0) {
-        const double by = l.bytes * ((nrhs + 3) / 4);
+        const ApplyLaunch::Form& f = l.form[nrhs > 1];
+        const double by = l.bytes * ((nrhs + 63) / 64);
         timed(HIF_KCLASS_GEMV, 2.0 * l.bytes / 8 * nrhs, by, [&] {
-          launch_gemv_fast(l.d_seg, l.d_segoff, 1, l.units, l.layout, vec[l.in_vec],
-                           vec[l.out_vec], nrhs, n3, contrib_ld, stream);
+          launch_gemv(f.d_seg, f.d_segoff, 1, f.units, f.lay, vec[l.in_vec], vec[l.out_vec],
+                      d_contrib, nrhs, stream);
         });
       } else {
         timed(HIF_KCLASS_VECTOR, 0, 0, [&] {
-          launch_reduce_scatter(l.d_dof, l.d_off, l.d_slot, d_contrib, l.ndof, contrib_ld,
-                                l.alpha, vec[l.out_vec], nrhs, n3, stream);
+          launch_reduce_scatter(l.d_dof, l.d_off, l.d_slot, d_contrib, l.ndof, l.alpha,
+                                vec[l.out_vec], nrhs, stream);
         });
       }
       HIF_CK(cudaGetLastError());
@@ -4063,23 +3981,21 @@ class Engine {
   }
 
   void apply_device(double* du, int nrhs, long long ldu, bool inverse) {
+    apply_device(du, ldu, du, ldu, nrhs, inverse);
+  }
+  // dst = F src or F^{-1} src (columns of right-hand sides; dst may be src)
+  void apply_device(const double* src, long long lds, double* dst, long long ldd, int nrhs,
+                    bool inverse) {
     if (!factored) throw Error{HIF_ERR_STATE, "Apply before Factor"};
-    if (nrhs <= 0 || ldu < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ldu"};
+    if (nrhs <= 0 || lds < n3 || ldd < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ldu"};
     ensure_workspace(nrhs);
-    for (int c = 0; c < nrhs; ++c)
-      HIF_CK(cudaMemcpyAsync(d_ua + c * n3, du + c * ldu, n3 * 8, cudaMemcpyDeviceToDevice,
-                             stream));
     ApplyPlan& plan = inverse ? plan_inv : plan_fwd;
-    GemmPlan* gp = nrhs >= kGemmApplyMinRhs ? &gemm_plan(plan, inverse ? 1 : 0, nrhs) : nullptr;
-    auto sweep = [&] {
-      timed(HIF_KCLASS_VECTOR, 0, 8.0 * n3 * nrhs,
-            [&] { launch_zero_boundary(d_ua, NC, nrhs, n3, stream); });
-      HIF_CK(cudaMemsetAsync(d_ub, 0, n3 * nrhs * 8, stream));
-      if (gp) run_gemm_plan(plan, *gp, nrhs);
-      else run_plan(plan, nrhs);
-    };
+    if (nrhs > 1) ensure_multi(plan, stream);
+    timed(HIF_KCLASS_VECTOR, 0, 24.0 * n3 * nrhs,
+          [&] { launch_apply_in(src, lds, d_ua, d_ub, NC, nrhs, stream); });
+    HIF_CK(cudaGetLastError());
     if (profile) {
-      sweep();  // per-launch events: no graph
+      run_plan(plan, nrhs);  // per-launch events: no graph
     } else {
       const std::pair<int, int> key(inverse ? 1 : 0, nrhs);
       auto it = apply_graphs.find(key);
@@ -4088,7 +4004,7 @@ class Engine {
         cudaGraphExec_t ge = nullptr;
         HIF_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
-          sweep();
+          run_plan(plan, nrhs);
         } catch (...) {
           cudaStreamEndCapture(stream, &g);
           if (g) cudaGraphDestroy(g);
@@ -4102,9 +4018,9 @@ class Engine {
       }
       HIF_CK(cudaGraphLaunch(it->second, stream));
     }
-    for (int c = 0; c < nrhs; ++c)
-      HIF_CK(cudaMemcpyAsync(du + c * ldu, d_ub + c * n3, n3 * 8, cudaMemcpyDeviceToDevice,
-                             stream));
+    timed(HIF_KCLASS_VECTOR, 0, 16.0 * n3 * nrhs,
+          [&] { launch_apply_out(d_ub, dst, ldd, n3, nrhs, stream); });
+    HIF_CK(cudaGetLastError());
   }
 
   // ---- PCG with the inverse apply as preconditioner -----------------------
@@ -4137,9 +4053,7 @@ class Engine {
     timed(HIF_KCLASS_VECTOR, 0, vb, [&] { launch_dot(r, r, n3, nrhs, n3, part, bb, stream); }, 2);
     // z = M r
     auto precond = [&](double* in, double* outv) {
-      if (outv != in)
-        HIF_CK(cudaMemcpyAsync(outv, in, n3 * nrhs * 8, cudaMemcpyDeviceToDevice, stream));
-      apply_device(outv, nrhs, n3, true);
+      apply_device(in, n3, outv, n3, nrhs, true);
     };
     precond(r, z);
     HIF_CK(cudaMemcpyAsync(p, z, n3 * nrhs * 8, cudaMemcpyDeviceToDevice, stream));

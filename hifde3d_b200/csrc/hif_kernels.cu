@@ -3294,255 +3294,515 @@ void launch_member_faces(const int* d_skel, const long long* d_off, const int* d
 }
 
 // ===========================================================================
-// Apply: batched gather - GEMV - scatter over right-hand sides.
-// trans = 0: 256 output rows per CTA, one row per thread (coalesced along M's
-//            columns); trans = 1: 32 output columns per CTA, one warp per
-//            column (coalesced down the column).
+// Apply sweeps: y = op(M) x[in] for every block of a phase, x and y through DOF lists.
+// The work vectors hold the right-hand sides of a DOF side by side (element (p, c) at
+// u[p * nrhs + c]; contribution slots likewise), so that a gather or scatter moves
+// whole rows of right-hand sides. One vector: streaming GEMVs, bound by reading the
+// factor once. Several: DMMA tiles over all of them, each factor entry read once per
+// 64. Every sum has a fixed order.
 // ===========================================================================
-constexpr int kRhsGroup = 4;
-constexpr int kXChunk = 256;
-
-
-__device__ __forceinline__ void gemv_emit(const GemvDesc& g, int i, int c, double y,
-                                          double* u_out, long long ldu, long long contrib_ld) {
-  if (g.mode == 1) g.contrib[i + (long long)c * contrib_ld] = y;
-  else if (g.mode == 0) u_out[g.out_idx[i] + (long long)c * ldu] += g.alpha * y;
-  else u_out[g.out_idx[i] + (long long)c * ldu] = g.alpha * y;
+struct GemvCtx {
+  const double* uin;
+  double* uout;
+  double* contrib;
+  int nrhs;
+};
+__device__ __forceinline__ GemvCtx gemv_ctx(const GemvDesc& g, const GemvCtx& k) {
+  return g.uin ? GemvCtx{g.uin, g.uout, g.contrib, g.nrhs} : k;
 }
 
-// RG right-hand sides per pass: 4, or 1 for single-vector launches (fewer
-// registers, so more CTAs and more loads in flight); a column of results is the
-// same sequence of operations either way.
-template <int RG>
-__device__ __forceinline__ void gemv_tile(const GemvDesc& g0, int local,
-                                          const double* __restrict__ u_in_k,
-                                          double* __restrict__ u_out_k, int nrhs_k,
-                                          long long ldu_k, long long contrib_ld_k) {
-  GemvDesc g = g0;
-  const double* u_in = g.uin ? g.uin : u_in_k;
-  double* u_out = g.uin ? g.uout : u_out_k;
-  const int nrhs = g.uin ? g.nrhs : nrhs_k;
-  const long long ldu = g.uin ? g.ldu : ldu_k;
-  const long long contrib_ld = g.uin ? g.cld : contrib_ld_k;
-  __shared__ double xs[kXChunk][RG];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if constexpr (RG == 1) {
-    // one vector: x is read where it is used (a broadcast load per column or
-    // row) instead of being staged per chunk, so no barrier interrupts the
-    // stream of M; the columns of each warp and the order of every sum are
-    // those of the staged form, so the results are the same bit for bit
+__device__ __forceinline__ void gemv_emit(const GemvDesc& g, const GemvCtx& x, int i, int c,
+                                          double y) {
+  if (g.mode == 1) {
+    x.contrib[(g.cslot + i) * x.nrhs + c] = y;
+  } else {
+    double* u = x.uout + (long long)g.out_idx[i] * x.nrhs + c;
+    *u = g.mode == 0 ? *u + g.alpha * y : g.alpha * y;
+  }
+}
+
+// One vector, blocks of at most kGemvSmallElems entries, a warp each: the whole block
+// and its x go to shared memory first, every load independent of the others (a warp
+// that loads an index, then x, then a column at a time waits for each: 0.9 TB/s on
+// level 0's 27 x 54 blocks), then lane = output.
+__global__ void __launch_bounds__(256) k_gemv_small(const GemvFastSeg* __restrict__ segs,
+                                                    const int* __restrict__ seg_off, int nseg,
+                                                    GemvCtx k, int elems) {
+  extern __shared__ double gs_sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int unit = blockIdx.x * 8 + warp;
+  if (unit >= seg_off[nseg]) return;
+  const int si = nseg == 1 ? 0 : find_desc(seg_off, nseg, unit);
+  const GemvDesc g = segs[si].desc[unit - seg_off[si]];
+  const GemvCtx x = gemv_ctx(g, k);
+  double* S = gs_sm + warp * (elems + kGemvSmallMax);
+  double* xs = S + elems;
+  const int len = g.trans ? g.m : g.n, out = g.trans ? g.n : g.m, mn = g.m * g.n;
+  // ld == m: the block is contiguous
+  for (int e0 = 0; e0 < mn; e0 += 32 * 16) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int e = e0 + u * 32 + lane;
+      v[u] = e < mn ? __ldg(g.M + e) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int e = e0 + u * 32 + lane;
+      if (e < mn) S[e] = v[u];
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < kGemvSmallMax / 32; ++h) {
+    const int j = lane + 32 * h;
+    if (j < len) xs[j] = x.uin[g.in_idx[j]];
+  }
+  __syncwarp();
+  for (int i = lane; i < out; i += 32) {
+    double acc = 0.0;
     if (g.trans == 0) {
-      __shared__ double red1[8][32];
-      const int i = local * 32 + lane;
-      for (int c0 = 0; c0 < nrhs; ++c0) {
-        double acc = 0.0;
-        const int jend = g.tri ? min(g.n, (local + 1) * 32) : g.n;
-        for (int j0 = 0; j0 < jend; j0 += kXChunk) {
-          const int jb = warp * 32, cnt = min(32, min(kXChunk, jend - j0) - jb);
-          if (i < g.m && cnt > 0) {
-            const double* col = g.M + i + (long long)(j0 + jb) * g.ld;
-            const int* idx = g.in_idx + j0 + jb;
-            const double* x = u_in + (long long)c0 * ldu;
-#pragma unroll 16
-            for (int jj = 0; jj < cnt; ++jj)
-              acc = fma(col[(long long)jj * g.ld], x[idx[jj]], acc);
-          }
-        }
-        __syncthreads();  // the previous vector's sums have been read
-        red1[warp][lane] = acc;
-        __syncthreads();
-        if (warp == 0 && i < g.m) {
-          double y = red1[0][lane];
-#pragma unroll
-          for (int w = 1; w < 8; ++w) y += red1[w][lane];
-          gemv_emit(g, i, c0, y, u_out, ldu, contrib_ld);
-        }
-      }
+      const int jend = g.tri ? min(g.n, i + 1) : g.n;
+#pragma unroll 8
+      for (int j = 0; j < jend; ++j) acc = fma(S[i + j * g.m], xs[j], acc);
     } else {
-      const int jw = local * 32 + warp * 4;
-      const int ibeg = g.tri ? ((local * 32) / kXChunk) * kXChunk : 0;
-      for (int c0 = 0; c0 < nrhs; ++c0) {
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        const double* x = u_in + (long long)c0 * ldu;
-        for (int i0 = ibeg; i0 < g.m; i0 += kXChunk) {
-          const int ni = min(kXChunk, g.m - i0);
-#pragma unroll 2
-          for (int ii = lane; ii < ni; ii += 32) {
-            const double xv = x[g.in_idx[i0 + ii]];
+      const int r0 = g.tri ? i : 0;
+#pragma unroll 8
+      for (int r = r0; r < g.m; ++r) acc = fma(S[r + i * g.m], xs[r], acc);
+    }
+    gemv_emit(g, x, i, 0, acc);
+  }
+}
+
+// One vector, larger blocks: a unit is a run of 32-wide tiles of outputs of one block.
+// y = M x: lane = row, the columns of a chunk split over the 8 warps; y = M^T x: a
+// warp's four columns at each row. x goes to shared memory in chunks (kept from tile
+// to tile where one chunk is all of it) after the first 16 entries of M a thread needs
+// have been requested, so the two gathers and the stream of M overlap. Where a launch
+// has few units, a cluster of CTAs shares each and adds its parts in rank order
+// through distributed shared memory: the top levels' blocks, 82 tiles of 2612 columns
+// at n = 96, else leave half the SMs idle and the others latency-bound (1.8 TB/s).
+constexpr int kG1Chunk = 1024;
+__global__ void __launch_bounds__(256, 3) k_gemv1(const GemvFastSeg* __restrict__ segs,
+                                                  const int* __restrict__ seg_off, int nseg,
+                                                  GemvCtx k) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  __shared__ double xs[kG1Chunk];
+  __shared__ double red[8][33];
+  __shared__ double part[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int unit = blockIdx.x / C;
+  const int si = nseg == 1 ? 0 : find_desc(seg_off, nseg, unit);
+  const int4 t = segs[si].tab[unit - seg_off[si]];
+  const GemvDesc g = segs[si].desc[t.x];
+  const GemvCtx x = gemv_ctx(g, k);
+  const int len = g.trans ? g.m : g.n, out = g.trans ? g.n : g.m;
+  int held0 = -1, held1 = -1;  // range of x in xs
+  for (int tile = t.y; tile < t.y + t.z; ++tile) {
+    const int o0 = tile * 32;
+    // lower triangular: a strip of rows needs no column past its last row, a tile of
+    // columns no row before its first
+    const int lo = (g.tri && g.trans) ? o0 : 0, hi = (g.tri && !g.trans) ? min(len, o0 + 32) : len;
+    const int per = (((hi - lo + C - 1) / C) + 31) & ~31;
+    const int a = lo + rank * per, b = min(hi, a + per);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int c0 = a; c0 < b; c0 += kG1Chunk) {
+      const int nj = min(kG1Chunk, b - c0);
+      const bool stage = c0 != held0 || c0 + nj != held1;
+      // first loads of M, then x
+      double v[16];
+      const double* Mp;
+      int j0, j1;  // columns of this warp in the chunk (y = M x)
+      if (g.trans == 0) {
+        const int cnt = (nj + 7) / 8;
+        j0 = warp * cnt;
+        j1 = min(nj, j0 + cnt);
+        Mp = g.M + min(o0 + lane, g.m - 1) + (long long)c0 * g.ld;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const double mv = jw + q < g.n ? g.M[(long long)(jw + q) * g.ld + i0 + ii] : 0.0;
-              acc[q] = fma(mv, xv, acc[q]);
-            }
-          }
-        }
+        for (int u = 0; u < 16; ++u)
+          v[u] = j0 + u < j1 ? __ldg(Mp + (long long)(j0 + u) * g.ld) : 0.0;
+      } else {
+        j0 = j1 = 0;
+        Mp = g.M + c0 + lane;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const double y = warp_sum(acc[q]);
-          if (lane == 0 && jw + q < g.n) gemv_emit(g, jw + q, c0, y, u_out, ldu, contrib_ld);
+          const double* col = Mp + (long long)min(o0 + warp * 4 + q, g.n - 1) * g.ld;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            v[q * 4 + u] = u * 32 + lane < nj ? __ldg(col + u * 32) : 0.0;
         }
       }
-    }
-    return;
-  }
-  if (g.trans == 0) {
-    // 32-row strip, lane = row; of every staged chunk of x, warp w takes the
-    // 32 columns [32 w, 32 w + 32), so that a warp's loads are whole 256-byte
-    // column segments and several are in flight; the eight partial sums are
-    // added in warp order
-    __shared__ double red[8][32][RG];
-    const int i = local * 32 + lane;
-    for (int c0 = 0; c0 < nrhs; c0 += RG) {
-      const int nc = min(RG, nrhs - c0);
-      double acc[RG];
+      if (stage) {
+        __syncthreads();  // readers of the previous chunk are done
+        int id[kG1Chunk / 256];
 #pragma unroll
-      for (int cc = 0; cc < RG; ++cc) acc[cc] = 0.0;
-      // lower triangular: this strip's rows need no column right of its last row
-      const int jend = g.tri ? min(g.n, (local + 1) * 32) : g.n;
-      for (int j0 = 0; j0 < jend; j0 += kXChunk) {
-        const int nj = min(kXChunk, jend - j0);
-        __syncthreads();
-        for (int e = tid; e < nj * RG; e += 256) {
-          const int jj = e / RG, cc = e % RG;
-          xs[jj][cc] = (cc < nc) ? u_in[g.in_idx[j0 + jj] + (long long)(c0 + cc) * ldu] : 0.0;
+        for (int u = 0; u < kG1Chunk / 256; ++u) {
+          const int e = u * 256 + tid;
+          id[u] = e < nj ? g.in_idx[c0 + e] : -1;
         }
-        __syncthreads();
-        const int jb = warp * 32, cnt = min(32, nj - jb);
-        if (i < g.m && cnt > 0) {
-          const double* col = g.M + i + (long long)(j0 + jb) * g.ld;
-#pragma unroll 8
-          for (int jj = 0; jj < cnt; ++jj) {
-            const double mv = col[(long long)jj * g.ld];
 #pragma unroll
-            for (int cc = 0; cc < RG; ++cc)
-              acc[cc] = fma(mv, xs[jb + jj][cc], acc[cc]);
+        for (int u = 0; u < kG1Chunk / 256; ++u)
+          xs[u * 256 + tid] = id[u] >= 0 ? x.uin[id[u]] : 0.0;
+        __syncthreads();
+        held0 = c0;
+        held1 = c0 + nj;
+      }
+      if (g.trans == 0) {
+        double s0 = acc[0];
+        for (int j = j0; j < j1; j += 16) {
+          if (j > j0) {
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+              v[u] = j + u < j1 ? __ldg(Mp + (long long)(j + u) * g.ld) : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+            if (j + u < j1) s0 = fma(v[u], xs[j + u], s0);
+        }
+        acc[0] = s0;
+      } else {
+        for (int r0 = 0; r0 < nj; r0 += 128) {
+          if (r0 > 0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const double* col = Mp + r0 + (long long)min(o0 + warp * 4 + q, g.n - 1) * g.ld;
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                v[q * 4 + u] = r0 + u * 32 + lane < nj ? __ldg(col + u * 32) : 0.0;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const double xv = r0 + u * 32 + lane < nj ? xs[r0 + u * 32 + lane] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = fma(v[q * 4 + u], xv, acc[q]);
           }
         }
       }
-#pragma unroll
-      for (int cc = 0; cc < RG; ++cc) red[warp][lane][cc] = acc[cc];
-      __syncthreads();
-      if (warp == 0 && i < g.m) {
-        for (int cc = 0; cc < nc; ++cc) {
-          double y = red[0][lane][cc];
-#pragma unroll
-          for (int w = 1; w < 8; ++w) y += red[w][lane][cc];
-          gemv_emit(g, i, c0 + cc, y, u_out, ldu, contrib_ld);
-        }
-      }
     }
-  } else {
-    for (int c0 = 0; c0 < nrhs; c0 += RG) {
-      const int nc = min(RG, nrhs - c0);
-      double acc[4][RG];
+    if (g.trans == 0) {
+      red[warp][lane] = acc[0];
+      __syncthreads();
+      if (warp == 0) {
+        double y = red[0][lane];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int cc = 0; cc < RG; ++cc) acc[q][cc] = 0.0;
-      // lower triangular: these columns have no entry above their first column
-      const int ibeg = g.tri ? ((local * 32) / kXChunk) * kXChunk : 0;
-      const int jw = local * 32 + warp * 4;  // this warp's first column
-      for (int i0 = ibeg; i0 < g.m; i0 += kXChunk) {
-        const int ni = min(kXChunk, g.m - i0);
-        __syncthreads();
-        for (int e = tid; e < ni * RG; e += 256) {
-          const int ii = e / RG, cc = e % RG;
-          xs[ii][cc] = (cc < nc) ? u_in[g.in_idx[i0 + ii] + (long long)(c0 + cc) * ldu] : 0.0;
-        }
-        __syncthreads();
-        // the warp's four columns at each row: four independent loads a step
-#pragma unroll 2
-        for (int ii = lane; ii < ni; ii += 32) {
-          double mv[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            mv[q] = jw + q < g.n ? g.M[(long long)(jw + q) * g.ld + i0 + ii] : 0.0;
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int cc = 0; cc < RG; ++cc) acc[q][cc] = fma(mv[q], xs[ii][cc], acc[q][cc]);
-        }
+        for (int w = 1; w < 8; ++w) y += red[w][lane];
+        part[lane] = y;
       }
+    } else {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int j = jw + q;
-#pragma unroll
-        for (int cc = 0; cc < RG; ++cc) {
-          const double y = warp_sum(acc[q][cc]);
-          if (lane == 0 && j < g.n && cc < nc) gemv_emit(g, j, c0 + cc, y, u_out, ldu, contrib_ld);
-        }
+        const double y = warp_sum(acc[q]);
+        if (lane == 0) part[warp * 4 + q] = y;
       }
+    }
+    if (C > 1) {
+      cl.sync();
+      if (rank == 0 && tid < 32 && o0 + tid < out) {
+        double y = part[tid];
+        for (int q = 1; q < C; ++q) y += cl.map_shared_rank(part, q)[tid];
+        gemv_emit(g, x, o0 + tid, 0, y);
+      }
+      cl.sync();
+    } else {
+      __syncthreads();
+      if (tid < 32 && o0 + tid < out) gemv_emit(g, x, o0 + tid, 0, part[tid]);
+      __syncthreads();
     }
   }
 }
 
-__device__ __forceinline__ int find_desc_ll(const long long* __restrict__ off, int nd,
-                                            long long t) {
-  int lo = 0, hi = nd - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= t) lo = mid; else hi = mid - 1;
+// Several vectors: 64 outputs x BN right-hand sides per CTA on DMMA, the reduction
+// through the cp.async pipeline of k_dgemm with the B rows gathered from u. Four warps
+// of 16 outputs; a cluster shares the reduction where tiles are few (as in k_gemv1),
+// each rank adding up its share of the outputs. Bound by the factor's stream up to
+// about 20 right-hand sides, by the DMMA pipe beyond. It replaced gather, product and
+// emit launches for 16 and more vectors, padded to 64 (F u of 24 vectors at n = 48:
+// 1.21 ms), and GEMVs over groups of 4 below that.
+constexpr int kMmaIdx = 2048;
+template <int BN>
+constexpr int apply_mma_smem() {
+  return (BN >= 32 ? 3 : 4) * kGBK * (64 + 4 + BN + 4) * (int)sizeof(double);
+}
+template <int BN>
+__global__ void __launch_bounds__(128, BN == 64 ? 3 : 4)
+    k_apply_mma(const GemvFastSeg* __restrict__ segs, const int* __restrict__ seg_off, int nseg,
+                GemvCtx kx) {
+  namespace cg = cooperative_groups;
+  constexpr int T = 128, BM = 64, ST = BN >= 32 ? 3 : 4;
+  constexpr int SA = BM + 4, SB = BN + 4, QA = BM * kGBK / T, QB = BN * kGBK / T;
+  constexpr int NB = BN / 8;
+  extern __shared__ double lsm[];
+  double* As = lsm;
+  double* Bs = lsm + ST * kGBK * SA;
+  __shared__ int idx[kMmaIdx];
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int unit = blockIdx.x / C;
+  const int si = nseg == 1 ? 0 : find_desc(seg_off, nseg, unit);
+  const int4 tb = segs[si].tab[unit - seg_off[si]];
+  const GemvDesc g = segs[si].desc[tb.x];
+  const GemvCtx x = gemv_ctx(g, kx);
+  const int r0 = blockIdx.y * BN;  // first right-hand side
+  if (r0 >= x.nrhs) return;        // the same in every CTA of the cluster
+  const int nr = min(BN, x.nrhs - r0);
+  const int len = g.trans ? g.m : g.n, out = g.trans ? g.n : g.m;
+  const int m0 = tb.y * BM;
+  const int lo = (g.tri && g.trans) ? m0 : 0, hi = (g.tri && !g.trans) ? min(len, m0 + BM) : len;
+  const int per = (((hi - lo + C - 1) / C) + kGBK - 1) / kGBK * kGBK;
+  const int ka = lo + rank * per, kb = min(hi, ka + per);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  // A(row, k): M[row + k ld], or M[k + row ld] transposed; copies as in k_dgemm
+  const bool ta = g.trans != 0;
+  const int amm = ta ? tid / kGBK : tid % BM, akk = ta ? tid % kGBK : tid / BM;
+  const long long astep = (long long)(ta ? T / kGBK : T / BM) * g.ld;
+  const long long aadv = ta ? kGBK : (long long)kGBK * g.ld;
+  const int as0 = akk * SA + amm, asq = ta ? T / kGBK : (T / BM) * SA;
+  const int bc = tid % BN, bkk = tid / BN;
+  const bool bok = bc < nr;
+  unsigned amask = 0;
+#pragma unroll
+  for (int q = 0; q < QA; ++q)
+    if (m0 + amm + (ta ? (T / kGBK) * q : 0) < out) amask |= 1u << q;
+  double acc[2][NB][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  for (int s0 = ka; s0 < kb; s0 += kMmaIdx) {
+    const int s1 = min(kb, s0 + kMmaIdx), nk = (s1 - s0 + kGBK - 1) / kGBK;
+    __syncthreads();
+    for (int e = tid; e < s1 - s0; e += T) idx[e] = g.in_idx[s0 + e];
+    __syncthreads();
+    const double* ap = ta ? g.M + s0 + akk + (long long)(m0 + amm) * g.ld
+                          : g.M + (m0 + amm) + (long long)(s0 + akk) * g.ld;
+    auto issue_a = [&](int stage, int k0, int part, int parts) {
+      double* as = As + stage * kGBK * SA + as0;
+#pragma unroll
+      for (int q = 0; q < QA; ++q)
+        if (q >= QA / parts * part && q < QA / parts * (part + 1)) {
+          const bool ok = (amask >> q & 1) && k0 + akk + (ta ? 0 : (T / BM) * q) < s1;
+          cp_async8(as + q * asq, ok ? ap + q * astep : g.M, ok);
+        }
+    };
+    auto issue_b = [&](int stage, int k0) {
+      double* bs = Bs + stage * kGBK * SB;
+#pragma unroll
+      for (int q = 0; q < QB; ++q) {
+        const int kk = bkk + (T / BN) * q;
+        const bool ok = bok && k0 + kk < s1;
+        cp_async8(bs + kk * SB + bc,
+                  ok ? x.uin + (long long)idx[k0 + kk - s0] * x.nrhs + r0 + bc : x.uin, ok);
+      }
+    };
+#pragma unroll
+    for (int st = 0; st < ST - 1; ++st) {
+      if (st < nk) {
+        issue_a(st, s0 + st * kGBK, 0, 1);
+        issue_b(st, s0 + st * kGBK);
+        ap += aadv;
+      }
+      cp_async_commit();
+    }
+    for (int t = 0; t < nk; ++t) {
+      cp_async_wait<ST - 2>();
+      __syncthreads();
+      const int nt = t + ST - 1, k0n = s0 + nt * kGBK;
+      const double* as = As + (t % ST) * kGBK * SA + tq * SA + warp * 16 + gq;
+      const double* bs = Bs + (t % ST) * kGBK * SB + tq * SB + gq;
+      if (nt < nk) issue_b(nt % ST, k0n);
+#pragma unroll
+      for (int k4 = 0; k4 < kGBK / 4; ++k4) {
+        double af[2], bf[NB];
+#pragma unroll
+        for (int a = 0; a < 2; ++a) af[a] = as[k4 * 4 * SA + a * 8];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) bf[b] = bs[k4 * 4 * SB + b * 8];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < NB; ++b) dmma(acc[a][b], af[a], bf[b]);
+        if (nt < nk) issue_a(nt % ST, k0n, k4, kGBK / 4);
+      }
+      cp_async_commit();
+      ap += aadv;
+    }
+    cp_async_wait<0>();
   }
-  return lo;
-}
-
-__global__ void k_apply_gather(const ApplyGatherDesc* __restrict__ descs,
-                               const long long* __restrict__ off, int nd, long long total,
-                               const double* __restrict__ u, long long ldu) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int di = find_desc_ll(off, nd, t);
-    const ApplyGatherDesc d = descs[di];
-    const long long e = t - off[di];
-    const int k = (int)(e % d.len);
-    const long long c = e / d.len;
-    d.dst[e] = u[d.idx[k] + c * ldu];
+  if (C > 1) {
+    // parts to shared memory, [output][right-hand side]
+    constexpr int LP = BN + 2;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          lsm[(warp * 16 + a * 8 + gq) * LP + b * 8 + tq * 2 + c] = acc[a][b][c];
+    cl.sync();
+    const int rows = BM / C;
+    for (int e = tid; e < rows * BN; e += T) {
+      const int i = rank * rows + e / BN, c = e % BN;
+      if (m0 + i >= out || c >= nr) continue;
+      double y = 0.0;
+      for (int q = 0; q < C; ++q) y += cl.map_shared_rank(lsm, q)[i * LP + c];
+      gemv_emit(g, x, m0 + i, r0 + c, y);
+    }
+    cl.sync();
+  } else {
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const int i = m0 + warp * 16 + a * 8 + gq;
+      if (i >= out) continue;
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int rc = b * 8 + tq * 2 + c;
+          if (rc < nr) gemv_emit(g, x, i, r0 + rc, acc[a][b][c]);
+        }
+    }
   }
 }
 
-void launch_apply_gather(const ApplyGatherDesc* d_desc, const long long* d_off, int nd,
-                         long long total, const double* u, long long ldu, cudaStream_t s) {
-  if (total <= 0) return;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-  k_apply_gather<<<blocks, 256, 0, s>>>(d_desc, d_off, nd, total, u, ldu);
+template <class K>
+void launch_clustered(K kernel, dim3 grid, int threads, int smem, int cluster, cudaStream_t s,
+                      const GemvFastSeg* segs, const int* off, int nseg, GemvCtx k) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, segs, off, nseg, k);
 }
 
-__global__ void k_apply_emit(const ApplyEmitDesc* __restrict__ descs,
-                             const long long* __restrict__ off, int nd, long long total,
-                             double* __restrict__ u, long long ldu, long long contrib_ld) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int di = find_desc_ll(off, nd, t);
-    const ApplyEmitDesc d = descs[di];
-    const long long e = t - off[di];
-    const int i = (int)(e % d.rows);
-    const long long c = e / d.rows;
-    const double y = d.Y[e];
-    if (d.mode == 1) d.contrib[i + c * contrib_ld] = y;
-    else if (d.mode == 0) u[d.out_idx[i] + c * ldu] += d.alpha * y;
-    else u[d.out_idx[i] + c * ldu] = d.alpha * y;
+int apply_rhs_class(int nrhs) {
+  return nrhs == 1 ? 1 : nrhs <= 8 ? 8 : nrhs <= 16 ? 16 : nrhs <= 32 ? 32 : 64;
+}
+
+void launch_gemv(const GemvFastSeg* d_segs, const int* d_seg_off, int nseg, int units,
+                 const GemvLayout& lay, const double* u_in, double* u_out, double* contrib,
+                 int nrhs, cudaStream_t s) {
+  if (units <= 0) return;
+  const GemvCtx k{u_in, u_out, contrib, nrhs};
+  const dim3 grid(units * lay.cluster, (nrhs + 63) / 64);
+  switch (lay.kind == kGemvMulti ? apply_rhs_class(std::max(2, nrhs)) : lay.kind) {
+    case kGemvSmall: {
+      const int smem = 8 * (lay.elems + kGemvSmallMax) * (int)sizeof(double);
+      ensure_smem((const void*)k_gemv_small, smem);
+      k_gemv_small<<<(units + 7) / 8, 256, smem, s>>>(d_segs, d_seg_off, nseg, k, lay.elems);
+      break;
+    }
+    case kGemvTiles:
+      launch_clustered(k_gemv1, dim3(units * lay.cluster), 256, 0, lay.cluster, s, d_segs,
+                       d_seg_off, nseg, k);
+      break;
+    case 8:
+      ensure_smem((const void*)k_apply_mma<8>, apply_mma_smem<8>());
+      launch_clustered(k_apply_mma<8>, grid, 128, apply_mma_smem<8>(), lay.cluster, s, d_segs,
+                       d_seg_off, nseg, k);
+      break;
+    case 16:
+      ensure_smem((const void*)k_apply_mma<16>, apply_mma_smem<16>());
+      launch_clustered(k_apply_mma<16>, grid, 128, apply_mma_smem<16>(), lay.cluster, s, d_segs,
+                       d_seg_off, nseg, k);
+      break;
+    case 32:
+      ensure_smem((const void*)k_apply_mma<32>, apply_mma_smem<32>());
+      launch_clustered(k_apply_mma<32>, grid, 128, apply_mma_smem<32>(), lay.cluster, s, d_segs,
+                       d_seg_off, nseg, k);
+      break;
+    default:
+      ensure_smem((const void*)k_apply_mma<64>, apply_mma_smem<64>());
+      launch_clustered(k_apply_mma<64>, grid, 128, apply_mma_smem<64>(), lay.cluster, s, d_segs,
+                       d_seg_off, nseg, k);
   }
 }
 
-void launch_apply_emit(const ApplyEmitDesc* d_desc, const long long* d_off, int nd,
-                       long long total, double* u, long long ldu, long long contrib_ld,
-                       cudaStream_t s) {
-  if (total <= 0) return;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-  k_apply_emit<<<blocks, 256, 0, s>>>(d_desc, d_off, nd, total, u, ldu, contrib_ld);
+// ua(p, c) = src[p + c lds], zero on the index-0 planes; ub = 0. Tiles of 32 DOFs x 32
+// right-hand sides, transposed through shared memory.
+__global__ void __launch_bounds__(256) k_apply_in(const double* __restrict__ src, long long lds,
+                                                  double* __restrict__ ua,
+                                                  double* __restrict__ ub, int NC, int nrhs) {
+  const long long n3 = (long long)NC * NC * NC;
+  if (nrhs == 1) {
+    const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (p >= n3) return;
+    const int i = (int)(p % NC), j = (int)((p / NC) % NC), k = (int)(p / ((long long)NC * NC));
+    ua[p] = (i == 0 || j == 0 || k == 0) ? 0.0 : src[p];
+    ub[p] = 0.0;
+    return;
+  }
+  __shared__ double tl[32][33];
+  const long long p0 = (long long)blockIdx.x * 32;
+  const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long p = p0 + lane;
+  const int i = (int)(p % NC), j = (int)((p / NC) % NC), k = (int)(p / ((long long)NC * NC));
+  const bool in = p < n3 && i && j && k;
+  for (int c = w; c < 32; c += 8)
+    tl[c][lane] = (in && c0 + c < nrhs) ? src[p + (c0 + c) * lds] : 0.0;
+  __syncthreads();
+  for (int q = w; q < 32; q += 8)
+    if (p0 + q < n3 && c0 + lane < nrhs) {
+      ua[(p0 + q) * nrhs + c0 + lane] = tl[lane][q];
+      ub[(p0 + q) * nrhs + c0 + lane] = 0.0;
+    }
 }
 
-__global__ void k_reduce_seg(const ReduceSeg* __restrict__ segs, const int* __restrict__ seg_off,
-                             int nseg) {
+void launch_apply_in(const double* src, long long lds, double* ua, double* ub, int NC, int nrhs,
+                     cudaStream_t s) {
+  const long long n3 = (long long)NC * NC * NC;
+  if (nrhs == 1) k_apply_in<<<(int)((n3 + 255) / 256), 256, 0, s>>>(src, lds, ua, ub, NC, 1);
+  else
+    k_apply_in<<<dim3((int)((n3 + 31) / 32), (nrhs + 31) / 32), 256, 0, s>>>(src, lds, ua, ub, NC,
+                                                                            nrhs);
+}
+
+// dst[p + c ldd] = u(p, c)
+__global__ void __launch_bounds__(256) k_apply_out(const double* __restrict__ u,
+                                                   double* __restrict__ dst, long long ldd,
+                                                   long long n3, int nrhs) {
+  __shared__ double tl[32][33];
+  const long long p0 = (long long)blockIdx.x * 32;
+  const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int q = w; q < 32; q += 8)
+    tl[q][lane] = (p0 + q < n3 && c0 + lane < nrhs) ? u[(p0 + q) * nrhs + c0 + lane] : 0.0;
+  __syncthreads();
+  for (int c = w; c < 32; c += 8)
+    if (p0 + lane < n3 && c0 + c < nrhs) dst[p0 + lane + (c0 + c) * ldd] = tl[lane][c];
+}
+
+void launch_apply_out(const double* u, double* dst, long long ldd, long long n3, int nrhs,
+                      cudaStream_t s) {
+  if (nrhs == 1) {
+    cudaMemcpyAsync(dst, u, n3 * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    return;
+  }
+  k_apply_out<<<dim3((int)((n3 + 31) / 32), (nrhs + 31) / 32), 256, 0, s>>>(u, dst, ldd, n3, nrhs);
+}
+
+// u(dof[d], c) += alpha * sum over the DOF's slots in order; one segment per operator.
+__global__ void __launch_bounds__(256) k_reduce_seg(const ReduceSeg* __restrict__ segs,
+                                                    const int* __restrict__ seg_off, int nseg) {
   const int total = seg_off[nseg];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int si = find_desc(seg_off, nseg, t);
+    const int si = nseg == 1 ? 0 : find_desc(seg_off, nseg, t);
     const ReduceSeg sg = segs[si];
-    const int e = t - seg_off[si];
-    const int d = e % sg.ndof, c = e / sg.ndof;
+    const int e = t - seg_off[si], d = e / sg.nrhs, c = e - d * sg.nrhs;
     double sum = 0.0;
-    for (int q = sg.off[d]; q < sg.off[d + 1]; ++q) sum += sg.contrib[sg.slot[q] + (long long)c * sg.cld];
-    sg.u[sg.dof[d] + (long long)c * sg.ldu] += sg.alpha * sum;
+    const int q1 = sg.off[d + 1];
+    for (int q = sg.off[d]; q < q1; ++q) sum += sg.contrib[(long long)sg.slot[q] * sg.nrhs + c];
+    sg.u[(long long)sg.dof[d] * sg.nrhs + c] += sg.alpha * sum;
   }
 }
 
@@ -3553,142 +3813,26 @@ void launch_reduce_seg(const ReduceSeg* d_segs, const int* d_seg_off, int nseg, 
   k_reduce_seg<<<blocks, 256, 0, s>>>(d_segs, d_seg_off, nseg);
 }
 
-// ---- apply GEMV, the plans' layouts ----------------------------------------
-// A launch covers segments (one per operator / request: the serving loop runs
-// several requests' stages in one launch), each a descriptor array and, for
-// the larger layouts, a unit table; seg_off holds the units' prefix over
-// segments. Every descriptor's own vectors (uin, uout, nrhs, ldu, cld) apply
-// when set, else the launch's.
-struct GemvCtx {
-  const double* uin;
-  double* uout;
-  int nrhs;
-  long long ldu, cld;
-};
-__device__ __forceinline__ GemvCtx gemv_ctx(const GemvDesc& g, const double* u_in, double* u_out,
-                                            int nrhs, long long ldu, long long cld) {
-  return g.uin ? GemvCtx{g.uin, g.uout, g.nrhs, g.ldu, g.cld}
-               : GemvCtx{u_in, u_out, nrhs, ldu, cld};
-}
-
-// Small blocks (both dimensions at most 64): one warp per descriptor. y = M x:
-// lane = row, columns in order. y = M^T x: lanes over rows, one warp sum per
-// column (fixed shuffle order). Entries above the diagonal of a triangular M
-// are not read.
-__global__ void __launch_bounds__(256, 3) k_gemv_small(const GemvFastSeg* __restrict__ segs,
-                                                    const int* __restrict__ seg_off, int nseg,
-                                                    const double* __restrict__ u_in,
-                                                    double* __restrict__ u_out, int nrhs_k,
-                                                    long long ldu_k, long long cld_k) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * 8 + warp;
-  if (unit >= seg_off[nseg]) return;
-  const int si = find_desc(seg_off, nseg, unit);
-  const GemvDesc g = segs[si].desc[unit - seg_off[si]];
-  const GemvCtx x = gemv_ctx(g, u_in, u_out, nrhs_k, ldu_k, cld_k);
-  for (int c0 = 0; c0 < x.nrhs; c0 += kRhsGroup) {
-    const int nc = min(kRhsGroup, x.nrhs - c0);
-    if (g.trans == 0) {
-      for (int i = lane; i < g.m; i += 32) {
-        double acc[kRhsGroup] = {0.0, 0.0, 0.0, 0.0};
-        const int jend = g.tri ? min(g.n, i + 1) : g.n;
-        for (int j = 0; j < jend; ++j) {
-          const double mv = g.M[i + (long long)j * g.ld];
-          const long long xo = g.in_idx[j] + (long long)c0 * x.ldu;
-#pragma unroll
-          for (int cc = 0; cc < kRhsGroup; ++cc)
-            if (cc < nc) acc[cc] = fma(mv, x.uin[xo + (long long)cc * x.ldu], acc[cc]);
-        }
-        for (int cc = 0; cc < nc; ++cc) gemv_emit(g, i, c0 + cc, acc[cc], x.uout, x.ldu, x.cld);
-      }
-    } else {
-      double xr[2][kRhsGroup];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = lane + 32 * h;
-#pragma unroll
-        for (int cc = 0; cc < kRhsGroup; ++cc)
-          xr[h][cc] = (i < g.m && cc < nc)
-                          ? x.uin[g.in_idx[i] + (long long)(c0 + cc) * x.ldu] : 0.0;
-      }
-      for (int j = 0; j < g.n; ++j) {
-        double acc[kRhsGroup] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int i = lane + 32 * h;
-          if (i < g.m && (!g.tri || i >= j)) {
-            const double mv = g.M[i + (long long)j * g.ld];
-#pragma unroll
-            for (int cc = 0; cc < kRhsGroup; ++cc) acc[cc] = fma(mv, xr[h][cc], acc[cc]);
-          }
-        }
-#pragma unroll
-        for (int cc = 0; cc < kRhsGroup; ++cc)
-          if (cc < nc) acc[cc] = warp_sum(acc[cc]);  // nc is the same on every lane
-        if (lane == 0)
-          for (int cc = 0; cc < nc; ++cc) gemv_emit(g, j, c0 + cc, acc[cc], x.uout, x.ldu, x.cld);
-      }
-    }
-  }
-}
-
-// Larger blocks: gemv_tile's tiles (y = M x: 32-row strips; y = M^T x:
-// 32-column tiles), located from the unit table (descriptor, tile) rather than
-// a search over tile offsets. Two CTAs per SM: each warp keeps eight column
-// loads in flight, which covers the memory latency at this occupancy.
-template <int RG>
-__global__ void __launch_bounds__(256, RG == 1 ? 3 : 2)
-    k_gemv_tiles(const GemvFastSeg* __restrict__ segs, const int* __restrict__ seg_off, int nseg,
-                 const double* __restrict__ u_in, double* __restrict__ u_out, int nrhs,
-                 long long ldu, long long contrib_ld) {
-  const int si = find_desc(seg_off, nseg, blockIdx.x);
-  const int2 t = segs[si].tab[blockIdx.x - seg_off[si]];
-  gemv_tile<RG>(segs[si].desc[t.x], t.y, u_in, u_out, nrhs, ldu, contrib_ld);
-}
-
-int gemv_tile_count(int m, int n, int trans) {
-  if (m <= 0 || n <= 0) return 0;
-  // y = M x: 32-row strips; y = M^T x: 32-column tiles
-  return ((trans == 0 ? m : n) + 31) / 32;
-}
-
-void launch_gemv_fast(const GemvFastSeg* d_segs, const int* d_seg_off, int nseg, int units,
-                      int layout, const double* u_in, double* u_out, int nrhs, long long ldu,
-                      long long contrib_ld, cudaStream_t s) {
-  if (units <= 0) return;
-  if (layout == kGemvSmall)
-    k_gemv_small<<<(units + 7) / 8, 256, 0, s>>>(d_segs, d_seg_off, nseg, u_in, u_out, nrhs, ldu,
-                                                 contrib_ld);
-  else if (nrhs == 1)
-    k_gemv_tiles<1><<<units, 256, 0, s>>>(d_segs, d_seg_off, nseg, u_in, u_out, nrhs, ldu,
-                                          contrib_ld);
-  else  // several vectors, or per-descriptor vectors (serving: nrhs 0)
-    k_gemv_tiles<kRhsGroup><<<units, 256, 0, s>>>(d_segs, d_seg_off, nseg, u_in, u_out, nrhs,
-                                                  ldu, contrib_ld);
-}
-
-
 __global__ void k_reduce_scatter(const int* __restrict__ dof, const int* __restrict__ off,
                                  const int* __restrict__ slot,
-                                 const double* __restrict__ contrib, int ndof,
-                                 long long contrib_ld, double alpha, double* __restrict__ u,
-                                 int nrhs, long long ldu) {
+                                 const double* __restrict__ contrib, int ndof, double alpha,
+                                 double* __restrict__ u, int nrhs) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)ndof * nrhs) return;
-  const int d = (int)(t % ndof), c = (int)(t / ndof);
+  const int d = (int)(t / nrhs), c = (int)(t - (long long)d * nrhs);
   double s = 0.0;
-  for (int q = off[d]; q < off[d + 1]; ++q) s += contrib[slot[q] + (long long)c * contrib_ld];
-  u[dof[d] + (long long)c * ldu] += alpha * s;
+  const int q1 = off[d + 1];
+  for (int q = off[d]; q < q1; ++q) s += contrib[(long long)slot[q] * nrhs + c];
+  u[(long long)dof[d] * nrhs + c] += alpha * s;
 }
 
 void launch_reduce_scatter(const int* d_dof, const int* d_off, const int* d_slot,
-                           const double* d_contrib, int ndof, long long contrib_ld,
-                           double alpha, double* u, int nrhs, long long ldu, cudaStream_t s) {
+                           const double* d_contrib, int ndof, double alpha, double* u, int nrhs,
+                           cudaStream_t s) {
   const long long total = (long long)ndof * nrhs;
   if (total <= 0) return;
   k_reduce_scatter<<<(int)((total + 255) / 256), 256, 0, s>>>(d_dof, d_off, d_slot, d_contrib,
-                                                             ndof, contrib_ld, alpha, u, nrhs,
-                                                             ldu);
+                                                             ndof, alpha, u, nrhs);
 }
 
 // ===========================================================================

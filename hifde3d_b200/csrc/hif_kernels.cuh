@@ -178,46 +178,26 @@ void launch_member_cells(const int* d_skel, const long long* d_off, const int* d
 void launch_member_faces(const int* d_skel, const long long* d_off, const int* d_cnt,
                          const int* d_src, int nq, long long n3, int* d_dof_src, cudaStream_t s);
 
-// Apply for many right-hand sides as gather / GEMM / emit: the input rows of a
-// descriptor are gathered into a dense block (len x nrhs, ld len), multiplied
-// by op(M) with the batched GEMM, and the result (rows x nrhs, ld rows) is
-// emitted like the GEMV's output (mode 0: u[out] += alpha y; 1: contrib = y;
-// 2: u[out] = alpha y). Element counts are prefix sums over descriptors.
-struct ApplyGatherDesc {
-  const int* idx;
-  double* dst;
-  int len;
-};
-struct ApplyEmitDesc {
-  const double* Y;
-  const int* out_idx;
-  double* contrib;
-  int rows, mode;
-  double alpha;
-};
-void launch_apply_gather(const ApplyGatherDesc* d_desc, const long long* d_off, int nd,
-                         long long total, const double* u, long long ldu, cudaStream_t s);
-void launch_apply_emit(const ApplyEmitDesc* d_desc, const long long* d_off, int nd,
-                       long long total, double* u, long long ldu, long long contrib_ld,
-                       cudaStream_t s);
-// Apply: y = op(M) x[in] with x, y gathered / scattered through DOF lists.
+// Apply: y = op(M) x[in] with x, y gathered / scattered through DOF lists. The work
+// vectors and the contribution buffer hold the right-hand sides of an entry side by
+// side: (p, c) at u[p * nrhs + c].
 struct GemvDesc {
-  const double* M;
+  const double* M;      // m x n, ld == m
   long long ld;
   const int* in_idx;
   const int* out_idx;   // mode 0 / 2
-  double* contrib;      // mode 1: contribution slots (length = rows of op(M))
+  long long cslot;      // mode 1: first contribution slot of the block
   int m, n;             // M is m x n
   int trans;            // 0: y = M x (len m), 1: y = M^T x (len n)
-  int tri;              // 1: M is lower triangular (square); entries above the diagonal are not read
+  int tri;              // 1: M is lower triangular (square); entries above the diagonal are not used
   double alpha;
   int mode;             // 0: u_out[out] += alpha y; 1: contrib = y; 2: u_out[out] = alpha y
   // Optional per-descriptor vectors (batched solves of several operators in one
-  // launch); when uin is null the launch's vectors and sizes apply.
+  // launch); when uin is null the launch's vectors apply.
   const double* uin;
   double* uout;
+  double* contrib;
   int nrhs;
-  long long ldu, cld;
 };
 
 // The serving loop's batched reduce-scatter: one segment per request.
@@ -227,13 +207,18 @@ struct ReduceSeg {
   const int* slot;
   const double* contrib;
   double* u;
-  long long cld, ldu;
   int ndof, nrhs;
   double alpha;
 };
 // d_seg_off: prefix over segments of ndof * nrhs.
 void launch_reduce_seg(const ReduceSeg* d_segs, const int* d_seg_off, int nseg, int total,
                        cudaStream_t s);
+// Into the work vectors (boundary planes zeroed, ub cleared) and out of them; src / dst
+// hold the right-hand sides as columns.
+void launch_apply_in(const double* src, long long lds, double* ua, double* ub, int NC, int nrhs,
+                     cudaStream_t s);
+void launch_apply_out(const double* u, double* dst, long long ldd, long long n3, int nrhs,
+                      cudaStream_t s);
 
 struct CopyDesc {
   const double* src;
@@ -456,29 +441,33 @@ void launch_trsm_upper(const double* R, long long ldr, int k, double* B, long lo
                        cudaStream_t s);
 int copy_tiles(int m, int n);
 
-// contrib_ld: stride between right-hand sides in the contribution buffer.
-// The apply's GEMV launches (the engine's plans and the serving loop's batched
-// stages). Layouts: kGemvSmall, one warp per descriptor (both dimensions <=
-// kGemvSmallMax; units = descriptors); kGemvTiles, y = M x by 32-row strips or
-// y = M^T x by 32-column tiles (units = entries (descriptor, tile) of the
-// segment's table, gemv_tile_count tiles per descriptor). A launch covers
-// segments (one per operator or request) of one layout; seg_off: prefix of the
-// units over the segments.
-constexpr int kGemvSmall = 0, kGemvTiles = 1, kGemvLayouts = 2;
-int gemv_tile_count(int m, int n, int trans);
-constexpr int kGemvSmallMax = 64;
+// The apply's product launches (the engine's plans and the serving loop's batched
+// stages). Kinds: one vector, small blocks (a warp per descriptor; units =
+// descriptors); one vector, larger blocks (units = runs of 32-wide output tiles: {desc,
+// first tile, tiles}); several vectors (units = 64-wide output tiles). `cluster` CTAs
+// share a unit's reduction. A launch covers segments (one per operator or request) of
+// one layout; seg_off: prefix of the units over the segments.
+constexpr int kGemvSmall = 0, kGemvTiles = 1, kGemvMulti = 2;
+constexpr int kGemvSmallMax = 64;       // small blocks: both dimensions at most
+constexpr int kGemvSmallElems = 2048;   // and this many entries
+struct GemvLayout {
+  int kind = kGemvSmall, cluster = 1, elems = 0;  // elems: the largest small block
+};
 struct GemvFastSeg {
   const GemvDesc* desc;
-  const int2* tab;  // null for kGemvSmall
+  const int4* tab;  // null for kGemvSmall
 };
-void launch_gemv_fast(const GemvFastSeg* d_segs, const int* d_seg_off, int nseg, int units,
-                      int layout, const double* u_in, double* u_out, int nrhs, long long ldu,
-                      long long contrib_ld, cudaStream_t s);
+// Right-hand sides of one CTA tile for a count of them: 1, 8, 16, 32 or 64.
+int apply_rhs_class(int nrhs);
+// nrhs: the launch's right-hand sides (with per-descriptor vectors: the largest count).
+void launch_gemv(const GemvFastSeg* d_segs, const int* d_seg_off, int nseg, int units,
+                 const GemvLayout& lay, const double* u_in, double* u_out, double* contrib,
+                 int nrhs, cudaStream_t s);
 
-// u[dof[d]] += alpha * sum_{t in [off[d], off[d+1])} contrib[slot[t]], in order.
+// u(dof[d], c) += alpha * sum_{t in [off[d], off[d+1])} contrib(slot[t], c), in order.
 void launch_reduce_scatter(const int* d_dof, const int* d_off, const int* d_slot,
-                           const double* d_contrib, int ndof, long long contrib_ld,
-                           double alpha, double* u, int nrhs, long long ldu, cudaStream_t s);
+                           const double* d_contrib, int ndof, double alpha, double* u, int nrhs,
+                           cudaStream_t s);
 
 // Operators and vectors.
 void launch_setup_node(const double* d_A, const double* d_V, int N, double h, double* d_band,

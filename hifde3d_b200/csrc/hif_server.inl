@@ -294,9 +294,9 @@ class Server {
       long long key;
       int type;
       GemvFastSeg gs;  // descriptors bound to this request's vectors
-      int layout;
+      GemvLayout lay;
       ReduceSeg rs;
-      int tiles;  // units of the GEMV layout, or reduced entries
+      int tiles;  // units of the layout, or reduced entries
     };
     std::vector<L> launches;
     BufList bufs;
@@ -324,28 +324,28 @@ class Server {
     HIF_CK(cudaMemcpyAsync(a.rv, a.r->b.data(), nv * 8, cudaMemcpyHostToDevice, sstream_));
     a.r->b.clear();
     // bind the operator's inverse-apply plan to this request's vectors
+    if (a.nrhs > 1) e.ensure_multi(e.plan_inv, sstream_);
     double* vec[3] = {a.ua, a.ub, a.uc};
     for (const ApplyLaunch& l : e.plan_inv.launches) {
       Active::L x{};
       x.key = l.key;
       x.type = l.type;
       if (l.type == 0) {
+        const ApplyLaunch::Form& f = l.form[a.nrhs > 1];
         std::vector<GemvDesc> dd = l.hdesc;
         for (GemvDesc& g : dd) {
           g.uin = vec[l.in_vec];
           g.uout = vec[l.out_vec];
+          g.contrib = a.contrib;
           g.nrhs = a.nrhs;
-          g.ldu = a.n3;
-          g.cld = cl;
-          if (g.mode == 1) g.contrib = a.contrib + (g.contrib - e.d_contrib);
         }
         x.gs.desc = a.bufs.add(upload(dd, sstream_));
-        x.gs.tab = l.d_tab;
-        x.layout = l.layout;
-        x.tiles = l.units;
+        x.gs.tab = f.d_tab;
+        x.lay = f.lay;
+        x.tiles = f.units;
       } else {
-        x.rs = ReduceSeg{l.d_dof, l.d_off, l.d_slot, a.contrib, vec[l.out_vec], cl, a.n3, l.ndof,
-                         a.nrhs, l.alpha};
+        x.rs = ReduceSeg{l.d_dof, l.d_off, l.d_slot, a.contrib, vec[l.out_vec], l.ndof, a.nrhs,
+                         l.alpha};
         x.tiles = l.ndof * a.nrhs;
       }
       a.launches.push_back(x);
@@ -359,38 +359,46 @@ class Server {
   // z = M^{-1} r for every request in `set`: per-request copies, then one launch
   // per stage key over all requests that have it.
   void batched_apply(std::vector<Active*>& set) {
-    for (Active* a : set) {
-      HIF_CK(cudaMemcpyAsync(a->ua, a->rv, a->n3 * a->nrhs * 8, cudaMemcpyDeviceToDevice, sstream_));
-      launch_zero_boundary(a->ua, a->e->NC, a->nrhs, a->n3, sstream_);
-      HIF_CK(cudaMemsetAsync(a->ub, 0, a->n3 * a->nrhs * 8, sstream_));
-    }
+    for (Active* a : set) launch_apply_in(a->rv, a->n3, a->ua, a->ub, a->e->NC, a->nrhs, sstream_);
     std::map<long long, std::vector<std::pair<Active*, size_t>>> stages;
     for (Active* a : set)
       for (size_t i = 0; i < a->launches.size(); ++i) stages[a->launches[i].key].push_back({a, i});
     BufList tick;
     for (auto& kv : stages) {
-      // one launch per GEMV layout present at this stage (the same kernels as
-      // hif_apply's, so each request computes exactly what it would alone)
-      std::vector<GemvFastSeg> gs[kGemvLayouts];
-      std::vector<int> goff[kGemvLayouts] = {{0}, {0}};
+      // one launch per layout and right-hand-side class present at this stage (the same
+      // kernels and tables as hif_apply's, so each request computes exactly what it
+      // would alone)
+      struct Group {
+        GemvLayout lay;
+        int nrhs = 1;
+        std::vector<GemvFastSeg> gs;
+        std::vector<int> off{0};
+      };
+      std::map<std::array<int, 3>, Group> groups;
       std::vector<ReduceSeg> rs;
       std::vector<int> roff(1, 0);
       for (auto& pr : kv.second) {
         const Active::L& l = pr.first->launches[pr.second];
         if (l.type == 0) {
-          gs[l.layout].push_back(l.gs);
-          goff[l.layout].push_back(goff[l.layout].back() + l.tiles);
+          Group& g = groups[{l.lay.kind, l.lay.cluster, apply_rhs_class(pr.first->nrhs)}];
+          g.lay.kind = l.lay.kind;
+          g.lay.cluster = l.lay.cluster;
+          g.lay.elems = std::max(g.lay.elems, l.lay.elems);
+          g.nrhs = std::max(g.nrhs, pr.first->nrhs);
+          g.gs.push_back(l.gs);
+          g.off.push_back(g.off.back() + l.tiles);
         } else {
           rs.push_back(l.rs);
           roff.push_back(roff.back() + l.tiles);
         }
       }
-      for (int lay = 0; lay < kGemvLayouts; ++lay) {
-        if (gs[lay].empty() || goff[lay].back() == 0) continue;
-        GemvFastSeg* dg = tick.add(upload(gs[lay], sstream_));
-        int* dgo = tick.add(upload(goff[lay], sstream_));
-        launch_gemv_fast(dg, dgo, (int)gs[lay].size(), goff[lay].back(), lay, nullptr, nullptr, 0,
-                         0, 0, sstream_);
+      for (auto& gk : groups) {
+        const Group& g = gk.second;
+        if (g.off.back() == 0) continue;
+        GemvFastSeg* dg = tick.add(upload(g.gs, sstream_));
+        int* dgo = tick.add(upload(g.off, sstream_));
+        launch_gemv(dg, dgo, (int)g.gs.size(), g.off.back(), g.lay, nullptr, nullptr, nullptr,
+                    g.nrhs, sstream_);
         ++merged_launches_;
       }
       if (!rs.empty() && roff.back() > 0) {
@@ -402,7 +410,8 @@ class Server {
       HIF_CK(cudaGetLastError());
     }
     for (Active* a : set)
-      HIF_CK(cudaMemcpyAsync(a->z, a->ub, a->n3 * a->nrhs * 8, cudaMemcpyDeviceToDevice, sstream_));
+      launch_apply_out(a->ub, a->z, a->n3, a->n3, a->nrhs, sstream_);
+    HIF_CK(cudaGetLastError());
     tick.release(sstream_);
   }
 
