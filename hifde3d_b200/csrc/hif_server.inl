@@ -75,6 +75,7 @@ class Server {
     cv_.notify_all();
     solver_.join();
     for (std::thread& t : workers_) t.join();
+    drop_bound();
     ops_.clear();
     cudaStreamSynchronize(sstream_);
     cudaStreamDestroy(sstream_);
@@ -356,14 +357,41 @@ class Server {
     a.iters.assign(a.nrhs, 0);
   }
 
-  // z = M^{-1} r for every request in `set`: per-request copies, then one launch
-  // per stage key over all requests that have it.
-  void batched_apply(std::vector<Active*>& set) {
-    for (Active* a : set) launch_apply_in(a->rv, a->n3, a->ua, a->ub, a->e->NC, a->nrhs, sstream_);
+  // The batched apply's launches for one set of requests: their segment tables lie in
+  // one device buffer, built when the set changes. An allocation and a copy per table
+  // and iteration set the pace of small operators.
+  struct Stage {
+    bool reduce = false;
+    GemvLayout lay;
+    int nrhs = 1, nseg = 0, total = 0;
+    size_t o_seg = 0, o_off = 0;  // offsets in the buffer
+  };
+  struct Bound {
+    std::vector<long long> ids;  // the set, by request
+    std::vector<Stage> stages;
+    char* d = nullptr;
+  };
+  Bound bound_;
+  void drop_bound() {
+    if (bound_.d) dfree(bound_.d, sstream_);
+    bound_ = Bound{};
+  }
+  void bind(const std::vector<Active*>& set) {
+    std::vector<long long> ids;
+    for (const Active* a : set) ids.push_back(a->r->id);
+    if (bound_.d && ids == bound_.ids) return;
+    drop_bound();
     std::map<long long, std::vector<std::pair<Active*, size_t>>> stages;
     for (Active* a : set)
       for (size_t i = 0; i < a->launches.size(); ++i) stages[a->launches[i].key].push_back({a, i});
-    BufList tick;
+    std::vector<char> host;
+    auto put = [&](const auto& v) {
+      host.resize((host.size() + 15) & ~size_t(15));
+      const size_t at = host.size(), bytes = v.size() * sizeof(v[0]);
+      host.resize(at + bytes);
+      std::memcpy(host.data() + at, v.data(), bytes);
+      return at;
+    };
     for (auto& kv : stages) {
       // one launch per layout and right-hand-side class present at this stage (the same
       // kernels and tables as hif_apply's, so each request computes exactly what it
@@ -395,24 +423,48 @@ class Server {
       for (auto& gk : groups) {
         const Group& g = gk.second;
         if (g.off.back() == 0) continue;
-        GemvFastSeg* dg = tick.add(upload(g.gs, sstream_));
-        int* dgo = tick.add(upload(g.off, sstream_));
-        launch_gemv(dg, dgo, (int)g.gs.size(), g.off.back(), g.lay, nullptr, nullptr, nullptr,
-                    g.nrhs, sstream_);
-        ++merged_launches_;
+        Stage t;
+        t.lay = g.lay;
+        t.nrhs = g.nrhs;
+        t.nseg = (int)g.gs.size();
+        t.total = g.off.back();
+        t.o_seg = put(g.gs);
+        t.o_off = put(g.off);
+        bound_.stages.push_back(t);
       }
       if (!rs.empty() && roff.back() > 0) {
-        ReduceSeg* dr = tick.add(upload(rs, sstream_));
-        int* dro = tick.add(upload(roff, sstream_));
-        launch_reduce_seg(dr, dro, (int)rs.size(), roff.back(), sstream_);
-        ++merged_launches_;
+        Stage t;
+        t.reduce = true;
+        t.nseg = (int)rs.size();
+        t.total = roff.back();
+        t.o_seg = put(rs);
+        t.o_off = put(roff);
+        bound_.stages.push_back(t);
       }
-      HIF_CK(cudaGetLastError());
     }
-    for (Active* a : set)
-      launch_apply_out(a->ub, a->z, a->n3, a->n3, a->nrhs, sstream_);
+    bound_.d = dalloc<char>(host.size(), sstream_);
+    HIF_CK(cudaMemcpyAsync(bound_.d, host.data(), host.size(), cudaMemcpyHostToDevice, sstream_));
+    bound_.ids = std::move(ids);
+  }
+
+  // z = M^{-1} r for every request in `set`: one launch per stage key, layout and
+  // right-hand-side class over all requests that have it.
+  void batched_apply(std::vector<Active*>& set) {
+    bind(set);
+    for (Active* a : set) launch_apply_in(a->rv, a->n3, a->ua, a->ub, a->e->NC, a->nrhs, sstream_);
+    for (const Stage& t : bound_.stages) {
+      const int* off = reinterpret_cast<const int*>(bound_.d + t.o_off);
+      if (t.reduce)
+        launch_reduce_seg(reinterpret_cast<const ReduceSeg*>(bound_.d + t.o_seg), off, t.nseg,
+                          t.total, sstream_);
+      else
+        launch_gemv(reinterpret_cast<const GemvFastSeg*>(bound_.d + t.o_seg), off, t.nseg,
+                    t.total, t.lay, nullptr, nullptr, nullptr, t.nrhs, sstream_);
+      ++merged_launches_;
+    }
     HIF_CK(cudaGetLastError());
-    tick.release(sstream_);
+    for (Active* a : set) launch_apply_out(a->ub, a->z, a->n3, a->n3, a->nrhs, sstream_);
+    HIF_CK(cudaGetLastError());
   }
 
   void solve_loop() {
