@@ -1254,9 +1254,6 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
         int* dow = step.add(upload(otw, stream));
         timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_tcopy(dw, dow, (int)tw.size(), otw.back(), stream); });
       }
-      timed(HIF_KCLASS_SWEEP_PANEL, 0, 0, [&] {
-        launch_sweep_setdiag(dd, dact, (int)active.size(), k0, dinv, stream);
-      });
       HIF_CK(cudaGetLastError());
       step.release(stream);
     }
@@ -1349,9 +1346,6 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
       gemm_batch(rowg, step, stream, HIF_KCLASS_SWEEP_PANEL, timed, 128);
       gemm_batch(gd, step, stream, HIF_KCLASS_GEMM, timed);
       gemm_batch(colg, step, stream, HIF_KCLASS_SWEEP_PANEL, timed, 128);
-      timed(HIF_KCLASS_SWEEP_PANEL, 0, 0, [&] {
-        launch_sweep_setdiag(dd, dact, (int)active.size(), k0, dinv, stream);
-      });
       HIF_CK(cudaGetLastError());
       step.release(stream);
     }

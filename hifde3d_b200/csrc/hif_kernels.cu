@@ -1394,9 +1394,9 @@ void launch_sweep_small(const SweepDesc* d_desc, int nd, int max_n, int* d_statu
 }
 
 // --- blocked sweep ---------------------------------------------------------
-// Step for pivot block K = [k0, k1) of A22: Dinv = B[K, K]^{-1} (k_sweep_diag);
-// the row / column panels and the rank-128 update are batched GEMMs issued by
-// the host; B[K, K] = Dinv (k_sweep_setdiag).
+// Step for pivot block K = [k0, k1) of A22: Dinv = B[K, K]^{-1}, also over B[K, K]
+// (k_pivot_block); the row / column panels and the rank-128 update are batched GEMMs
+// issued by the host.
 // The pivot block of both eliminations, 128 x 128, by 16-wide block steps: one CTA
 // per block, and on the critical path of the top levels, where one or a few blocks
 // remain, so it is built for latency. 16 worker warps hold the block as DMMA
@@ -1670,7 +1670,10 @@ __global__ void __launch_bounds__(kPbThreads, 1)
   double* out = dinv + (long long)di * kSweepNB * kSweepNB;
   for (int e = tid; e < nb * nb; e += kPbThreads) {
     const int i = e % nb, j = e / nb;
-    out[e] = (CHOL && i < j) ? 0.0 : St[i + j * kPbSt];
+    const double v = (CHOL && i < j) ? 0.0 : St[i + j * kPbSt];
+    out[e] = v;
+    // Gauss-Jordan: the step's panels and updates leave block KK alone
+    if (!CHOL) d.B[(k0 + i) + (long long)(k0 + j) * d.n] = v;
   }
 }
 
@@ -1688,25 +1691,6 @@ void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, in
   ensure_smem((const void*)k_pivot_block<true>, kPbSmem);
   k_pivot_block<true><<<nact, kPbThreads, kPbSmem, s>>>(d_desc, d_active, k0, d_dinv, d_status,
                                                         1);
-}
-
-__global__ void k_sweep_setdiag(const SweepDesc* __restrict__ descs,
-                                const int* __restrict__ active, int k0,
-                                const double* __restrict__ dinv) {
-  const int di = active[blockIdx.x];
-  const SweepDesc d = descs[di];
-  const int nb = min(kSweepNB, d.r - k0);
-  const double* Dg = dinv + (long long)di * kSweepNB * kSweepNB;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e % nb, j = e / nb;
-    d.B[(k0 + i) + (long long)(k0 + j) * d.n] = Dg[e];
-  }
-}
-
-void launch_sweep_setdiag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
-                          const double* d_dinv, cudaStream_t s) {
-  if (nact <= 0) return;
-  k_sweep_setdiag<<<nact, 256, 0, s>>>(d_desc, d_active, k0, d_dinv);
 }
 
 // ===========================================================================
@@ -2785,116 +2769,202 @@ void launch_trsm_upper(const double* R, long long ldr, int k, double* B, long lo
 }
 
 // ===========================================================================
-// Pivoted Cholesky ID (mixed precision mode), one CTA per face.
+// Pivoted Cholesky panels: nb steps of a face's G, by one CTA, or a cluster that
+// splits the columns of a wide face (the panel's rows of R stay in shared memory).
+// Bound by the latency of a step: the pivot search, the pivot's column of G from L2 or
+// HBM, the products with the panel's earlier rows. A step is one block barrier (and one
+// cluster barrier): every warp reduces the warps' candidates itself, and the earlier
+// rows' pivot entries are broadcast reads. With R's rows re-read from L2 and a serial
+// search a step took about 15 us (144 faces of 767 columns, 0.5 ms a panel).
 // ===========================================================================
+constexpr int kPcMaxW = 832;  // columns of one CTA: 32 rows of them in shared memory
+__device__ __forceinline__ void argmax_step(double& best, int& bi, double ob, int oi) {
+  if (ob > best || (ob == best && oi < bi)) {
+    best = ob;
+    bi = oi;
+  }
+}
 __global__ void __launch_bounds__(512) k_pchol_panel(const PcholDesc* __restrict__ descs,
                                                      const int* __restrict__ active, int i0,
                                                      int nb, double eps, int* __restrict__ status) {
-  const PcholDesc P = descs[active[blockIdx.x]];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const PcholDesc P = descs[active[blockIdx.x / C]];
   const int n = P.id.n, tid = threadIdx.x, nthr = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
-  extern __shared__ double pc_sm[];
-  double* d = pc_sm;                              // current Schur diagonal
-  int* ch = reinterpret_cast<int*>(pc_sm + n);    // chosen flags
-  __shared__ double red_v[32];
-  __shared__ int red_i[32];
-  __shared__ double pcol[64];                     // R[l, p] for the panel's rows
-  __shared__ int s_p, s_stop;
-  __shared__ double s_dp, s_d0;
+  const int w = (n + C - 1) / C, c0 = rank * w, cols = max(0, min(w, n - c0));
+  extern __shared__ double pc_sm[];  // [row of the panel][own column], ld w
+  __shared__ double s_v[2][16];
+  __shared__ int s_i[2][16];
+  __shared__ double x_v[2][16];  // candidates of the cluster's CTAs
+  __shared__ int x_i[2][16];
+  __shared__ double pcol[32];
   const double* G = P.G;
   double* R = P.R;
-  if (P.info[1]) return;
-  if (i0 == 0) {
-    double mx = 0.0;
-    for (int j = tid; j < n; j += nthr) {
-      const double v = G[j + (long long)j * n];
-      d[j] = v;
-      ch[j] = 0;
-      mx = fmax(mx, v);
-    }
+  if (P.info[1]) return;  // the same in every CTA of the face
+  // own columns tid, tid + nthr: remaining diagonal, -1 once chosen
+  constexpr int Q = 2;
+  double d[Q];
+  double mx = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) red_v[warp] = mx;
+  for (int q = 0; q < Q; ++q) {
+    const int j = tid + q * nthr;
+    d[q] = -1.0;
+    if (j < cols && (i0 == 0 || !P.chosen[c0 + j])) {
+      d[q] = fmax(G[(c0 + j) + (long long)(c0 + j) * n], 0.0);
+      mx = fmax(mx, d[q]);
+    }
+  }
+  double d0;
+  int buf = 0;
+  // best over the face of each thread's (best, index): the same on every thread
+  auto face_argmax = [&](double& best, int& bi) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      argmax_step(best, bi, __shfl_xor_sync(0xffffffffu, best, o),
+                  __shfl_xor_sync(0xffffffffu, bi, o));
+    if (lane == 0) {
+      s_v[buf][warp] = best;
+      s_i[buf][warp] = bi;
+    }
     __syncthreads();
-    if (tid == 0) {
-      double m0 = 0.0;
-      for (int w = 0; w < nw; ++w) m0 = fmax(m0, red_v[w]);
-      s_d0 = m0;
-      *P.d0 = m0;
-      if (!(m0 > 0.0)) atomicOr(status, kStatusIdZero);
+    best = lane < nw ? s_v[buf][lane & 15] : -2.0;
+    bi = lane < nw ? s_i[buf][lane & 15] : INT_MAX;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      argmax_step(best, bi, __shfl_xor_sync(0xffffffffu, best, o),
+                  __shfl_xor_sync(0xffffffffu, bi, o));
+    best = __shfl_sync(0xffffffffu, best, 0);
+    bi = __shfl_sync(0xffffffffu, bi, 0);
+    if (C > 1) {
+      if (tid < C) {
+        cl.map_shared_rank(&x_v[buf][0], tid)[rank] = best;
+        cl.map_shared_rank(&x_i[buf][0], tid)[rank] = bi;
+      }
+      cl.sync();
+      best = x_v[buf][0];
+      bi = x_i[buf][0];
+      for (int q = 1; q < C; ++q) argmax_step(best, bi, x_v[buf][q], x_i[buf][q]);
+    }
+    buf ^= 1;
+  };
+  if (i0 == 0) {
+    int dummy = 0;
+    face_argmax(mx, dummy);
+    d0 = mx;
+    if (tid == 0 && rank == 0) {
+      *P.d0 = d0;
+      if (!(d0 > 0.0)) atomicOr(status, kStatusIdZero);
     }
   } else {
-    for (int j = tid; j < n; j += nthr) {
-      const int c = P.chosen[j];
-      ch[j] = c;
-      d[j] = c ? 0.0 : G[j + (long long)j * n];
-    }
-    if (tid == 0) s_d0 = *P.d0;
+    d0 = *P.d0;
   }
-  if (tid == 0) s_stop = 0;
-  __syncthreads();
-  const double thr = eps * eps * s_d0;
+  const double thr = eps * eps * d0;
   const int iend = min(n, i0 + nb);
   int i = i0;
+  bool stop = false;
   for (; i < iend; ++i) {
     // pivot: largest remaining diagonal, smallest index on ties
-    double best = -1.0;
+    double best = -2.0;
     int bi = INT_MAX;
-    for (int j = tid; j < n; j += nthr)
-      if (!ch[j] && (d[j] > best || (d[j] == best && j < bi))) { best = d[j]; bi = j; }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+    for (int q = 0; q < Q; ++q) {
+      const int j = tid + q * nthr;
+      if (j < cols && d[q] >= 0.0) argmax_step(best, bi, d[q], c0 + j);
     }
-    if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
-    __syncthreads();
-    if (tid == 0) {
-      double b = red_v[0];
-      int bb = red_i[0];
-      for (int w = 1; w < nw; ++w)
-        if (red_v[w] > b || (red_v[w] == b && red_i[w] < bb)) { b = red_v[w]; bb = red_i[w]; }
-      s_p = bb;
-      s_dp = b;
-      // R_ii <= eps R_00 (or nothing left): the rank is i
-      if (bb == INT_MAX || !(b > thr)) s_stop = 1;
-      else P.piv[i] = bb;
+    face_argmax(best, bi);
+    // R_ii <= eps R_00 (or nothing left): the rank is i
+    if (bi == INT_MAX || !(best > thr)) {
+      stop = true;
+      break;
     }
-    __syncthreads();
-    if (s_stop) break;
-    const int p = s_p;
-    const double rii = sqrt(s_dp);
-    for (int l = tid; l < i - i0; l += nthr) pcol[l] = R[(long long)(i0 + l) * n + p];
-    __syncthreads();
-    double* Ri = R + (long long)i * n;
-    for (int j = tid; j < n; j += nthr) {
-      if (ch[j]) { Ri[j] = 0.0; continue; }
-      if (j == p) { Ri[j] = rii; continue; }
+    const int p = bi, rows = i - i0;
+    double g[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int j = c0 + tid + q * nthr;
       // only the lower triangle of G is kept: G[j, p] for j > p, G[p, j] above
-      double sacc = (j > p) ? G[j + (long long)p * n] : G[p + (long long)j * n];
-      for (int l = 0; l < i - i0; ++l) sacc = fma(-pcol[l], R[(long long)(i0 + l) * n + j], sacc);
-      const double r = sacc / rii;
-      Ri[j] = r;
-      d[j] = fma(-r, r, d[j]);
+      g[q] = (tid + q * nthr < cols && d[q] >= 0.0 && j != p)
+                 ? ((j > p) ? G[j + (long long)p * n] : G[p + (long long)j * n]) : 0.0;
     }
-    __syncthreads();
-    if (tid == 0) ch[p] = 1;
-    __syncthreads();
+    const double rii = sqrt(best), inv = 1.0 / rii;
+    const double* pr;  // the earlier rows' entries at the pivot
+    int ps;
+    if (C == 1) {
+      pr = pc_sm + p;
+      ps = w;
+    } else {
+      const int own = p / w;
+      if (tid < rows) pcol[tid] = cl.map_shared_rank(pc_sm, own)[tid * w + (p - own * w)];
+      __syncthreads();
+      pr = pcol;
+      ps = 1;
+    }
+    double* Ri = R + (long long)i * n + c0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int j = tid + q * nthr;
+      if (j >= cols) continue;
+      double r = 0.0;
+      if (d[q] >= 0.0) {
+        if (c0 + j == p) {
+          r = rii;
+          d[q] = -1.0;
+        } else {
+          double s0 = g[q], s1 = 0.0;
+          int l = 0;
+#pragma unroll 4
+          for (; l + 1 < rows; l += 2) {
+            s0 = fma(-pr[l * ps], pc_sm[l * w + j], s0);
+            s1 = fma(-pr[(l + 1) * ps], pc_sm[(l + 1) * w + j], s1);
+          }
+          if (l < rows) s0 = fma(-pr[l * ps], pc_sm[l * w + j], s0);
+          r = (s0 + s1) * inv;
+          // the remaining diagonal stays a candidate: not below zero
+          d[q] = fmax(fma(-r, r, d[q]), 0.0);
+        }
+      }
+      pc_sm[(i - i0) * w + j] = r;
+      Ri[j] = r;
+    }
+    if (tid == 0 && rank == 0) P.piv[i] = p;
   }
-  for (int j = tid; j < n; j += nthr) P.chosen[j] = ch[j];
-  if (tid == 0) {
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int j = tid + q * nthr;
+    if (j < cols) P.chosen[c0 + j] = d[q] < 0.0;
+  }
+  if (C > 1) cl.sync();  // every CTA has read info[1], and the last remote rows
+  if (tid == 0 && rank == 0) {
     P.info[0] = i;
-    if (s_stop || i == n) P.info[1] = 1;
+    if (stop || i == n) P.info[1] = 1;
   }
 }
 
 void launch_pchol_panel(const PcholDesc* d_desc, const int* d_active, int nact, int i0, int nb,
                         double eps, int max_n, int* d_status, cudaStream_t s) {
   if (nact <= 0) return;
-  const size_t smem = (size_t)max_n * (sizeof(double) + sizeof(int));
-  if (smem > 48 * 1024) ensure_smem((const void*)k_pchol_panel, smem);
-  k_pchol_panel<<<nact, 512, smem, s>>>(d_desc, d_active, i0, nb, eps, d_status);
+  int C = 1;
+  while (C < 16 && max_n > C * kPcMaxW) C *= 2;
+  if (C == 16)
+    cudaFuncSetAttribute(k_pchol_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const int w = (max_n + C - 1) / C;
+  const size_t smem = (size_t)nb * w * sizeof(double);
+  ensure_smem((const void*)k_pchol_panel, (size_t)32 * kPcMaxW * sizeof(double));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nact * C, 1, 1);
+  cfg.blockDim = dim3(w <= 256 ? 256 : 512, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_pchol_panel, d_desc, d_active, i0, nb, eps, d_status);
 }
 
 __global__ void __launch_bounds__(512) k_pchol_finish(const PcholDesc* __restrict__ descs) {
@@ -3131,8 +3201,11 @@ void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s) 
   k_pqr_trinv<<<dim3((max_k + kPqrTi - 1) / kPqrTi, nd), 256, smem, s>>>(d_desc);
 }
 
-// A CTA per 32 columns of [R1 | Q1^T T]: with C the columns in shared memory and E
-// read once per CTA, row a needs sum_{l<a}, l = a and sum_{l>a} of E(a, l) C(l).
+// A CTA per 32 columns of [R1 | Q1^T T], C in shared memory: row a needs the sums of
+// E(a, l) C(l) over l < a and l > a. A thread holds 4 rows (32 apart) x 4 columns, so a
+// row block's E entries are coalesced loads shared by four columns and its C entries
+// broadcasts shared by four rows (with one row a thread, bound by its loads: 3.0 ms a
+// launch over 1344 faces of 224 columns).
 constexpr int kPqrFc = 32;
 __global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ descs,
                                                  int* __restrict__ flag) {
@@ -3140,50 +3213,82 @@ __global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ des
   const int k = d.k, cols = d.n - d.o, c0 = blockIdx.x * kPqrFc, tid = threadIdx.x;
   if (c0 >= cols) return;
   const int nc = min(kPqrFc, cols - c0);
-  extern __shared__ double fx_sm[];  // [c][row], ld k | 1
-  const int ld = k | 1;
-  for (int e = tid; e < k * nc; e += 256) {
+  extern __shared__ double fx_sm[];  // [row][c], ld kPqrFc
+  for (int e = tid; e < k * kPqrFc; e += 256) {
     const int a = e % k, c = e / k, j = c0 + c;
-    fx_sm[a + c * ld] = (j < k) ? d.R1[a + (long long)j * k] : d.Z[a + (long long)j * k];
+    fx_sm[a * kPqrFc + c] =
+        c >= nc ? 0.0 : (j < k) ? d.R1[a + (long long)j * k] : d.Z[a + (long long)j * k];
   }
   __syncthreads();
   const int tx = tid & 31, ty = tid >> 5;  // row within 32, group of 4 columns
+  const double* E = d.Z;                   // Q1^T Q1 (symmetric), ld k
   bool bad = false;
-  for (int a0 = 0; a0 < k; a0 += 32) {
-    const int a = a0 + tx;
-    if (a >= k) continue;
-    double lo[4] = {}, up[4] = {};
-    const double* Ea = d.Z + a;  // row a of Q1^T Q1 (symmetric)
-    auto add = [&](double (&acc)[4], int l) {
-      const double e = Ea[(long long)l * k];
-      bad |= !(fabs(e) <= kPqrMaxE);
+  for (int a0 = 0; a0 < k; a0 += 128) {
+    double lo[4][4] = {}, up[4][4] = {}, ed[4] = {};
+    const int a1 = min(k, a0 + 128);
+    auto row = [&](int l, double (&e)[4], double (&c)[4]) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = fma(e, fx_sm[l + (ty * 4 + q) * ld], acc[q]);
+      for (int u = 0; u < 4; ++u) {
+        const int a = a0 + tx + 32 * u;
+        e[u] = a < k ? E[a + (long long)l * k] : 0.0;
+      }
+      const double2* cp = reinterpret_cast<const double2*>(fx_sm + l * kPqrFc + ty * 4);
+      const double2 c01 = cp[0], c23 = cp[1];
+      c[0] = c01.x;
+      c[1] = c01.y;
+      c[2] = c23.x;
+      c[3] = c23.y;
     };
-#pragma unroll 4
-    for (int l = 0; l < a0; ++l) add(lo, l);
-    const int a1 = min(k, a0 + 32);
-    for (int l = a0; l < a1; ++l) {
-      if (l < a) add(lo, l);
-      else if (l > a) add(up, l);
-    }
-#pragma unroll 4
-    for (int l = a1; l < k; ++l) add(up, l);
-    const double ed = Ea[(long long)a * k] - 1.0;
-    bad |= !(fabs(ed) <= kPqrMaxE);
+    auto add = [&](double (&acc)[4][4], int l) {
+      double e[4], c[4];
+      row(l, e, c);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = ty * 4 + q, j = c0 + c;
-      if (c >= nc) continue;
-      const double v = fx_sm[a + c * ld];
-      double* row = d.Rr + (long long)(d.o + a) * d.n;
-      const int col = d.perm[d.o + j];
-      if (j < k) {
-        // column j of R11 = (I + U) R1 (zero below the diagonal)
-        row[col] = (j >= a) ? v + 0.5 * ed * v + up[q] : 0.0;
-      } else {
-        row[col] = v - (lo[q] + 0.5 * ed * v);
-        d.Z[a + (long long)j * k] = v - (lo[q] + ed * v + up[q]);
+      for (int u = 0; u < 4; ++u) {
+        bad |= !(fabs(e[u]) <= kPqrMaxE);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[u][q] = fma(e[u], c[q], acc[u][q]);
+      }
+    };
+#pragma unroll 2
+    for (int l = 0; l < a0; ++l) add(lo, l);
+    for (int l = a0; l < a1; ++l) {
+      double e[4], c[4];
+      row(l, e, c);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int a = a0 + tx + 32 * u;
+        if (l == a) {
+          ed[u] = e[u] - 1.0;
+          e[u] = 0.0;
+        }
+        bad |= !(fabs(e[u]) <= kPqrMaxE) || !(fabs(ed[u]) <= kPqrMaxE);
+        const double el = l < a ? e[u] : 0.0, eu = l > a ? e[u] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          lo[u][q] = fma(el, c[q], lo[u][q]);
+          up[u][q] = fma(eu, c[q], up[u][q]);
+        }
+      }
+    }
+#pragma unroll 2
+    for (int l = a1; l < k; ++l) add(up, l);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int a = a0 + tx + 32 * u;
+      if (a >= k) continue;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int c = ty * 4 + q, j = c0 + c;
+        if (c >= nc) continue;
+        const double v = fx_sm[a * kPqrFc + c];
+        double* out = d.Rr + (long long)(d.o + a) * d.n + d.perm[d.o + j];
+        if (j < k) {
+          // column j of R11 = (I + U) R1 (zero below the diagonal)
+          *out = (j >= a) ? v + 0.5 * ed[u] * v + up[u][q] : 0.0;
+        } else {
+          *out = v - (lo[u][q] + 0.5 * ed[u] * v);
+          d.Z[a + (long long)j * k] = v - (lo[u][q] + ed[u] * v + up[u][q]);
+        }
       }
     }
   }
@@ -3192,7 +3297,7 @@ __global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ des
 
 void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_cols, int* flag, cudaStream_t s) {
   if (nd <= 0) return;
-  const int smem = kPqrFc * (kPqrCap + 1) * (int)sizeof(double);
+  const int smem = kPqrFc * kPqrCap * (int)sizeof(double);
   ensure_smem((const void*)k_pqr_fix, smem);
   k_pqr_fix<<<dim3((max_cols + kPqrFc - 1) / kPqrFc, nd), 256, smem, s>>>(d_desc, flag);
 }

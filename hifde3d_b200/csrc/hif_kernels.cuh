@@ -109,7 +109,7 @@ struct PcholDesc {
   double* d0;      // R_00^2
   IdDesc id;       // outputs (jpvt, rdiag, keep, rank, W) and n
 };
-// nb steps from step i0 for the active faces; dynamic smem n doubles + n ints.
+// nb (at most 32) steps from step i0 for the active faces.
 void launch_pchol_panel(const PcholDesc* d_desc, const int* d_active, int nact, int i0, int nb,
                         double eps, int max_n, int* d_status, cudaStream_t s);
 // Outputs after the last panel: jpvt (skeleton pivots, then the redundant
@@ -357,8 +357,6 @@ void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status
 // above) into dinv (128 x 128 per active block, ld = its width).
 void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
                       double* d_dinv, int* d_status, cudaStream_t s);
-void launch_sweep_setdiag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
-                          const double* d_dinv, cudaStream_t s);
 
 // Column-pivoted Householder QR + rank + interpolation matrix, one CTA per face.
 // W is written to IdDesc::W, which must hold at least n*n/4 + n doubles.
