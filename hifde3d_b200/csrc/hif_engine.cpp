@@ -2454,9 +2454,13 @@ class Engine {
     if (!small_id.empty()) {
       IdDesc* d_idd = tmp.add(upload(small_id, stream));
       long long max_mn = 0;
-      for (const IdDesc& d : small_id) max_mn = std::max(max_mn, (long long)d.m * d.n);
+      int max_m = 0;
+      for (const IdDesc& d : small_id) {
+        max_mn = std::max(max_mn, (long long)d.m * d.n);
+        max_m = std::max(max_m, d.m);
+      }
       timed(HIF_KCLASS_ID, idfl, 0, [&] {
-        launch_id(d_idd, (int)small_id.size(), small_n, eps, d_status, stream, max_mn);
+        launch_id(d_idd, (int)small_id.size(), small_n, eps, d_status, stream, max_mn, max_m);
       });
       idfl = 0;
     }
@@ -2905,8 +2909,8 @@ class Engine {
         const int k = h_info[2 * q], w = d.n - c.o;
         if (k == 0) {
           // nothing of the face is left: rows of zeros, the columns in their order
-          HIF_CK(cudaMemsetAsync(Rr + c.g + (long long)c.o * d.n, 0,
-                                 (size_t)w * d.n * sizeof(double), stream));
+          HIF_CK(cudaMemset2DAsync(Rr + c.g + c.o, d.n * sizeof(double), 0, w * sizeof(double),
+                                   d.n, stream));
           c.o = d.n;
           continue;
         }
@@ -2980,7 +2984,7 @@ class Engine {
         HIF_CK(cudaGetLastError());
         gemm_batch(gq, step, stream, HIF_KCLASS_QR, tm);
         gemm_batch(gz, step, stream, HIF_KCLASS_QR, tm);
-        timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mc, flag, stream); }, 1);
+        timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mk_, mc, flag, stream); }, 1);
         HIF_CK(cudaGetLastError());
         gemm_batch(gu, step, stream, HIF_KCLASS_QR, tm);
       }

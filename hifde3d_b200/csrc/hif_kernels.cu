@@ -104,8 +104,8 @@ __device__ double block_sum(double v, double* scratch) {
 // ===========================================================================
 // Tiles of 32 rows x 64 columns: lane x of warp w assembles row x of columns
 // w, w + 8, ..., w + 56, so a thread's row, its stencil row and its row covers
-// (up to three sources, each turned into a pointer to the source's row) stay in
-// registers, and a column's covers are warp-uniform shared-memory reads.
+// (up to three sources and positions) stay in registers, and a column's covers (each
+// turned into a pointer to the source's column) are warp-uniform shared-memory reads.
 constexpr int kGTM = 32, kGTN = 64;
 
 int gather_tiles(int m, int n) {
@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(256) k_gather(const GatherTarget* __restrict__
   int d = find_desc(tile_off, ntg, t0);
   int dbeg = tile_off[d], dend = tile_off[d + 1];
   __shared__ int s_col[kGTN];
-  __shared__ CoverEntry s_cc[kGTN][kCover];
+  __shared__ int s_src[kGTN][kCover];             // a column's sources, -2: none
+  __shared__ const double* s_base[kGTN][kCover];  // their columns
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int NC2 = NC * NC;
   for (int t = t0; t < t1; ++t) {
@@ -162,42 +163,52 @@ __global__ void __launch_bounds__(256) k_gather(const GatherTarget* __restrict__
     const int local = t - dbeg;
     const int tiles_m = (g.m + kGTM - 1) / kGTM;
     const int i0 = (local % tiles_m) * kGTM, j0 = (local / tiles_m) * kGTN;
-    __syncthreads();  // the previous tile's readers of s_col / s_cc are done
+    __syncthreads();  // the previous tile's readers of the column tables are done
     if (threadIdx.x < kGTN) {
       const int j = j0 + threadIdx.x;
       const int q = (j < g.n) ? g.cols[j] : -1;
       s_col[threadIdx.x] = q;
-      resolve_cover(g, q, dof_src, src_owner, ncell3, s_cc[threadIdx.x]);
+      CoverEntry cc[kCover];
+      resolve_cover(g, q, dof_src, src_owner, ncell3, cc);
+#pragma unroll
+      for (int c = 0; c < kCover; ++c) {
+        const bool has = cc[c].src >= 0;
+        s_src[threadIdx.x][c] = has ? cc[c].src : -2;
+        if (has) {
+          const SourceDesc sd = src[cc[c].src];
+          s_base[threadIdx.x][c] = sd.ptr + (long long)cc[c].pos * sd.ld;
+        } else {
+          s_base[threadIdx.x][c] = nullptr;
+        }
+      }
     }
-    // this thread's row: DOF, stencil row and source rows (a source's entries
-    // are addressed with 32-bit positions times its leading dimension)
+    // this thread's row: DOF, stencil row, sources and its positions in them
     const int i = i0 + lane;
     const int p = (i < g.m) ? g.rows[i] : -1;
     CoverEntry rc[kCover];
     resolve_cover(g, p, dof_src, src_owner, ncell3, rc);
-    const double* rp[kCover];
-    int rs[kCover], rld[kCover];
-#pragma unroll
-    for (int a = 0; a < kCover; ++a) {
-      rs[a] = rc[a].src;
-      rp[a] = nullptr;
-      rld[a] = 0;
-      if (rc[a].src >= 0) {
-        const SourceDesc sd = src[rc[a].src];
-        rp[a] = sd.ptr + rc[a].pos;
-        rld[a] = (int)sd.ld;
-      }
-    }
     __syncthreads();
     if (i < g.m) {
       const bool row_a0 = i < g.a0_skip;
       const bool row_a22 = g.a22_out != nullptr && i < g.r;
       const int ld = (int)g.ld;
       double* orow = g.out + i;
-#pragma unroll 2
+#pragma unroll 4
       for (int cc = warp; cc < kGTN; cc += 8) {
         const int j = j0 + cc;
         if (j >= g.n) break;
+        // sources holding both DOFs, in the column's cover order: a row is in a source
+        // at most once, so its position is selected and one load is issued per column
+        // source (a column's sources are warp-uniform shared-memory reads)
+        double tv[kCover];
+#pragma unroll
+        for (int c = 0; c < kCover; ++c) {
+          const int sc = s_src[cc][c];
+          int pos = -1;
+#pragma unroll
+          for (int a = kCover - 1; a >= 0; --a) pos = rc[a].src == sc ? rc[a].pos : pos;
+          tv[c] = pos >= 0 ? __ldg(s_base[cc][c] + pos) : 0.0;
+        }
         double v = 0.0;
         if (row_a0 || j < g.a0_skip) {
           // stencil term: q - p in {0, -1, 1, -NC, NC, -NC^2, NC^2} -> bands 0..6
@@ -207,16 +218,8 @@ __global__ void __launch_bounds__(256) k_gather(const GatherTarget* __restrict__
             v = band[b * ncell3 + p];
           }
         }
-        // sources holding both DOFs, in the column's cover order (a column cover
-        // is warp-uniform, so an empty one is skipped by the whole warp)
 #pragma unroll
-        for (int c = 0; c < kCover; ++c) {
-          const CoverEntry ce = s_cc[cc][c];
-          if (ce.src < 0) continue;
-#pragma unroll
-          for (int a = 0; a < kCover; ++a)
-            if (rs[a] == ce.src) v += rp[a][(long long)ce.pos * rld[a]];
-        }
+        for (int c = 0; c < kCover; ++c) v += tv[c];
         orow[(long long)j * ld] = v;
         if (row_a22 && j < g.r) g.a22_out[i + (long long)j * g.r] = v;
       }
@@ -1327,70 +1330,157 @@ void launch_gemm_oz(const OzGemm* d_desc, const int* d_tile_off, int nd, int tot
 }
 
 // ===========================================================================
+// Cholesky elimination (symmetric positive definite interiors; the lower
+// triangle of every block is the one read and written).
+//   [A22 A12^T; A12 A11] = [L 0; Y^T I] [I 0; 0 S] [L^T Y; 0 I],
+//   A22 = L L^T, Y = L^{-1} A12^T, S = A11 - Y^T Y.
+// The factor keeps L (for F u), L^{-1} and Y (for F^{-1} u): in exact
+// arithmetic X = L^{-T} Y and A22^{-1} = L^{-T} L^{-1}, the reference's
+// Schur() outputs (include/Schur.hpp:72-100).
+// ===========================================================================
+
+// ===========================================================================
 // Gauss-Jordan sweep. For B = [A22 A21; A12 A11] (red first), eliminating
 // pivots 0..r-1 in place gives [A22^{-1} X; * A11 - A12 X] with
 // X = A22^{-1} A21: the three outputs of the reference's Schur().
 // Entries of the bottom-left block whose column is already pivoted are never
 // read again and are not updated.
 // ===========================================================================
-__global__ void __launch_bounds__(256) k_sweep_small(const SweepDesc* __restrict__ descs,
-                                                     int* __restrict__ status) {
+//
+// Small blocks (n <= kSmallSweepN), a CTA each, by Gauss-Jordan or (CHOL) Cholesky: the
+// block lives in registers, thread (tx, ty) of a 16 x 16 grid holding rows tx + 16a and
+// columns ty + 16b, and a pivot is one barrier: the owners of row and column k publish
+// them (two buffers, alternating) and every thread updates its TS x TS entries.
+//   Gauss-Jordan, p = a_kk: row k * (1 / p); column k * (-1 / p); the rest a - a_ik r_j.
+//   Cholesky, t = 1 / sqrt(a_kk), l = t a_ik (i > k): column k of [L; Y^T] is l, kept in
+//   shared memory; row k * t (left of k: L^{-1}; its diagonal t); rows below: a - l_i r_j,
+//   with -l_i t in column k.
+// Bound by the barrier and the publish of a pivot. In shared memory, with four barriers
+// and an integer division per entry, level 0's 27-of-81 blocks of n = 128 took 7.8 ms
+// (Cholesky 6.5 ms); reading and writing them takes 0.5 ms.
+template <int TS, bool CHOL>
+__global__ void __launch_bounds__(256, TS == 6 ? 2 : 1) k_elim_small(const SweepDesc* __restrict__ descs,
+                                                    int* __restrict__ status) {
   const SweepDesc d = descs[blockIdx.x];
-  const int n = d.n, r = d.r;
-  extern __shared__ double S[];  // n x n, ld n
+  const int n = d.n, r = d.r, s = n - r;
+  extern __shared__ double S[];  // n x n, ld n: staging
+  __shared__ double rowk[2][16 * TS], colk[2][16 * TS];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
   const int nn = n * n;
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) S[e] = d.B[e];
+#pragma unroll 8
+  for (int e = tid; e < nn; e += 256) S[e] = d.B[e];
   __syncthreads();
-  __shared__ double s_ip;
+  double a[TS][TS];
+#pragma unroll
+  for (int u = 0; u < TS; ++u)
+#pragma unroll
+    for (int v = 0; v < TS; ++v) {
+      const int i = tx + 16 * u, j = ty + 16 * v;
+      // Cholesky: the lower triangle, mirrored
+      a[u][v] = (i < n && j < n) ? ((CHOL && i < j) ? S[j + i * n] : S[i + j * n]) : 0.0;
+    }
   int bad = 0;
-  for (int k = 0; k < r; ++k) {
-    if (threadIdx.x == 0) {
-      const double p = S[k + k * n];
-      if (!(fabs(p) > 1e-300) || !isfinite(p)) bad = 1;
-      s_ip = 1.0 / p;
+#pragma unroll
+  for (int kb = 0; kb < TS; ++kb) {
+    for (int kk = 0; kk < 16; ++kk) {
+      const int k = kb * 16 + kk, buf = k & 1;
+      if (k >= r) break;
+      if (tx == kk) {
+#pragma unroll
+        for (int v = 0; v < TS; ++v) rowk[buf][ty + 16 * v] = a[kb][v];
+      }
+      if (ty == kk) {
+#pragma unroll
+        for (int u = 0; u < TS; ++u) colk[buf][tx + 16 * u] = a[u][kb];
+      }
+      __syncthreads();
+      const double p = rowk[buf][k];
+      double t;
+      if (CHOL) {
+        if (!(p > 1e-300) || !isfinite(p)) bad = 1;
+        t = rsqrt(fabs(p) > 1e-300 ? fabs(p) : 1.0);
+      } else {
+        if (!(fabs(p) > 1e-300) || !isfinite(p)) bad = 1;
+        t = 1.0 / p;
+      }
+      double rj[TS], ci[TS];
+#pragma unroll
+      for (int v = 0; v < TS; ++v)
+        rj[v] = (ty + 16 * v == k) ? t : rowk[buf][ty + 16 * v] * t;
+#pragma unroll
+      for (int u = 0; u < TS; ++u) {
+        const int i = tx + 16 * u;
+        ci[u] = colk[buf][i];
+        if (CHOL) ci[u] = i > k ? ci[u] * t : 0.0;
+      }
+      // column k restarts from zero (Cholesky: below the diagonal)
+      if (ty == kk) {
+#pragma unroll
+        for (int u = 0; u < TS; ++u)
+          if (!CHOL || tx + 16 * u > k) a[u][kb] = 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < TS; ++u)
+#pragma unroll
+        for (int v = 0; v < TS; ++v) a[u][v] = fma(-ci[u], rj[v], a[u][v]);
+      if (tx == kk) {
+#pragma unroll
+        for (int v = 0; v < TS; ++v) a[kb][v] = rj[v];
+      }
+      if (CHOL && ty == kk) {
+        // column k of [L; Y^T], zero above the diagonal
+        const double q = fabs(p) > 1e-300 ? fabs(p) : 1.0;
+#pragma unroll
+        for (int u = 0; u < TS; ++u) {
+          const int i = tx + 16 * u;
+          if (i < n) S[i + k * n] = i == k ? q * t : ci[u];
+        }
+      }
     }
-    __syncthreads();
-    const double ip = s_ip;
-    // new pivot row
-    for (int j = threadIdx.x; j < n; j += blockDim.x)
-      if (j != k) S[k + j * n] *= ip;
-    __syncthreads();
-    // rank-1 update of every entry outside row / column k
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-      const int i = e % n, j = e / n;
-      if (i == k || j == k) continue;
-      if (i >= r && j < k) continue;
-      S[e] = fma(-S[i + k * n], S[k + j * n], S[e]);
+  }
+  if (bad && tid == 0) atomicOr(status, kStatusTinyPivot);
+  __syncthreads();
+  // compact outputs: A22^{-1} or L^{-1} (r x r), X or Y (r x s), L; A11 - A12 X stays
+  // in B
+#pragma unroll
+  for (int u = 0; u < TS; ++u)
+#pragma unroll
+    for (int v = 0; v < TS; ++v) {
+      const int i = tx + 16 * u, j = ty + 16 * v;
+      if (i >= n || j >= n) continue;
+      if (i < r && j < r) d.a22inv[i + (long long)j * r] = (CHOL && i < j) ? 0.0 : a[u][v];
+      else if (!CHOL && i < r) d.X[i + (long long)(j - r) * r] = a[u][v];
+      else if (i >= r && j >= r) d.B[i + (long long)j * n] = a[u][v];
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < r; i += blockDim.x)
-      if (i != k) S[i + k * n] *= -ip;
-    if (threadIdx.x == 0) S[k + k * n] = ip;
-    __syncthreads();
-  }
-  if (bad) atomicOr(status, kStatusTinyPivot);
-  // compact outputs: A22^{-1} (r x r), X (r x s); T = A11 - A12 X stays in B
-  const int s = n - r;
-  for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-    const int i = e % r, j = e / r;
-    d.a22inv[e] = S[i + j * n];
-  }
-  for (int e = threadIdx.x; e < r * s; e += blockDim.x) {
-    const int i = e % r, j = e / r;
-    d.X[e] = S[i + (r + j) * n];
-  }
-  for (int e = threadIdx.x; e < s * s; e += blockDim.x) {
-    const int i = e % s, j = e / s;
-    d.B[(r + i) + (long long)(r + j) * n] = S[(r + i) + (r + j) * n];
+  if (CHOL) {
+    for (int j = warp; j < r; j += 8)
+      for (int i = lane; i < r; i += 32) d.L[i + (long long)j * r] = S[i + j * n];
+    for (int j = warp; j < s; j += 8)
+      for (int i = lane; i < r; i += 32) d.X[i + (long long)j * r] = S[(r + j) + i * n];
   }
 }
 
-void launch_sweep_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
-                        cudaStream_t s) {
+template <bool CHOL>
+void launch_elim_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
+                       cudaStream_t s) {
   if (nd <= 0) return;
   const size_t smem = (size_t)max_n * max_n * sizeof(double);
-  ensure_smem((const void*)k_sweep_small, kSmallSweepN * kSmallSweepN * sizeof(double));
-  k_sweep_small<<<nd, 256, smem, s>>>(d_desc, d_status);
+  if (max_n <= 96) {
+    ensure_smem((const void*)k_elim_small<6, CHOL>, 96 * 96 * sizeof(double));
+    k_elim_small<6, CHOL><<<nd, 256, smem, s>>>(d_desc, d_status);
+  } else {
+    ensure_smem((const void*)k_elim_small<10, CHOL>,
+                kSmallSweepN * kSmallSweepN * sizeof(double));
+    k_elim_small<10, CHOL><<<nd, 256, smem, s>>>(d_desc, d_status);
+  }
+}
+void launch_sweep_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
+                        cudaStream_t s) {
+  launch_elim_small<false>(d_desc, nd, max_n, d_status, s);
+}
+void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
+                       cudaStream_t s) {
+  launch_elim_small<true>(d_desc, nd, max_n, d_status, s);
 }
 
 // --- blocked sweep ---------------------------------------------------------
@@ -1694,99 +1784,6 @@ void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, in
 }
 
 // ===========================================================================
-// Cholesky elimination (symmetric positive definite interiors; the lower
-// triangle of every block is the one read and written).
-//   [A22 A12^T; A12 A11] = [L 0; Y^T I] [I 0; 0 S] [L^T Y; 0 I],
-//   A22 = L L^T, Y = L^{-1} A12^T, S = A11 - Y^T Y.
-// The factor keeps L (for F u), L^{-1} and Y (for F^{-1} u): in exact
-// arithmetic X = L^{-T} Y and A22^{-1} = L^{-T} L^{-1}, the reference's
-// Schur() outputs (include/Schur.hpp:72-100).
-// ===========================================================================
-
-// Small blocks whole in shared memory. Right-looking: for k < r, d = sqrt(S_kk),
-// column k below the diagonal / d, then S_ij -= S_ik S_jk for k < j <= i; after
-// r steps S[0:r, 0:r] = L, S[r:n, 0:r] = Y^T and S[r:n, r:n] = A11 - Y^T Y
-// (lower). L^{-1} then replaces L in place by Gauss-Jordan on the lower
-// triangle (entries above the diagonal stay zero under those steps).
-__global__ void __launch_bounds__(256) k_chol_small(const SweepDesc* __restrict__ descs,
-                                                    int* __restrict__ status) {
-  const SweepDesc d = descs[blockIdx.x];
-  const int n = d.n, r = d.r, s = n - r;
-  extern __shared__ double S[];  // n x n, ld n; lower triangle used
-  const int nn = n * n;
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    S[e] = (i >= j) ? d.B[e] : 0.0;
-  }
-  __syncthreads();
-  __shared__ double s_d;
-  int bad = 0;
-  for (int k = 0; k < r; ++k) {
-    if (threadIdx.x == 0) {
-      const double p = S[k + k * n];
-      if (!(p > 1e-300) || !isfinite(p)) bad = 1;
-      s_d = sqrt(fabs(p) > 1e-300 ? fabs(p) : 1.0);
-    }
-    __syncthreads();
-    const double dk = s_d, idk = 1.0 / dk;
-    for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) S[i + k * n] *= idk;
-    if (threadIdx.x == 0) S[k + k * n] = dk;
-    __syncthreads();
-    const int m = n - k - 1;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int ii = e % m, jj = e / m;
-      if (ii < jj) continue;
-      const int i = k + 1 + ii, j = k + 1 + jj;
-      S[i + j * n] = fma(-S[i + k * n], S[j + k * n], S[i + j * n]);
-    }
-    __syncthreads();
-  }
-  // outputs: L (zeros above), Y = (S[r:n, 0:r])^T, Schur complement (mirrored)
-  for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-    const int i = e % r, j = e / r;
-    d.L[e] = (i >= j) ? S[i + j * n] : 0.0;
-  }
-  for (int e = threadIdx.x; e < r * s; e += blockDim.x) {
-    const int i = e % r, j = e / r;
-    d.X[e] = S[(r + j) + i * n];
-  }
-  for (int e = threadIdx.x; e < s * s; e += blockDim.x) {
-    const int i = e % s, j = e / s;
-    const int a = max(i, j), b = min(i, j);
-    d.B[(r + i) + (long long)(r + j) * n] = S[(r + a) + (r + b) * n];
-  }
-  __syncthreads();
-  // L^{-1} in place (lower triangle of S[0:r, 0:r])
-  for (int k = 0; k < r; ++k) {
-    const double ip = 1.0 / S[k + k * n];
-    for (int j = threadIdx.x; j < k; j += blockDim.x) S[k + j * n] *= ip;
-    __syncthreads();
-    const int m = r - k - 1;
-    for (int e = threadIdx.x; e < m * k; e += blockDim.x) {
-      const int i = k + 1 + e % m, j = e / m;
-      S[i + j * n] = fma(-S[i + k * n], S[k + j * n], S[i + j * n]);
-    }
-    __syncthreads();
-    for (int i = k + 1 + threadIdx.x; i < r; i += blockDim.x) S[i + k * n] *= -ip;
-    if (threadIdx.x == 0) S[k + k * n] = ip;
-    __syncthreads();
-  }
-  if (bad) atomicOr(status, kStatusTinyPivot);
-  for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-    const int i = e % r, j = e / r;
-    d.a22inv[e] = (i >= j) ? S[i + j * n] : 0.0;
-  }
-}
-
-void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
-                       cudaStream_t s) {
-  if (nd <= 0) return;
-  const size_t smem = (size_t)max_n * max_n * sizeof(double);
-  ensure_smem((const void*)k_chol_small, kSmallSweepN * kSmallSweepN * sizeof(double));
-  k_chol_small<<<nd, 256, smem, s>>>(d_desc, d_status);
-}
-
-// ===========================================================================
 // Interpolative decomposition (one CTA per face).
 //
 // Column-pivoted Householder QR (Businger-Golub greedy pivoting on partial
@@ -1993,6 +1990,195 @@ __global__ void __launch_bounds__(512) k_id(const IdDesc* __restrict__ descs, do
   }
   if (stage_off > 0)
     for (long long e = threadIdx.x; e < (long long)m * n; e += blockDim.x) d.M[e] = M[e];
+}
+
+// The same for narrow faces (n <= 64 columns, m <= 32 RPL rows), NW warps a face, the
+// face in shared memory for good. A step is one barrier: every warp finds the pivot and
+// forms the reflector itself (columns are swapped by index only, the reflector is
+// applied unscaled), then takes its columns through registers: product, update, norm
+// downdate or recomputation. The index and norm arrays alternate between two buffers.
+// Bound by a step's instructions and latency (every warp's reflector among them).
+// k_id's step has about ten barriers: level 1's 11520 faces of 49 columns of n = 128
+// took 20.6 ms there, 15.2 ms here; 12 such faces 0.36 and 0.19 ms.
+template <int NW, int RPL>
+__global__ void __launch_bounds__(NW == 1 ? 128 : NW * 32)
+    k_id_small(const IdDesc* __restrict__ descs, int nd, double eps, int* __restrict__ status,
+               int max_mn, int max_n) {
+  const int lane = threadIdx.x & 31, wi = NW == 1 ? 0 : threadIdx.x >> 5;
+  const int slot = NW == 1 ? threadIdx.x >> 5 : 0;
+  const int fi = NW == 1 ? blockIdx.x * 4 + slot : blockIdx.x;
+  if (fi >= nd) return;
+  const IdDesc d = descs[fi];
+  const int m = d.m, n = d.n;
+  extern __shared__ double is_sm[];
+  double* S = is_sm + (size_t)slot * (max_mn + 8 * max_n);
+  double* vn1 = S + max_mn;        // 2 x n
+  double* vn2 = vn1 + 2 * max_n;   // 2 x n
+  double* rd = vn2 + 2 * max_n;    // R's diagonal
+  double* sc = rd + max_n;         // scale of the reflector below it
+  int* cof = reinterpret_cast<int*>(sc + max_n);  // 2 x n: column at each position
+  int* jp = cof + 2 * max_n;
+  int* pos = jp + max_n;
+  auto sync = [&] {
+    if (NW == 1) __syncwarp();
+    else __syncthreads();
+  };
+  const double tol3z = sqrt(DBL_EPSILON * 0.5);
+  for (int e = (wi << 5) + lane; e < m * n; e += NW * 32) S[e] = d.M[e];
+  sync();
+  for (int j = wi; j < n; j += NW) {
+    double t = 0.0;
+    for (int r = lane; r < m; r += 32) t = fma(S[r + j * m], S[r + j * m], t);
+    t = sqrt(warp_sum(t));
+    if (lane == 0) {
+      vn1[j] = vn2[j] = t;
+      cof[j] = j;
+    }
+  }
+  sync();
+  const int steps = min(m, n);
+  for (int i = 0; i < steps; ++i) {
+    const int b = (i & 1) * max_n, nb = max_n - b;
+    // pivot: first position of the largest norm (or the prescribed column)
+    double best = -1.0;
+    int pvt = INT_MAX;
+    const int want = d.order ? d.order[i] : -1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = i + lane + 32 * h;
+      if (j >= n) continue;
+      const double v = d.order ? (cof[b + j] == want ? 1.0 : -1.0) : vn1[b + j];
+      if (v > best) {
+        best = v;
+        pvt = j;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, pvt, o);
+      if (ob > best || (ob == best && oi < pvt)) {
+        best = ob;
+        pvt = oi;
+      }
+    }
+    if (pvt == INT_MAX) pvt = i;
+    const int ci = cof[b + pvt];
+    const double* x = S + ci * m;
+    const double alpha = x[i];
+    double xr[RPL], xs[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int r = lane + 32 * u;
+      xr[u] = (r > i && r < m) ? x[r] : 0.0;
+      xs[u & 1] = fma(xr[u], xr[u], xs[u & 1]);
+    }
+    const double x2 = warp_sum(xs[0] + xs[1]);
+    double tau = 0.0, beta = alpha, scal = 1.0;
+    if (x2 != 0.0) {
+      beta = -copysign(sqrt(fma(alpha, alpha, x2)), alpha);
+      tau = (beta - alpha) / beta;
+      scal = 1.0 / (alpha - beta);
+    }
+    if (wi == 0 && lane == 0) {
+      rd[i] = beta;
+      sc[i] = scal;
+      jp[i] = ci;
+    }
+    for (int j = i + 1 + wi; j < n; j += NW) {
+      const int from = j == pvt ? i : j;  // position pvt takes over position i's column
+      const int cj = cof[b + from];
+      double v1 = vn1[b + from], v2 = vn2[b + from];
+      double* c = S + cj * m;
+      double ar[RPL], ws[2] = {0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < RPL; ++u) {
+        const int r = lane + 32 * u;
+        ar[u] = (r > i && r < m) ? c[r] : 0.0;
+        ws[u & 1] = fma(xr[u], ar[u], ws[u & 1]);
+      }
+      double aij = c[i];
+      double w = tau * fma(scal, warp_sum(ws[0] + ws[1]), aij);
+      aij -= w;
+      w *= scal;
+      double ns[2] = {0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < RPL; ++u) {
+        const int r = lane + 32 * u;
+        ar[u] = fma(-w, xr[u], ar[u]);
+        ns[u & 1] = fma(ar[u], ar[u], ns[u & 1]);
+        if (r > i && r < m) c[r] = ar[u];
+      }
+      // partial norm downdate, recomputed on cancellation
+      if (v1 != 0.0) {
+        double temp = fabs(aij) / v1;
+        temp = fmax(1.0 - temp * temp, 0.0);
+        const double q = v1 / v2;
+        if (temp * q * q <= tol3z) v1 = v2 = (i + 1 < m) ? sqrt(warp_sum(ns[0] + ns[1])) : 0.0;
+        else v1 *= sqrt(temp);
+      }
+      __syncwarp();  // every lane has read c[i]
+      if (lane == 0) {
+        c[i] = aij;
+        vn1[nb + j] = v1;
+        vn2[nb + j] = v2;
+        cof[nb + j] = cj;
+      }
+    }
+    sync();
+  }
+  // rank test on every diagonal entry
+  const double r00 = fabs(rd[0]), tol = r00 * eps;
+  const bool k0 = lane < n && fabs(rd[min(lane, n - 1)]) > tol;
+  const bool k1 = lane + 32 < n && fabs(rd[min(lane + 32, n - 1)]) > tol;
+  const unsigned m0 = __ballot_sync(0xffffffffu, k0), m1 = __ballot_sync(0xffffffffu, k1);
+  const int k = __popc(m0) + __popc(m1);
+  if (wi == 0) {
+    const unsigned below = (1u << lane) - 1u;
+    const int q0 = __popc(m0 & below), q1 = __popc(m0) + __popc(m1 & below);
+    if (lane < n) pos[k0 ? q0 : k + lane - q0] = lane;
+    if (lane + 32 < n) pos[k1 ? q1 : k + lane + 32 - q1] = lane + 32;
+    if (lane == 0) {
+      *d.rank = k;
+      if (r00 == 0.0) atomicOr(status, kStatusIdZero);
+    }
+    for (int h = 0; h < 2; ++h) {
+      const int j = lane + 32 * h;
+      if (j >= n) continue;
+      d.jpvt[j] = jp[j];
+      d.keep[j] = h ? k1 : k0;
+      d.rdiag[j] = rd[j];
+    }
+  }
+  sync();
+  // W = R_skel^{-1} W_full, a warp per redundant column, lanes over the rows. at(r, c):
+  // the QR array as geqp3 leaves it (R, and the scaled reflectors below)
+  auto at = [&](int r, int c) {
+    const double v = S[r + jp[c] * m];
+    return r < c ? v : (r == c ? rd[c] : v * sc[c]);
+  };
+  for (int q = wi; q < n - k; q += NW) {
+    const int c = pos[k + q];
+    double x[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int a = lane + 32 * h;
+      x[h] = (a < k && c >= a) ? at(pos[a], c) : 0.0;
+    }
+    for (int a = k - 1; a >= 0; --a) {
+      const double xa =
+          __shfl_sync(0xffffffffu, a < 32 ? x[0] : x[1], a & 31) / at(pos[a], a);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = lane + 32 * h;
+        if (t == a) x[h] = xa;
+        else if (t < a) x[h] = fma(-at(pos[t], a), xa, x[h]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (lane + 32 * h < k) d.W[(long long)q * k + lane + 32 * h] = x[h];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2273,9 +2459,31 @@ cudaError_t launch_id_group(const IdGroupDesc* d_desc, int nd, int group, double
   return cudaGetLastError();
 }
 
+template <int NW, int RPL>
+static void launch_id_small(const IdDesc* d_desc, int nd, int max_n, double eps, int* d_status,
+                            cudaStream_t s, int max_mn) {
+  const int per = NW == 1 ? 4 : 1;
+  const size_t smem = (size_t)per * (max_mn + 8 * max_n) * sizeof(double);
+  ensure_smem((const void*)k_id_small<NW, RPL>, smem);
+  k_id_small<NW, RPL><<<(nd + per - 1) / per, NW == 1 ? 128 : NW * 32, smem, s>>>(
+      d_desc, nd, eps, d_status, max_mn, max_n);
+}
+
 void launch_id(const IdDesc* d_desc, int nd, int max_n, double eps, int* d_status,
-               cudaStream_t s, long long max_mn) {
+               cudaStream_t s, long long max_mn, int max_m) {
   if (nd <= 0) return;
+  // narrow faces that fit in shared memory, their M not needed afterwards: a warp a face
+  // up to 16 columns and 128 rows, else sixteen
+  if (max_mn > 0 && max_m > 0 && max_n <= 64 && max_m <= 640 &&
+      (size_t)(max_mn + 8 * max_n) * sizeof(double) <= (size_t)220 * 1024) {
+    if (max_m <= 128 && max_n <= 16)
+      launch_id_small<1, 4>(d_desc, nd, max_n, eps, d_status, s, (int)max_mn);
+    else if (max_m <= 128)
+      launch_id_small<16, 4>(d_desc, nd, max_n, eps, d_status, s, (int)max_mn);
+    else
+      launch_id_small<16, 20>(d_desc, nd, max_n, eps, d_status, s, (int)max_mn);
+    return;
+  }
   size_t smem = (size_t)max_n * 2 * sizeof(double) + 64 * sizeof(double) +
                 (size_t)max_n * 3 * sizeof(int) + 32 * sizeof(int);
   // faces that fit run from shared memory (the Householder updates then read
@@ -3202,76 +3410,81 @@ void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s) 
 }
 
 // A CTA per 32 columns of [R1 | Q1^T T], C in shared memory: row a needs the sums of
-// E(a, l) C(l) over l < a and l > a. A thread holds 4 rows (32 apart) x 4 columns, so a
-// row block's E entries are coalesced loads shared by four columns and its C entries
-// broadcasts shared by four rows (with one row a thread, bound by its loads: 3.0 ms a
-// launch over 1344 faces of 224 columns).
+// E(a, l) C(l) over l < a and l > a. A thread holds 4 rows (32 apart) x 4 columns; E goes
+// through shared memory 32 columns at a time, in ascending l, so a row block's running
+// sum is the first until its diagonal block and the second after it. (Reading E from L2
+// at every l, bound by that latency: 3.0 ms a launch over 1344 faces of 224 columns.)
 constexpr int kPqrFc = 32;
-__global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ descs,
-                                                 int* __restrict__ flag) {
+__global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ descs,
+                                                    int* __restrict__ flag) {
   const PqrDesc d = descs[blockIdx.y];
   const int k = d.k, cols = d.n - d.o, c0 = blockIdx.x * kPqrFc, tid = threadIdx.x;
   if (c0 >= cols) return;
   const int nc = min(kPqrFc, cols - c0);
   extern __shared__ double fx_sm[];  // [row][c], ld kPqrFc
+  __shared__ double Es[32][128];
   for (int e = tid; e < k * kPqrFc; e += 256) {
     const int a = e % k, c = e / k, j = c0 + c;
     fx_sm[a * kPqrFc + c] =
         c >= nc ? 0.0 : (j < k) ? d.R1[a + (long long)j * k] : d.Z[a + (long long)j * k];
   }
-  __syncthreads();
   const int tx = tid & 31, ty = tid >> 5;  // row within 32, group of 4 columns
   const double* E = d.Z;                   // Q1^T Q1 (symmetric), ld k
   bool bad = false;
   for (int a0 = 0; a0 < k; a0 += 128) {
-    double lo[4][4] = {}, up[4][4] = {}, ed[4] = {};
-    const int a1 = min(k, a0 + 128);
-    auto row = [&](int l, double (&e)[4], double (&c)[4]) {
+    double lo[4][4] = {}, acc[4][4] = {}, ed[4] = {};
+    const int nu = min(4, (k - a0 + 31) / 32);
+    for (int l0 = 0; l0 < k; l0 += 32) {
+      const int nl = min(32, k - l0);
+      __syncthreads();
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int a = a0 + tx + 32 * u;
-        e[u] = a < k ? E[a + (long long)l * k] : 0.0;
+      for (int q = 0; q < 16; ++q) {
+        const int e = tid + 256 * q, r = e & 127, l = e >> 7, a = a0 + r;
+        double v = (l < nl && a < k) ? E[a + (long long)(l0 + l) * k] : 0.0;
+        if (l < nl && a == l0 + l) v -= 1.0;
+        bad |= !(fabs(v) <= kPqrMaxE);
+        Es[l][r] = v;
       }
-      const double2* cp = reinterpret_cast<const double2*>(fx_sm + l * kPqrFc + ty * 4);
-      const double2 c01 = cp[0], c23 = cp[1];
-      c[0] = c01.x;
-      c[1] = c01.y;
-      c[2] = c23.x;
-      c[3] = c23.y;
-    };
-    auto add = [&](double (&acc)[4][4], int l) {
-      double e[4], c[4];
-      row(l, e, c);
+      __syncthreads();
+      const int ud = (l0 - a0) / 32;  // row block of this chunk's diagonal, if in [0, 4)
+      const bool diag = l0 >= a0 && ud < 4;
+      for (int l = 0; l < nl; ++l) {
+        const double2* cp = reinterpret_cast<const double2*>(fx_sm + (l0 + l) * kPqrFc + ty * 4);
+        const double2 c01 = cp[0], c23 = cp[1];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        bad |= !(fabs(e[u]) <= kPqrMaxE);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[u][q] = fma(e[u], c[q], acc[u][q]);
-      }
-    };
-#pragma unroll 2
-    for (int l = 0; l < a0; ++l) add(lo, l);
-    for (int l = a0; l < a1; ++l) {
-      double e[4], c[4];
-      row(l, e, c);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int a = a0 + tx + 32 * u;
-        if (l == a) {
-          ed[u] = e[u] - 1.0;
-          e[u] = 0.0;
+        for (int u = 0; u < 4; ++u) {
+          if (u >= nu) break;
+          const double e = (diag && u == ud) ? 0.0 : Es[l][tx + 32 * u];
+          acc[u][0] = fma(e, c01.x, acc[u][0]);
+          acc[u][1] = fma(e, c01.y, acc[u][1]);
+          acc[u][2] = fma(e, c23.x, acc[u][2]);
+          acc[u][3] = fma(e, c23.y, acc[u][3]);
         }
-        bad |= !(fabs(e[u]) <= kPqrMaxE) || !(fabs(ed[u]) <= kPqrMaxE);
-        const double el = l < a ? e[u] : 0.0, eu = l > a ? e[u] : 0.0;
+      }
+      if (diag) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          lo[u][q] = fma(el, c[q], lo[u][q]);
-          up[u][q] = fma(eu, c[q], up[u][q]);
+        for (int u = 0; u < 4; ++u) {
+          if (u != ud) continue;
+          double dn[4] = {0.0, 0.0, 0.0, 0.0};
+          for (int l = 0; l < nl; ++l) {
+            const double e = Es[l][tx + 32 * u];
+            const double el = l < tx ? e : 0.0, eu = l > tx ? e : 0.0;
+            if (l == tx) ed[u] = e;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const double c = fx_sm[(l0 + l) * kPqrFc + ty * 4 + q];
+              acc[u][q] = fma(el, c, acc[u][q]);
+              dn[q] = fma(eu, c, dn[q]);
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            lo[u][q] = acc[u][q];
+            acc[u][q] = dn[q];
+          }
         }
       }
     }
-#pragma unroll 2
-    for (int l = a1; l < k; ++l) add(up, l);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int a = a0 + tx + 32 * u;
@@ -3281,13 +3494,13 @@ __global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ des
         const int c = ty * 4 + q, j = c0 + c;
         if (c >= nc) continue;
         const double v = fx_sm[a * kPqrFc + c];
-        double* out = d.Rr + (long long)(d.o + a) * d.n + d.perm[d.o + j];
+        double* out = d.Rr + (long long)d.perm[d.o + j] * d.n + d.o + a;
         if (j < k) {
           // column j of R11 = (I + U) R1 (zero below the diagonal)
-          *out = (j >= a) ? v + 0.5 * ed[u] * v + up[u][q] : 0.0;
+          *out = (j >= a) ? v + 0.5 * ed[u] * v + acc[u][q] : 0.0;
         } else {
           *out = v - (lo[u][q] + 0.5 * ed[u] * v);
-          d.Z[a + (long long)j * k] = v - (lo[u][q] + ed[u] * v + up[u][q]);
+          d.Z[a + (long long)j * k] = v - (lo[u][q] + ed[u] * v + acc[u][q]);
         }
       }
     }
@@ -3295,10 +3508,11 @@ __global__ void __launch_bounds__(256) k_pqr_fix(const PqrDesc* __restrict__ des
   if (bad) atomicOr(flag, 1);
 }
 
-void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_cols, int* flag, cudaStream_t s) {
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, int* flag,
+                    cudaStream_t s) {
   if (nd <= 0) return;
-  const int smem = kPqrFc * kPqrCap * (int)sizeof(double);
-  ensure_smem((const void*)k_pqr_fix, smem);
+  const int smem = kPqrFc * max_k * (int)sizeof(double);
+  ensure_smem((const void*)k_pqr_fix, kPqrFc * kPqrCap * sizeof(double));
   k_pqr_fix<<<dim3((max_cols + kPqrFc - 1) / kPqrFc, nd), 256, smem, s>>>(d_desc, flag);
 }
 
@@ -3312,9 +3526,9 @@ __global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ o
   if (tid == 0) s_k = s_last = 0;
   for (int i = tid; i < n; i += nthr) pn_sm[i] = o.perm[i];
   __syncthreads();
-  const double r00 = fabs(o.Rr[pn_sm[0]]), tol = r00 * eps;
+  const double r00 = fabs(o.Rr[(long long)pn_sm[0] * n]), tol = r00 * eps;
   for (int i = tid; i < n; i += nthr) {
-    const double v = o.Rr[(long long)i * n + pn_sm[i]];
+    const double v = o.Rr[(long long)pn_sm[i] * n + i];
     const int kp = fabs(v) > tol;
     if (blockIdx.y == 0) {
       o.id.jpvt[i] = pn_sm[i];
@@ -3333,11 +3547,11 @@ __global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ o
     if (s_last != k) atomicOr(flag, 2);
     if (r00 == 0.0) atomicOr(status, kStatusIdZero);
   }
-  // rows of R by position: R11 (ld k, upper) and R12, split over the face's CTAs
+  // R by position: R11 (ld k, upper) and R12, split over the face's CTAs
   for (long long e = tid + (long long)blockIdx.y * nthr; e < (long long)k * n;
        e += (long long)nthr * gridDim.y) {
-    const int a = (int)(e / n), i = (int)(e % n);
-    const double v = (i >= a) ? o.Rr[(long long)a * n + pn_sm[i]] : 0.0;
+    const int a = (int)(e % k), i = (int)(e / k);
+    const double v = (i >= a) ? o.Rr[(long long)pn_sm[i] * n + a] : 0.0;
     if (i < k) o.R11[a + (long long)i * k] = v;
     else o.id.W[a + (long long)(i - k) * k] = v;
   }

@@ -146,7 +146,7 @@ struct PqrDesc {
   double* R1;     // k x k, ld k, upper
   double* R1inv;  // k x k, ld k, upper
   double* Z;      // k x (n - o), ld k: [Q1^T Q1 | Q1^T T]; the second part ends as (I - E) Q1^T T
-  double* Rr;     // n x n row-major: row i of R by column of the face
+  double* Rr;     // n x n, ld n: R by column of the face
   int* perm;      // n: column of the face at each position of T
   const double* Rsel;  // the phase's Cholesky rows (row-major, n - o wide)
   const int* piv;      // the phase's pivots as positions relative to o
@@ -156,7 +156,8 @@ struct PqrDesc {
 void launch_pqr_extract(const PqrDesc* d_desc, int nd, int max_m, cudaStream_t s);
 void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s);
 // R11 and B into Rr, (I - E) Q1^T T over Z; *flag |= 1 where |E| exceeds kPqrMaxE.
-void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_cols, int* flag, cudaStream_t s);
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, int* flag,
+                    cudaStream_t s);
 // After the last phase: jpvt, rdiag, keep, rank; R11 (k x k, ld k) into G and R12
 // into W for the triangular solve. *flag |= 2 where the kept columns are not a
 // prefix of the pivot order.
@@ -360,8 +361,9 @@ void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, in
 
 // Column-pivoted Householder QR + rank + interpolation matrix, one CTA per face.
 // W is written to IdDesc::W, which must hold at least n*n/4 + n doubles.
+// max_mn, max_m: largest m n and m when M need not be left overwritten (else 0).
 void launch_id(const IdDesc* d_desc, int nd, int max_n, double eps, int* d_status,
-               cudaStream_t s, long long max_mn = 0);
+               cudaStream_t s, long long max_mn = 0, int max_m = 0);
 
 void launch_copy(const CopyDesc* d_desc, const int* d_tile_off, int nd, int total_tiles,
                  cudaStream_t s);

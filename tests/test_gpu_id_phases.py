@@ -81,3 +81,40 @@ def test_wide_faces_match_oracle(N, part, field, eps):
                 assert err < min(0.5, max(1e-12, 10 * n * U / eps)), (lev, b, err)
     assert wide > 0
     f.close()
+
+
+@pytest.mark.parametrize("prec,eps", [(hb.PRECISION_FP64, 1e-6), (hb.PRECISION_MIXED, 1e-8)])
+def test_phases_match_column_by_column(prec, eps):
+    """The widest faces (n = 96: up to about 1600 columns, split over a cluster of CTAs)
+    by phases against the column-by-column QR of the same faces, selected by
+    HIF_OPT_ID_GROUP_MIN_N: the same skeletons and, with them, the same operator to the
+    bar of the parity tests (1e-9; in mixed precision the two factors differ by rounding
+    in what the int8 slices truncate: the mixed factor's own 1e-5)."""
+    n = 96
+    N = n - 1
+    a = synth.face_coefficients_lognormal(N, 5)
+    V = np.zeros((n + 1,) * 3)
+    u = synth.dof_vector(N, 1)
+    out, skel = [], []
+    for group in (0, 512):
+        f = hb.HIFFactor(N, 4, eps, hb.PARTITION_CLIPPED)
+        f.set_option(hb.OPT_PRECISION, prec)
+        if group:
+            f.set_option(hb.OPT_ID_GROUP_MIN_N, group)
+        hb.SetupStencilFaces(f, N, 1.0 / n, *a, V)
+        f.Factor()
+        out.append(f.Apply(u.copy(), True))
+        widest = 0
+        sk = []
+        for lev in range(2, f.num_levels() - 1):
+            for b in range(f.num_blocks(lev, 1)):
+                blk = f.block(lev, 1, b)
+                widest = max(widest, blk["global"].size)
+                sk.append(set(blk["skel"].tolist()))
+        assert widest > 832
+        skel.append(sk)
+        f.close()
+    if prec == hb.PRECISION_FP64:
+        assert skel[0] == skel[1]
+    bar = 1e-9 if prec == hb.PRECISION_FP64 else 1e-5
+    assert np.linalg.norm(out[0] - out[1]) < bar * np.linalg.norm(out[1])

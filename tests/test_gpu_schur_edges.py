@@ -1,6 +1,7 @@
-"""Schur of one dense block at the edges of the blocked elimination: redundant counts
-around the 128-wide pivot blocks and the 64 x 64 product tiles, skeleton counts of one
-and around a tile, ragged both ways.
+"""Schur of one dense block at the edges of its elimination: blocks taken whole (up to 160
+unknowns, register tiles of 96 and 160), then the blocked form: redundant counts around
+the 128-wide pivot blocks and the 64 x 64 product tiles, skeleton counts of one and
+around a tile, ragged both ways.
 
 The block is strictly diagonally dominant (each diagonal entry 1.5 times its row's
 absolute sum), so ||A22^{-1}||_inf ||A22||_inf <= (2.5 / 0.5) = 5 per unit of scaling and
@@ -16,7 +17,8 @@ from hifde3d_b200 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("r,s", [(161, 1), (127, 64), (128, 63), (129, 65), (191, 128),
+@pytest.mark.parametrize("r,s", [(1, 1), (15, 1), (16, 16), (17, 78), (95, 1), (96, 0),
+                                 (80, 17), (100, 60), (160, 0), (3, 157), (161, 1), (127, 64), (128, 63), (129, 65), (191, 128),
                                  (192, 129), (255, 17), (256, 0), (257, 191), (384, 64),
                                  (650, 129), (1023, 130)])
 def test_schur_edges(r, s):
