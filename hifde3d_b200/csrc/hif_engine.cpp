@@ -753,10 +753,11 @@ void gemm_batch_int8(const std::vector<GemmDesc>& gin, BufList& tmp, cudaStream_
     eo += x.m + (same ? 0 : x.n);
     if (kt > 0) {
       // A: element (i, kk) = op(A)[i, kk]; B: element (j, kk) = op(B)[kk, j]
-      ops.push_back(OzOperand{x.A, x.lda, x.transA, x.m, x.k, pa, ea});
+      ops.push_back(OzOperand{x.A, x.lda, x.transA, x.m, x.k, pa, ea, x.a_lower ? 1 : 0});
       ooff.push_back(ooff.back() + ta);
       if (!same) {
-        ops.push_back(OzOperand{x.B, x.ldb, x.transB ? 0 : 1, x.n, x.k, pb, eb});
+        ops.push_back(
+            OzOperand{x.B, x.ldb, x.transB ? 0 : 1, x.n, x.k, pb, eb, x.b_lower ? 2 : 0});
         ooff.push_back(ooff.back() + tb);
       }
     }
@@ -810,10 +811,10 @@ struct ElimArith {
 // Y = L^{-1} A21 (X); B's trailing block ends as A11 - Y^T Y, mirrored.
 //   small blocks: k_chol_small, whole in shared memory;
 //   large blocks: right-looking over 128-pivot blocks of A22 only:
-//     L_KK = chol(B[K, K]) and L_KK^{-1} (k_chol_diag),
+//     L_KK = chol(B[K, K]) and L_KK^{-1}, also the diagonal block K of L^{-1}
+//     (k_pivot_block),
 //     panel  B[K1:r, K] = B[K1:r, K] L_KK^{-T},
 //     update B[K1:r, K1:r] -= panel panel^T (lower tiles),
-//     L_KK^{-1} into the diagonal block K of L^{-1};
 //   then the rest of L^{-1} by a halving of the 128-blocks (X21 = -X22 L21 X11,
 //   bottom up, every node of a depth in two batched products),
 //   then Y = L^{-1} A21 and S = A11 - Y^T Y as long-K products (FP64, or from
@@ -881,8 +882,8 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
   }
   for (int k0 = 0; k0 < maxr; k0 += kSweepNB) {
     std::vector<int> active;
-    std::vector<CopyDesc> cq, cdg;
-    std::vector<int> ocq(1, 0), ocd(1, 0);
+    std::vector<CopyDesc> cq;
+    std::vector<int> ocq(1, 0);
     std::vector<GemmDesc> gp, gu;
     for (int b = 0; b < nl; ++b) {
       const SweepDesc& d = large[b];
@@ -923,8 +924,6 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
         u.lower = 2;
         gu.push_back(u);
       }
-      cdg.push_back(CopyDesc{Dv, d.a22inv + k0 + (long long)k0 * r, nbk, r, nbk, nbk});
-      ocd.push_back(ocd.back() + copy_tiles(nbk, nbk));
     }
     BufList step;
     int* dact = step.add(upload(active, stream));
@@ -939,11 +938,6 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
     gemm_batch(gp, step, stream, HIF_KCLASS_SWEEP_PANEL, timed);
     // rank-128 updates: FP64 (from int8 slices they are bound by their C traffic)
     gemm_batch(gu, step, stream, HIF_KCLASS_GEMM, timed);
-    {
-      CopyDesc* dc = step.add(upload(cdg, stream));
-      int* doc = step.add(upload(ocd, stream));
-      timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_copy(dc, doc, (int)cdg.size(), ocd.back(), stream); });
-    }
     HIF_CK(cudaGetLastError());
     step.release(stream);
   }
@@ -1636,10 +1630,16 @@ class Engine {
   // CUDA graphs of the apply sweep (boundary zeroing, output clearing and every
   // launch of the plan), one per (direction, right-hand-side count); valid
   // while the plans and the apply workspace stay as they were captured
+  // A graph is made once a pair has been applied kGraphAfter times: making one takes as
+  // long as about 15 applies by single launches (n = 16: 0.19 ms, against 30 us of
+  // launches), which a factor used for one solve does not give back.
+  static constexpr int kGraphAfter = 16;
   std::map<std::pair<int, int>, cudaGraphExec_t> apply_graphs;
+  std::map<std::pair<int, int>, int> apply_uses;
   void drop_graphs() {
     for (auto& kv : apply_graphs) cudaGraphExecDestroy(kv.second);
     apply_graphs.clear();
+    apply_uses.clear();
   }
 
   void release_plans() {
@@ -3992,11 +3992,11 @@ class Engine {
     timed(HIF_KCLASS_VECTOR, 0, 24.0 * n3 * nrhs,
           [&] { launch_apply_in(src, lds, d_ua, d_ub, NC, nrhs, stream); });
     HIF_CK(cudaGetLastError());
-    if (profile) {
-      run_plan(plan, nrhs);  // per-launch events: no graph
+    const std::pair<int, int> key(inverse ? 1 : 0, nrhs);
+    auto it = apply_graphs.find(key);
+    if (profile || (it == apply_graphs.end() && ++apply_uses[key] <= kGraphAfter)) {
+      run_plan(plan, nrhs);  // (profile: per-launch events, no graph)
     } else {
-      const std::pair<int, int> key(inverse ? 1 : 0, nrhs);
-      auto it = apply_graphs.find(key);
       if (it == apply_graphs.end()) {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t ge = nullptr;

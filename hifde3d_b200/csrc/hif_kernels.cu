@@ -879,10 +879,19 @@ __device__ __forceinline__ void oz_load_tile(const OzOperand& o, int rt, int kt,
   }
 }
 
+// Tiles of a triangular operand that no product reads (all above the diagonal).
+__device__ __forceinline__ bool oz_unread(const OzOperand& o, int rt, int kt) {
+  return (o.tri == 1 && kt * kOzK > rt * 128 + 127) || (o.tri == 2 && kt * kOzK + 63 < rt * 128);
+}
+
 // Row exponents, read in place along the operand's contiguous dimension:
 // trans = 0, two threads per row (lanes over consecutive rows), 32 k each;
 // trans = 1, a warp per row (lanes over consecutive k), 16 rows per warp. The
-// 32 loads of a thread are issued before the first maximum.
+// 32 loads of a thread are issued before the first maximum, which is taken over the
+// high words (an exponent needs no more; rows of subnormals take the exact way).
+__device__ __forceinline__ int oz_exponent(int hi) {  // m < 2^e, m >= 2^(e - 1)
+  return (hi >> 20) - 1022;
+}
 __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ ops,
                                                 const int* __restrict__ tile_off, int nops) {
   const int oi = find_desc(tile_off, nops, blockIdx.x);
@@ -890,6 +899,7 @@ __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ op
   const int local = blockIdx.x - tile_off[oi];
   const int kt_n = (o.kdim + kOzK - 1) / kOzK;
   const int rt = local / kt_n, kt = local % kt_n;
+  if (oz_unread(o, rt, kt)) return;
   const int k0 = kt * kOzK;
   double v[32];
   if (o.trans == 0) {
@@ -902,13 +912,18 @@ __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ op
       const int gk = k0 + 32 * half + e;
       v[e] = gk < o.kdim ? __ldg(src + (long long)gk * o.ld) : 0.0;
     }
-    double m = 0.0;
+    int h = 0;
 #pragma unroll
-    for (int e = 0; e < 32; ++e) m = fmax(m, fabs(v[e]));
-    if (m > 0.0) {
+    for (int e = 0; e < 32; ++e) h = max(h, __double2hiint(v[e]) & 0x7fffffff);
+    if (h >= 0x00100000) {
+      atomicMax(&o.rexp[gi], oz_exponent(h));
+    } else {
+      double m = 0.0;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) m = fmax(m, fabs(v[e]));
       int ex;
-      frexp(m, &ex);  // m < 2^ex
-      atomicMax(&o.rexp[gi], ex);
+      frexp(m, &ex);
+      if (m > 0.0) atomicMax(&o.rexp[gi], ex);
     }
   } else {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -923,27 +938,43 @@ __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ op
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const int gi = rt * 128 + warp + 8 * j;
-      double m = fmax(fabs(v[2 * j]), fabs(v[2 * j + 1]));
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-      if (lane == 0 && gi < o.rows && m > 0.0) {
+      const int h = __reduce_max_sync(
+          0xffffffffu, max(__double2hiint(v[2 * j]) & 0x7fffffff,
+                           __double2hiint(v[2 * j + 1]) & 0x7fffffff));
+      if (gi >= o.rows) continue;
+      if (h >= 0x00100000) {
+        if (lane == 0) atomicMax(&o.rexp[gi], oz_exponent(h));
+      } else {
+        double m = fmax(fabs(v[2 * j]), fabs(v[2 * j + 1]));
         int ex;
         frexp(m, &ex);
-        atomicMax(&o.rexp[gi], ex);
+        if (m > 0.0) atomicMax(&o.rexp[gi], ex);
       }
     }
   }
 }
 
+// The seven-bit digits of 28 bits, the lowest in byte 0; negated bytewise if neg.
+__device__ __forceinline__ unsigned oz_digits(unsigned x, bool neg) {
+  const unsigned d = (x & 0x7fu) | ((x << 1) & 0x7f00u) | ((x << 2) & 0x7f0000u) |
+                     ((x << 3) & 0x7f000000u);
+  return neg ? (0x80808080u - d) ^ 0x80808080u : d;  // digits below 128: no borrow
+}
+
+// |x| 2^{7S - e} truncated to an integer of 7S bits, cut into S digits with x's sign:
+// what truncating v <- 128 v digit by digit gives, from the bits of x. Done in FP64 the
+// S roundings and conversions per entry (a quarter of the FP64 rate or less) set the
+// pace: 2.7 TB/s.
+template <int S>
 __global__ void __launch_bounds__(256) k_oz_slice(const OzOperand* __restrict__ ops,
-                                                  const int* __restrict__ tile_off, int nops,
-                                                  int S) {
+                                                  const int* __restrict__ tile_off, int nops) {
   extern __shared__ double oz_t[];
   const int oi = find_desc(tile_off, nops, blockIdx.x);
   const OzOperand o = ops[oi];
   const int local = blockIdx.x - tile_off[oi];
   const int kt_n = (o.kdim + kOzK - 1) / kOzK;
   const int rt = local / kt_n, kt = local % kt_n;
+  if (oz_unread(o, rt, kt)) return;
   oz_load_tile(o, rt, kt, oz_t);
   __syncthreads();
   const int row = threadIdx.x & 127, half = threadIdx.x >> 7;
@@ -954,33 +985,47 @@ __global__ void __launch_bounds__(256) k_oz_slice(const OzOperand* __restrict__ 
 #pragma unroll 1
   for (int c = 0; c < 2; ++c) {
     const int kc = 2 * half + c;  // 16-byte chunk of the row's 64 bytes
-    unsigned w[kOzMaxS][4];
+    unsigned w[8][4];             // slice S - 1 - s of the chunk's entries, four a word
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-#pragma unroll
-      for (int s = 0; s < kOzMaxS; ++s) w[s][q] = 0u;
+      unsigned lo[4], hi[4];
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const double x = oz_t[row * kOzTs + 16 * kc + 4 * q + b];
-        double v = ldexp(x, -ex);  // |v| < 1
-#pragma unroll
-        for (int s = 0; s < kOzMaxS; ++s) {
-          if (s < S) {
-            v *= 128.0;
-            const double t = trunc(v);
-            v -= t;
-            w[s][q] |= ((unsigned)(int)t & 0xFFu) << (8 * b);
-          }
-        }
+        const int xh = __double2hiint(x), e = (xh >> 20) & 0x7ff;
+        const unsigned mh = (unsigned)(xh & 0xfffff) | (e ? 0x100000u : 0u);
+        const unsigned long long m =
+            e == 0x7ff ? 0ull : ((unsigned long long)mh << 32) | (unsigned)__double2loint(x);
+        const int t = max(e, 1) - 1075 + 7 * S - ex;  // at most 7 S - 53 <= 3
+        const unsigned long long f = t >= 0 ? m << t : (t > -64 ? m >> -t : 0ull);
+        lo[b] = oz_digits((unsigned)f & 0xfffffffu, xh < 0);
+        hi[b] = S > 4 ? oz_digits((unsigned)(f >> 28) & 0xfffffffu, xh < 0) : 0u;
       }
+      // 4 x 4 byte transpose: entries within a word, slices across words
+      auto words = [&](const unsigned (&v)[4], int s0) {
+        const unsigned t0 = __byte_perm(v[0], v[1], 0x5140), t1 = __byte_perm(v[2], v[3], 0x5140);
+        const unsigned t2 = __byte_perm(v[0], v[1], 0x7362), t3 = __byte_perm(v[2], v[3], 0x7362);
+        w[s0][q] = __byte_perm(t0, t1, 0x5410);
+        w[s0 + 1][q] = __byte_perm(t0, t1, 0x7632);
+        w[s0 + 2][q] = __byte_perm(t2, t3, 0x5410);
+        w[s0 + 3][q] = __byte_perm(t2, t3, 0x7632);
+      };
+      words(lo, 0);
+      if (S > 4) words(hi, 4);
     }
     const int off = ((row >> 3) * 4 + kc) * 128 + (row & 7) * 16;
 #pragma unroll
-    for (int s = 0; s < kOzMaxS; ++s)
-      if (s < S)
-        *reinterpret_cast<uint4*>(dst + (size_t)s * kOzPart + off) =
-            make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    for (int s = 0; s < S; ++s)
+      *reinterpret_cast<uint4*>(dst + (size_t)(S - 1 - s) * kOzPart + off) =
+          make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
   }
+}
+
+template <int S>
+static void launch_oz_slice(const OzOperand* d_ops, const int* d_tile_off, int nops,
+                            int total_tiles, cudaStream_t s) {
+  ensure_smem((const void*)k_oz_slice<S>, kOzConvSmem);
+  k_oz_slice<S><<<total_tiles, 256, kOzConvSmem, s>>>(d_ops, d_tile_off, nops);
 }
 
 void launch_oz_convert(const OzOperand* d_ops, const int* d_tile_off, int nops, int total_tiles,
@@ -988,9 +1033,17 @@ void launch_oz_convert(const OzOperand* d_ops, const int* d_tile_off, int nops, 
   if (total_tiles <= 0) return;
   // 0x80808080: below every exponent a double can have
   cudaMemsetAsync(d_rexp, 0x80, (size_t)n_rexp * sizeof(int), s);
-  ensure_smem((const void*)k_oz_slice, kOzConvSmem);
   k_oz_exp<<<total_tiles, 256, 0, s>>>(d_ops, d_tile_off, nops);
-  k_oz_slice<<<total_tiles, 256, kOzConvSmem, s>>>(d_ops, d_tile_off, nops, slices);
+  switch (slices) {
+    case 2: launch_oz_slice<2>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 3: launch_oz_slice<3>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 4: launch_oz_slice<4>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 5: launch_oz_slice<5>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 6: launch_oz_slice<6>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 7: launch_oz_slice<7>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    case 8: launch_oz_slice<8>(d_ops, d_tile_off, nops, total_tiles, s); break;
+    default: break;
+  }
 }
 
 // Shared-memory matrix descriptor: K-major, no swizzle, LBO 128 B, SBO 512 B.
@@ -1762,8 +1815,10 @@ __global__ void __launch_bounds__(kPbThreads, 1)
     const int i = e % nb, j = e / nb;
     const double v = (CHOL && i < j) ? 0.0 : St[i + j * kPbSt];
     out[e] = v;
-    // Gauss-Jordan: the step's panels and updates leave block KK alone
+    // Gauss-Jordan: the step's panels and updates leave block KK alone; Cholesky:
+    // diagonal block K of L^{-1}
     if (!CHOL) d.B[(k0 + i) + (long long)(k0 + j) * d.n] = v;
+    else d.a22inv[(k0 + i) + (long long)(k0 + j) * d.r] = v;
   }
 }
 

@@ -312,6 +312,8 @@ struct OzOperand {
   int rows, kdim;
   signed char* out;
   int* rexp;  // per-row exponent, rows entries
+  int tri;    // zero above the diagonal, whose tiles are not read: 1 element (i, kk) for
+              // kk > i (a lower op(A)), 2 for kk < i (a lower op(B))
 };
 // d_tile_off: prefix over operands of ceil(rows / 128) * ceil(kdim / 64).
 // Every rexp lies in [d_rexp, d_rexp + n_rexp): it is cleared, then the
