@@ -813,7 +813,7 @@ struct ElimArith {
 //   large blocks: right-looking over 128-pivot blocks of A22 only:
 //     L_KK = chol(B[K, K]) and L_KK^{-1}, also the diagonal block K of L^{-1}
 //     (k_pivot_block),
-//     panel  B[K1:r, K] = B[K1:r, K] L_KK^{-T},
+//     panel  L[K1:r, K] = B[K1:r, K] L_KK^{-T},
 //     update B[K1:r, K1:r] -= panel panel^T (lower tiles),
 //   then the rest of L^{-1} by a halving of the 128-blocks (X21 = -X22 L21 X11,
 //   bottom up, every node of a depth in two batched products),
@@ -857,14 +857,7 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
   SweepDesc* dd = tmp.add(upload(large, stream));
   double* dinv = big((size_t)nl * kSweepNB * kSweepNB);
   int maxr = 0;
-  std::vector<long long> oq(nl);
-  long long qsz = 0;
-  for (int b = 0; b < nl; ++b) {
-    maxr = std::max(maxr, large[b].r);
-    oq[b] = qsz;
-    qsz += (long long)large[b].r * kSweepNB;
-  }
-  double* Qb = big(qsz);  // per block: old panel (r x 128, ld r)
+  for (const SweepDesc& d : large) maxr = std::max(maxr, d.r);
   // L and L^{-1} read as zero above their diagonals
   {
     std::vector<GemmDesc> z;
@@ -882,26 +875,20 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
   }
   for (int k0 = 0; k0 < maxr; k0 += kSweepNB) {
     std::vector<int> active;
-    std::vector<CopyDesc> cq;
-    std::vector<int> ocq(1, 0);
     std::vector<GemmDesc> gp, gu;
     for (int b = 0; b < nl; ++b) {
       const SweepDesc& d = large[b];
       if (d.r <= k0) continue;
       active.push_back(b);
       const int r = d.r, k1 = std::min(r, k0 + kSweepNB), nbk = k1 - k0;
-      const double* Dv = dinv + (long long)b * kSweepNB * kSweepNB;  // nbk x nbk, ld nbk
-      double* Q = Qb + oq[b];
-      double* P = d.B + k1 + (long long)k0 * d.n;  // panel rows k1..r of column block K
       if (r > k1) {
-        cq.push_back(CopyDesc{P, Q, d.n, r, r - k1, nbk});
-        ocq.push_back(ocq.back() + copy_tiles(r - k1, nbk));
+        double* P = d.L + k1 + (long long)k0 * r;  // panel rows k1..r of L's column block K
         GemmDesc g{};
         g.C = P;
-        g.ldc = d.n;
-        g.A = Q;
-        g.lda = r;
-        g.B = Dv;
+        g.ldc = r;
+        g.A = d.B + k1 + (long long)k0 * d.n;
+        g.lda = d.n;
+        g.B = dinv + (long long)b * kSweepNB * kSweepNB;  // L_KK^{-1}, ld nbk
         g.ldb = nbk;
         g.transB = 1;
         g.m = r - k1;
@@ -913,15 +900,15 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
         u.C = d.B + k1 + (long long)k1 * d.n;
         u.ldc = d.n;
         u.A = P;
-        u.lda = d.n;
+        u.lda = r;
         u.B = P;
-        u.ldb = d.n;
+        u.ldb = r;
         u.transB = 1;
         u.m = u.n = r - k1;
         u.k = nbk;
         u.alpha = -1.0;
         u.beta = 1.0;
-        u.lower = 2;
+        u.lower = 2;  // the pivot block and the panels read the lower triangle only
         gu.push_back(u);
       }
     }
@@ -930,33 +917,11 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
     timed(HIF_KCLASS_SWEEP_PANEL, 0, 0, [&] {
       launch_chol_diag(dd, dact, (int)active.size(), k0, dinv, d_status, stream);
     });
-    if (!cq.empty()) {
-      CopyDesc* dq = step.add(upload(cq, stream));
-      int* doq = step.add(upload(ocq, stream));
-      timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_copy(dq, doq, (int)cq.size(), ocq.back(), stream); });
-    }
     gemm_batch(gp, step, stream, HIF_KCLASS_SWEEP_PANEL, timed);
     // rank-128 updates: FP64 (from int8 slices they are bound by their C traffic)
     gemm_batch(gu, step, stream, HIF_KCLASS_GEMM, timed);
     HIF_CK(cudaGetLastError());
     step.release(stream);
-  }
-  // L: the block-lower column strips of B[0:r, 0:r] (its diagonal tiles already
-  // hold zeros above the diagonal; the tiles above them still hold A22)
-  {
-    std::vector<CopyDesc> cl;
-    std::vector<int> ocl(1, 0);
-    for (const SweepDesc& d : large)
-      for (int j0 = 0; j0 < d.r; j0 += kSweepNB) {
-        const int nbj = std::min(kSweepNB, d.r - j0);
-        cl.push_back(CopyDesc{d.B + j0 + (long long)j0 * d.n, d.L + j0 + (long long)j0 * d.r,
-                              d.n, d.r, d.r - j0, nbj});
-        ocl.push_back(ocl.back() + copy_tiles(d.r - j0, nbj));
-      }
-    CopyDesc* dc = tmp.add(upload(cl, stream));
-    int* doc = tmp.add(upload(ocl, stream));
-    timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_copy(dc, doc, (int)cl.size(), ocl.back(), stream); });
-    HIF_CK(cudaGetLastError());
   }
   // L^{-1} off the diagonal blocks (which hold L_KK^{-1}), bottom up over a
   // halving of each block's 128-blocks: for a node [b0, b1) split at mid,
@@ -995,8 +960,8 @@ void chol_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_t
         GemmDesc t{};  // T = L21 X11 (X11 lower triangular)
         t.C = T;
         t.ldc = q.r2;
-        t.A = d.B + q.o2 + (long long)q.o1 * d.n;
-        t.lda = d.n;
+        t.A = d.L + q.o2 + (long long)q.o1 * d.r;
+        t.lda = d.r;
         t.B = d.a22inv + q.o1 + (long long)q.o1 * d.r;
         t.ldb = d.r;
         t.b_lower = 1;
@@ -1133,10 +1098,12 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
     // Symmetric A22 (the face operator): only the block-lower triangle is
     // kept. After the pivot blocks before K, entry (i, j) equals +(j, i) when
     // i and j are both pivoted or both not, -(j, i) otherwise. Step K with
-    // Q = the old column block K (rows above K from row block K, negated),
-    // W = -Q D^{-1}: new column block K = W (rows below K), new row block K
+    // Q = the old column block K (rows above K: the old row block K, transposed and
+    // negated), W = -Q D^{-1}: new column block K = W (rows below K), new row block K
     // = W^T (columns left of K), and lower tile (I, J) += tau_J W_I Q_J^T with
-    // tau_J = -1 left of K, +1 right of K. At the end every pivot is taken,
+    // tau_J = -1 left of K, +1 right of K. Both new panels are written in place from
+    // copies of the old ones and read from there by the update, so a step is the pivot
+    // block, one copy and two batches of products. At the end every pivot is taken,
     // the inverse is symmetric and the upper tiles are mirrored from the lower.
     // 2r^3 -> r^3 flops.
     std::vector<long long> oq(nl);
@@ -1145,14 +1112,12 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
       oq[b] = qsz;
       qsz += (long long)large[b].r * kSweepNB;
     }
-    double* Qb = big(qsz);
-    double* Wb = big(qsz);
+    double* Qb = big(qsz);  // old column block K, rows below it (ld r)
+    double* Rb = big(qsz);  // old row block K, columns left of it (ld 128)
     for (int k0 = 0; k0 < maxr; k0 += kSweepNB) {
       std::vector<int> active;
-      std::vector<CopyDesc> cq, cw;
-      std::vector<int> ocq(1, 0), ocw(1, 0);
-      std::vector<TCopyDesc> tq, tw;
-      std::vector<int> otq(1, 0), otw(1, 0);
+      std::vector<CopyDesc> cq;
+      std::vector<int> ocq(1, 0);
       std::vector<GemmDesc> gw, gu;
       for (int b = 0; b < nl; ++b) {
         const SweepDesc& d = large[b];
@@ -1161,55 +1126,67 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
         const int k1 = std::min(d.r, k0 + kSweepNB), nbk = k1 - k0, r = d.r;
         const double* Dv = dinv + (long long)b * kSweepNB * kSweepNB;
         double* Q = Qb + oq[b];
-        double* W = Wb + oq[b];
-        if (r > k1) {
-          cq.push_back(CopyDesc{d.B + k1 + (long long)k0 * d.n, Q + k1, d.n, r, r - k1, nbk});
+        double* R = Rb + oq[b];
+        double* colK = d.B + (long long)k0 * d.n;
+        double* rowK = d.B + k0;
+        GemmDesc g{};
+        g.k = nbk;
+        if (r > k1) {  // W below = -Q D^{-1}
+          cq.push_back(CopyDesc{colK + k1, Q + k1, d.n, r, r - k1, nbk});
           ocq.push_back(ocq.back() + copy_tiles(r - k1, nbk));
-          cw.push_back(CopyDesc{W + k1, d.B + k1 + (long long)k0 * d.n, r, d.n, r - k1, nbk});
-          ocw.push_back(ocw.back() + copy_tiles(r - k1, nbk));
-        }
-        if (k0 > 0) {
-          tq.push_back(TCopyDesc{d.B + k0, Q, d.n, r, k0, nbk, -1.0});
-          otq.push_back(otq.back() + copy_tiles(k0, nbk));
-          tw.push_back(TCopyDesc{W, d.B + k0, r, d.n, nbk, k0, 1.0});
-          otw.push_back(otw.back() + copy_tiles(nbk, k0));
-        }
-        auto wg = [&](int r0, int r1) {
-          if (r1 <= r0) return;
-          GemmDesc g{};
-          g.C = W + r0;
-          g.ldc = r;
-          g.A = Q + r0;
+          g.C = colK + k1;
+          g.ldc = d.n;
+          g.A = Q + k1;
           g.lda = r;
           g.B = Dv;
           g.ldb = nbk;
-          g.m = r1 - r0;
+          g.m = r - k1;
           g.n = nbk;
-          g.k = nbk;
           g.alpha = -1.0;
-          g.beta = 0.0;
           gw.push_back(g);
-        };
-        wg(0, k0);
-        wg(k1, r);
+        }
+        if (k0 > 0) {  // W^T left = D^{-T} R
+          cq.push_back(CopyDesc{rowK, R, d.n, kSweepNB, nbk, k0});
+          ocq.push_back(ocq.back() + copy_tiles(nbk, k0));
+          g.C = rowK;
+          g.ldc = d.n;
+          g.A = Dv;
+          g.lda = nbk;
+          g.transA = 1;
+          g.B = R;
+          g.ldb = kSweepNB;
+          g.m = nbk;
+          g.n = k0;
+          g.alpha = 1.0;
+          gw.push_back(g);
+        }
         for (int j0 = 0; j0 < r; j0 += kSweepNB) {
           if (j0 == k0) continue;
           const int j1 = std::min(r, j0 + kSweepNB);
-          const double tau = j0 < k0 ? -1.0 : 1.0;
           auto ug = [&](int r0, int r1) {
             if (r1 <= r0) return;
             GemmDesc g{};
             g.C = d.B + r0 + (long long)j0 * d.n;
             g.ldc = d.n;
-            g.A = W + r0;
-            g.lda = r;
-            g.B = Q + j0;
-            g.ldb = r;
-            g.transB = 1;
+            if (r0 < k0) {  // W_I from the new row block
+              g.A = rowK + (long long)r0 * d.n;
+              g.transA = 1;
+            } else {
+              g.A = colK + r0;
+            }
+            g.lda = d.n;
+            if (j0 < k0) {  // tau Q_J^T = -(-R_J)
+              g.B = R + (long long)j0 * kSweepNB;
+              g.ldb = kSweepNB;
+            } else {
+              g.B = Q + j0;
+              g.ldb = r;
+              g.transB = 1;
+            }
             g.m = r1 - r0;
             g.n = j1 - j0;
             g.k = nbk;
-            g.alpha = tau;
+            g.alpha = 1.0;
             g.beta = 1.0;
             gu.push_back(g);
           };
@@ -1231,23 +1208,8 @@ void sweep_blocks(const std::vector<SweepDesc>& descs, BufList& tmp, cudaStream_
         int* doq = step.add(upload(ocq, stream));
         timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_copy(dq, doq, (int)cq.size(), ocq.back(), stream); });
       }
-      if (!tq.empty()) {
-        TCopyDesc* dq = step.add(upload(tq, stream));
-        int* doq = step.add(upload(otq, stream));
-        timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_tcopy(dq, doq, (int)tq.size(), otq.back(), stream); });
-      }
       gemm_batch(gw, step, stream, HIF_KCLASS_SWEEP_PANEL, timed);
       gemm_batch(gu, step, stream, HIF_KCLASS_GEMM, timed);
-      if (!cw.empty()) {
-        CopyDesc* dw = step.add(upload(cw, stream));
-        int* dow = step.add(upload(ocw, stream));
-        timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_copy(dw, dow, (int)cw.size(), ocw.back(), stream); });
-      }
-      if (!tw.empty()) {
-        TCopyDesc* dw = step.add(upload(tw, stream));
-        int* dow = step.add(upload(otw, stream));
-        timed(HIF_KCLASS_COPY, 0, 0, [&] { launch_tcopy(dw, dow, (int)tw.size(), otw.back(), stream); });
-      }
       HIF_CK(cudaGetLastError());
       step.release(stream);
     }

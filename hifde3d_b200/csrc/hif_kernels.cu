@@ -1550,7 +1550,7 @@ void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status
 //     accumulators zeroed, R[:, K] = D^{-1} and C[K, :] = -I it is A - C R throughout;
 //   Cholesky: l = chol(D), x = l^{-1}; L_iK = A_iK x^T below, the finished part of
 //     L^{-1} left of K gets X_K = x X_K; R = [X_K | x | L_jK^T], rows K := R and rows
-//     below K := A - L_iK R. The lower triangle only; L goes straight to B.
+//     below K := A - L_iK R. The lower triangle only; L goes straight to its place.
 // The serial part, the 16 x 16 inverse (or factor and inverse), is a 17th warp's: the
 // owner of the next diagonal block updates that block first and hands it over, so the
 // inverse runs beside the rest of the update (4096 DMMA cycles a step; 128^3
@@ -1792,7 +1792,7 @@ __global__ void __launch_bounds__(kPbThreads, 1)
         for (int e = tid; e < kPbW * kSweepNB; e += 512) {
           const int i = e & (kSweepNB - 1), k = e / kSweepNB, r = i - K;
           if (i < nb && K + k < nb)
-            d.B[(k0 + i) + (long long)(k0 + K + k) * d.n] =
+            d.L[(k0 + i) + (long long)(k0 + K + k) * d.r] =
                 r < 0 ? 0.0 : (r < kPbW ? L[k * kPbD + r] : Rn[k * kPbLd + i]);
         }
       }

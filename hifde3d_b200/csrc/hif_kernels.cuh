@@ -356,8 +356,8 @@ void launch_sweep_diag(const SweepDesc* d_desc, const int* d_active, int nact, i
 void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
                        cudaStream_t s);
 // Pivot block K = [k0, k0 + 128) of the blocked factorization: L_KK = chol(B[K, K])
-// written over B[K, K] (zeros above its diagonal) and L_KK^{-1} (lower, zeros
-// above) into dinv (128 x 128 per active block, ld = its width).
+// into L's diagonal block (zeros above its diagonal) and L_KK^{-1} (lower, zeros
+// above) into L^{-1}'s and into dinv (128 x 128 per active block, ld = its width).
 void launch_chol_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
                       double* d_dinv, int* d_status, cudaStream_t s);
 
