@@ -1545,24 +1545,30 @@ void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status
 // remain, so it is built for latency. 16 worker warps hold the block as DMMA
 // accumulators (32 x 32 a warp); step K reads the panels of block K from the owners
 // through shared memory and updates everything by one rank-16 product:
-//   Gauss-Jordan: with D = block KK, R = D^{-1} (row panel), rows K := R, columns
-//     K := -C D^{-1}, the rest A - C R: with the K rows and columns of the
-//     accumulators zeroed, R[:, K] = D^{-1} and C[K, :] = -I it is A - C R throughout;
-//   Cholesky: l = chol(D), x = l^{-1}; L_iK = A_iK x^T below, the finished part of
-//     L^{-1} left of K gets X_K = x X_K; R = [X_K | x | L_jK^T], rows K := R and rows
-//     below K := A - L_iK R. The lower triangle only; L goes straight to its place.
-// The serial part, the 16 x 16 inverse (or factor and inverse), is a 17th warp's: the
-// owner of the next diagonal block updates that block first and hands it over, so the
-// inverse runs beside the rest of the update (4096 DMMA cycles a step; 128^3
+//   Gauss-Jordan: with D = LU = block KK, G = L^{-1} (row panel) and H = (column panel)
+//     U^{-1}: rows K := U^{-1} G, columns K := -H L^{-1}, the rest A - H G: with the K
+//     rows and columns of the accumulators zeroed, G[:, K] = L^{-1} and H[K, :] = -U^{-1}
+//     it is A - H G throughout;
+//   Cholesky: l = chol(D); L_iK = A_iK l^{-T} below, the finished part of
+//     L^{-1} left of K gets X_K = l^{-1} X_K; R = [X_K | l^{-1} | L_jK^T], rows K := R and
+//     rows below K := A - L_iK R. The lower triangle only; L goes straight to its place.
+// The panels are substituted, a column or row a thread, not multiplied by inverses of D
+// or of its factors: that keeps the errors of single pivots (a few u times the scaled
+// condition number), where products with D^{-1} were 20 to 100 times that for the wide
+// faces of a field of contrast 10^6, and costs fewer multiply-adds.
+// The serial part is four more warps', which hold no accumulators: the factors of D one
+// warp's, the substitutions all four's. The owner of the next diagonal block updates
+// that block first and hands it over, so its factors
+// run beside the rest of the update (4096 DMMA cycles a step; 128^3
 // multiply-adds take 32.8 k). Before, the inverse was one pivot and one barrier at a
 // time over registers: 200 us a block, the factor 32-wide by one warp, 150 us.
 constexpr int kPbW = 16;                  // block step
 constexpr int kPbLd = kSweepNB + 4;       // panel rows: 4 mod 16 doubles, conflict-free fragments
 constexpr int kPbSt = kSweepNB + 1;       // staging
 constexpr int kPbD = kPbW + 1;
-constexpr int kPbThreads = 17 * 32;
+constexpr int kPbThreads = 20 * 32;
 constexpr int kPbSmem =
-    (kSweepNB * kPbSt + 4 * kPbW * kPbLd + 4 * kPbW * kPbD) * (int)sizeof(double);
+    (kSweepNB * kPbSt + 4 * kPbW * kPbLd + 2 * kPbW * kPbW + 3 * kPbW * kPbD) * (int)sizeof(double);
 
 __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -1571,11 +1577,13 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// 16 x 16 inverse (CHOL: the inverse of the Cholesky factor, the factor itself to
-// Ls[k][i]) by one warp: lane = (row i, half h), columns 8h .. 8h + 7 in registers.
+// The factors of a 16 x 16 pivot D by one warp: lane = (row i, half h), columns
+// 8h .. 8h + 7 in registers. D = LU: F0[k][i] = L_ik below a diagonal of ones,
+// F1[k][i] = U_ki right of a diagonal of reciprocal pivots. CHOL, D = l l^T: F0[k][i] =
+// l_ik below a diagonal of reciprocals, l itself to Ls[k][i].
 template <bool CHOL>
-__device__ __forceinline__ void pivot16(const double* Dn, double* Di, double* Ls, int live,
-                                        int& bad) {
+__device__ __forceinline__ void pivot16(const double* Dn, double* F0, double* F1, double* Ls,
+                                        int live, int& bad) {
   const int lane = threadIdx.x & 31, i = lane & 15, h = lane >> 4;
   double a[8];
 #pragma unroll
@@ -1588,31 +1596,52 @@ __device__ __forceinline__ void pivot16(const double* Dn, double* Di, double* Ls
     double rj[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) rj[c] = __shfl_sync(0xffffffffu, a[c], k + 16 * h);
+    double li;
     if (CHOL) {
       if (k < live && (!(p > 1e-300) || !isfinite(p))) bad = 1;
-      const double q = fabs(p) > 1e-300 ? fabs(p) : 1.0;
-      const double rk = rsqrt(q), li = cik * rk;
-      if (h == 0) Ls[k * kPbD + i] = i > k ? li : (i == k ? q * rk : 0.0);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const double r = (8 * h + c == k) ? rk : rj[c] * rk;
-        const double old = (8 * h + c == k) ? 0.0 : a[c];
-        if (i == k) a[c] = r;
-        else if (i > k) a[c] = fma(-li, r, old);
+      const double q = fabs(p) > 1e-300 ? fabs(p) : 1.0, rk = rsqrt(q);
+      li = cik * rk;
+      if (h == 0) {
+        Ls[k * kPbD + i] = i > k ? li : (i == k ? q * rk : 0.0);
+        F0[k * kPbW + i] = i == k ? rk : li;
       }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) rj[c] *= rk;
     } else {
       if (k < live && (!(fabs(p) > 1e-300) || !isfinite(p))) bad = 1;
       const double ip = 1.0 / p;
+      li = cik * ip;
+      if (h == 0) F0[k * kPbW + i] = i == k ? 1.0 : li;
+      if (i == k) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const double r = (8 * h + c == k) ? ip : rj[c] * ip;
-        const double old = (8 * h + c == k) ? 0.0 : a[c];
-        a[c] = (i == k) ? r : fma(-cik, r, old);
+        for (int c = 0; c < 8; ++c) F1[k * kPbW + 8 * h + c] = 8 * h + c == k ? ip : a[c];
       }
     }
-  }
+    if (i > k) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) Di[i * kPbD + 8 * h + c] = (CHOL && 8 * h + c > i) ? 0.0 : a[c];
+      for (int c = 0; c < 8; ++c)
+        if (8 * h + c > k) a[c] = fma(-li, rj[c], a[c]);
+    }
+  }
+}
+
+// y := the solution of the triangle of F (its column k below the diagonal, its diagonal
+// inverted), y's entries in registers
+template <bool UNIT>
+__device__ __forceinline__ void substitute16(double (&y)[kPbW], const double* F) {
+#pragma unroll
+  for (int k = 0; k < kPbW; ++k) {
+    double f[kPbW];
+#pragma unroll
+    for (int i = k & ~1; i < kPbW; i += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(F + k * kPbW + i);
+      f[i] = v.x;
+      f[i + 1] = v.y;
+    }
+    if (!UNIT) y[k] *= f[k];
+#pragma unroll
+    for (int i = k + 1; i < kPbW; ++i) y[i] = fma(-f[i], y[k], y[i]);
+  }
 }
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
@@ -1635,12 +1664,13 @@ __global__ void __launch_bounds__(kPbThreads, 1)
   extern __shared__ double pb_sm[];
   double* St = pb_sm;                      // [col][row], staging
   double* Rowp = St + kSweepNB * kPbSt;    // [k][col]: rows K
-  double* Colp = Rowp + kPbW * kPbLd;      // [k][row]: columns K (Gauss-Jordan: -C, I at K, even K)
-  double* Rn = Colp + kPbW * kPbLd;        // [k][col]: R
-  double* An = Rn + kPbW * kPbLd;          // [k][row]: Cholesky's -L_iK, I at K; else Colp of odd K
-  double* Dn = An + kPbW * kPbLd;          // the next diagonal block
-  double* Di = Dn + kPbW * kPbD;           // its inverse
-  double* Ls = Di + kPbW * kPbD;           // 2 x its Cholesky factor, [k][row]
+  double* Colp = Rowp + kPbW * kPbLd;      // [k][row]: columns K
+  double* Rn = Colp + kPbW * kPbLd;        // [k][col]: G (Cholesky: R)
+  double* An = Rn + kPbW * kPbLd;          // [k][row]: -H (Cholesky: -L_iK, I at K)
+  double* F0 = An + kPbW * kPbLd;          // the factors of the diagonal block
+  double* F1 = F0 + kPbW * kPbW;
+  double* Dn = F1 + kPbW * kPbW;           // the next diagonal block
+  double* Ls = Dn + kPbW * kPbD;           // 2 x the Cholesky factor, [k][row]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tq = lane & 3;
   {
@@ -1655,18 +1685,40 @@ __global__ void __launch_bounds__(kPbThreads, 1)
     }
   }
   __syncthreads();
-  if (warp == 16) {
-    // the 16 x 16 pivots
+  if (warp >= 16) {
     int bad = 0;
-    for (int e = lane; e < kPbW * kPbW; e += 32)
-      Dn[(e & 15) * kPbD + (e >> 4)] = St[(e & 15) + (e >> 4) * kPbSt];
-    __syncwarp();
-    pivot16<CHOL>(Dn, Di, Ls, nb, bad);
+    if (warp == 16) {
+      for (int e = lane; e < kPbW * kPbW; e += 32)
+        Dn[(e & 15) * kPbD + (e >> 4)] = St[(e & 15) + (e >> 4) * kPbSt];
+      __syncwarp();
+      pivot16<CHOL>(Dn, F0, F1, Ls, nb, bad);
+    }
+    const int j = tid - 512;
     for (int kb = 0; kb < NBLK; ++kb) {
+      const int K = kb * kPbW;
+      const bool own = (unsigned)(j - K) < kPbW;
       bar_sync(1, kPbThreads);
-      if (kb + 1 == NBLK) break;
-      bar_sync(3, 64);
-      pivot16<CHOL>(Dn, Di, Ls + ((kb + 1) & 1) * kPbW * kPbD, nb - (kb + 1) * kPbW, bad);
+      // G and H (Cholesky: R), a column and a row a thread
+      const double* src = (CHOL && j > K) ? Colp : Rowp;
+      double y[kPbW], z[kPbW];
+#pragma unroll
+      for (int k = 0; k < kPbW; ++k) {
+        y[k] = own ? (j - K == k ? 1.0 : 0.0) : src[k * kPbLd + j];
+        if (!CHOL) z[k] = own ? (j - K == k ? 1.0 : 0.0) : -Colp[k * kPbLd + j];
+      }
+      substitute16<!CHOL>(y, F0);
+      if (!CHOL) substitute16<false>(z, F1);
+#pragma unroll
+      for (int k = 0; k < kPbW; ++k) {
+        Rn[k * kPbLd + j] = y[k];
+        An[k * kPbLd + j] =
+            !CHOL ? z[k] : (own ? (j - K == k ? 1.0 : 0.0) : (j > K ? -y[k] : 0.0));
+      }
+      bar_arrive(2, kPbThreads);
+      if (warp == 16 && kb + 1 < NBLK) {
+        bar_sync(3, 64);
+        pivot16<CHOL>(Dn, F0, F1, Ls + ((kb + 1) & 1) * kPbW * kPbD, nb - (kb + 1) * kPbW, bad);
+      }
     }
     if (bad) atomicOr(status, kStatusTinyPivot);
   } else {
@@ -1682,9 +1734,6 @@ __global__ void __launch_bounds__(kPbThreads, 1)
     auto step = [&](auto par_, int kb) {
       constexpr int P = decltype(par_)::value;  // kb & 1: the K rows are MMA tiles 2P, 2P + 1
       const int K = kb * kPbW;
-      // Gauss-Jordan reads the column panel through the update, so it alternates with
-      // the buffer that holds -L_iK in the Cholesky form
-      double* Cp = (!CHOL && P) ? An : Colp;
       if (wr == kb >> 1 && (!CHOL || wc <= wr)) {
 #pragma unroll
         for (int a = 0; a < 2; ++a)
@@ -1702,9 +1751,7 @@ __global__ void __launch_bounds__(kPbThreads, 1)
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
               const int i = wm + a * 8 + gq, k = b * 8 + tq * 2 + c;
-              const double v = acc[a][2 * P + b][c];
-              Cp[k * kPbLd + i] =
-                  CHOL ? v : ((unsigned)(i - K) < kPbW ? (i - K == k ? 1.0 : 0.0) : -v);
+              Colp[k * kPbLd + i] = acc[a][2 * P + b][c];
             }
       }
       // rows and columns K are replaced (Cholesky keeps columns K of the rows above)
@@ -1722,38 +1769,8 @@ __global__ void __launch_bounds__(kPbThreads, 1)
             if (!CHOL || wm + a * 8 >= K) acc[a][2 * P + b][0] = acc[a][2 * P + b][1] = 0.0;
       }
       bar_sync(1, kPbThreads);
-      // R, 8 columns a warp
-      {
-        const int j0 = warp * 8;
-        const bool own = (unsigned)(j0 - K) < kPbW;
-        const double* src = (CHOL && j0 > K) ? Cp : Rowp;
-        double r[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-        if (own) {
-#pragma unroll
-          for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-              r[a][c] = Di[(a * 8 + gq) * kPbD + (j0 - K) + tq * 2 + c];
-        } else {
-#pragma unroll
-          for (int k4 = 0; k4 < kPbW; k4 += 4) {
-            const double b = src[(k4 + tq) * kPbLd + j0 + gq];
-#pragma unroll
-            for (int a = 0; a < 2; ++a) dmma(r[a], Di[(a * 8 + gq) * kPbD + k4 + tq], b);
-          }
-        }
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int k = a * 8 + gq, j = j0 + tq * 2 + c;
-            Rn[k * kPbLd + j] = r[a][c];
-            if (CHOL) An[k * kPbLd + j] = own ? (j - K == k ? 1.0 : 0.0) : (j > K ? -r[a][c] : 0.0);
-          }
-      }
-      bar_sync(2, 512);
-      // A += An R, the quadrant that holds the next diagonal block first
-      const double* Aop = CHOL ? An : Cp;
+      bar_sync(2, kPbThreads);
+      // A += An Rn, the quadrant that holds the next diagonal block first
       const bool run = !CHOL || (wc <= wr && wm + 32 > K);
       if (run) {
 #pragma unroll
@@ -1764,7 +1781,7 @@ __global__ void __launch_bounds__(kPbThreads, 1)
             double af[2], bf[2];
 #pragma unroll
             for (int a = 0; a < 2; ++a)
-              af[a] = Aop[(k4 + tq) * kPbLd + wm + (2 * qa + a) * 8 + gq];
+              af[a] = An[(k4 + tq) * kPbLd + wm + (2 * qa + a) * 8 + gq];
 #pragma unroll
             for (int b = 0; b < 2; ++b)
               bf[b] = Rn[(k4 + tq) * kPbLd + wn + (2 * qb + b) * 8 + gq];
