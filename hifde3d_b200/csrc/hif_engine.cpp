@@ -90,7 +90,10 @@ void dfree(void* p, cudaStream_t s) {
 // it, which would stall the host behind the GPU at every descriptor upload;
 // from pinned memory the copy is queued and the host goes on. The staging is
 // bump-allocated in chunks kept for the owner's life and reused from the start
-// once the owner has synchronised (its copies are then complete).
+// once the owner has synchronised (its copies are then complete). Pinning takes
+// about 0.8 ms per MB, so the chunks start small and double: a first chunk of 32 MB
+// was most of the first factorization of a new handle up to n = 32 (n = 16: 28 ms
+// with it, 6.5 ms without; n = 32 node operator: 40 and 30 ms).
 struct PinnedStage {
   struct Chunk {
     char* p;
@@ -98,7 +101,7 @@ struct PinnedStage {
   };
   std::vector<Chunk> chunks;
   size_t cur = 0;
-  static constexpr size_t kMinChunk = size_t(32) << 20;
+  static constexpr size_t kMinChunk = size_t(1) << 20, kMaxChunk = size_t(32) << 20;
   void* get(size_t bytes) {
     bytes = (bytes + 255) & ~size_t(255);
     for (; cur < chunks.size(); ++cur) {
@@ -109,7 +112,8 @@ struct PinnedStage {
         return r;
       }
     }
-    const size_t sz = std::max(bytes, kMinChunk);
+    const size_t next = chunks.empty() ? kMinChunk : 2 * chunks.back().size;
+    const size_t sz = std::max(bytes, std::min(next, kMaxChunk));
     void* p = nullptr;
     HIF_CK(cudaHostAlloc(&p, sz, cudaHostAllocDefault));
     chunks.push_back(Chunk{static_cast<char*>(p), sz, bytes});
@@ -809,7 +813,7 @@ struct ElimArith {
 // Cholesky elimination of a batch of symmetric positive definite interiors
 // (lower triangles only): writes L (descs[b].L), L^{-1} (a22inv) and
 // Y = L^{-1} A21 (X); B's trailing block ends as A11 - Y^T Y, mirrored.
-//   small blocks: k_chol_small, whole in shared memory;
+//   small blocks: k_elim_small, whole in registers;
 //   large blocks: right-looking over 128-pivot blocks of A22 only:
 //     L_KK = chol(B[K, K]) and L_KK^{-1}, also the diagonal block K of L^{-1}
 //     (k_pivot_block),
@@ -2428,8 +2432,8 @@ class Engine {
     }
     if (!chol_id.empty()) id_cholesky(chol_id, tmp);
     // by phases, unless the order is prescribed or the grouped QR was asked for:
-    // n = 128 FP64, the three wide levels 758 ms column by column, 325 ms by
-    // phases; n = 32, 12 faces of 225 columns, 11.0 ms against 4.6 ms
+    // n = 128 FP64, the three wide levels 758 ms column by column, 218 ms by
+    // phases; n = 32, 12 faces of 225 columns, 11.0 ms against 2.4 ms
     if (!wide_id.empty() && (d_ord || group_asked)) {
       id_householder(wide_id, tmp);
     } else if (!wide_id.empty() && !id_phases(wide_id, tmp)) {
