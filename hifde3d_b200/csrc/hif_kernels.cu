@@ -964,7 +964,8 @@ __device__ __forceinline__ unsigned oz_digits(unsigned x, bool neg) {
 // |x| 2^{7S - e} truncated to an integer of 7S bits, cut into S digits with x's sign:
 // what truncating v <- 128 v digit by digit gives, from the bits of x. Done in FP64 the
 // S roundings and conversions per entry (a quarter of the FP64 rate or less) set the
-// pace: 2.7 TB/s.
+// pace: 2.7 TB/s. n = 128 mixed: 25.1 ms of slicing then, 17.7 ms now, the triangular
+// operands' unread tiles left out.
 template <int S>
 __global__ void __launch_bounds__(256) k_oz_slice(const OzOperand* __restrict__ ops,
                                                   const int* __restrict__ tile_off, int nops) {
@@ -1410,7 +1411,7 @@ void launch_gemm_oz(const OzGemm* d_desc, const int* d_tile_off, int nd, int tot
 //   with -l_i t in column k.
 // Bound by the barrier and the publish of a pivot. In shared memory, with four barriers
 // and an integer division per entry, level 0's 27-of-81 blocks of n = 128 took 7.8 ms
-// (Cholesky 6.5 ms); reading and writing them takes 0.5 ms.
+// (Cholesky 6.5 ms), 2.8 ms (3.3 ms) here; reading and writing them takes 0.5 ms.
 template <int TS, bool CHOL>
 __global__ void __launch_bounds__(256, TS == 6 ? 2 : 1) k_elim_small(const SweepDesc* __restrict__ descs,
                                                     int* __restrict__ status) {
@@ -3056,7 +3057,8 @@ void launch_trsm_upper(const double* R, long long ldr, int k, double* B, long lo
 // HBM, the products with the panel's earlier rows. A step is one block barrier (and one
 // cluster barrier): every warp reduces the warps' candidates itself, and the earlier
 // rows' pivot entries are broadcast reads. With R's rows re-read from L2 and a serial
-// search a step took about 15 us (144 faces of 767 columns, 0.5 ms a panel).
+// search a step took about 15 us (144 faces of 767 columns, 0.5 ms a panel); the
+// panels of an n = 128 factorization take 7.0 ms mixed and 9.5 ms FP64, 18 ms mixed then.
 // ===========================================================================
 constexpr int kPcMaxW = 832;  // columns of one CTA: 32 rows of them in shared memory
 __device__ __forceinline__ void argmax_step(double& best, int& bi, double ob, int oi) {
@@ -3486,7 +3488,8 @@ void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s) 
 // E(a, l) C(l) over l < a and l > a. A thread holds 4 rows (32 apart) x 4 columns; E goes
 // through shared memory 32 columns at a time, in ascending l, so a row block's running
 // sum is the first until its diagonal block and the second after it. (Reading E from L2
-// at every l, bound by that latency: 3.0 ms a launch over 1344 faces of 224 columns.)
+// at every l, bound by that latency: 3.0 ms a launch over 1344 faces of 224 columns,
+// 2.0 ms now.)
 constexpr int kPqrFc = 32;
 __global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ descs,
                                                     int* __restrict__ flag) {
