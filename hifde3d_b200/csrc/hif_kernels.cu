@@ -3086,6 +3086,7 @@ __global__ void __launch_bounds__(512) k_pchol_panel(const PcholDesc* __restrict
   const double* G = P.G;
   double* R = P.R;
   if (P.info[1]) return;  // the same in every CTA of the face
+  if (C > 1) cl.sync();   // every CTA runs before its shared memory is written from outside
   // own columns tid, tid + nthr: remaining diagonal, -1 once chosen
   constexpr int Q = 2;
   double d[Q];
