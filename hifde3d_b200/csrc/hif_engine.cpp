@@ -62,6 +62,7 @@ namespace {
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
     if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError(); /* reported here: not again by the next launch's check */       \
       throw ::hif::Error{e_ == cudaErrorMemoryAllocation ? HIF_ERR_NOMEM : HIF_ERR_CUDA,          \
                   std::string(#call) + ": " + cudaGetErrorString(e_)};                    \
     }                                                                                     \
@@ -3909,19 +3910,24 @@ class Engine {
     if (!plans_built) build_plans();
     if (contrib_cap < nrhs || !d_contrib) {
       drop_graphs();
-      dfree(d_contrib, stream);
-      d_contrib = dalloc<double>(contrib_ld * nrhs, stream);
+      contrib_cap = 0;
+      replace(d_contrib, contrib_ld * nrhs);
       contrib_cap = nrhs;
     }
     if (ws_nrhs >= nrhs && d_ua) return;
     drop_graphs();
-    dfree(d_ua, stream);
-    dfree(d_ub, stream);
-    dfree(d_uc, stream);
-    d_ua = dalloc<double>(n3 * nrhs, stream);
-    d_ub = dalloc<double>(n3 * nrhs, stream);
-    d_uc = dalloc<double>(n3 * nrhs, stream);
+    ws_nrhs = 0;
+    replace(d_ua, n3 * nrhs);
+    replace(d_ub, n3 * nrhs);
+    replace(d_uc, n3 * nrhs);
     ws_nrhs = nrhs;
+  }
+  // A buffer given back for a larger one. Where the device cannot hold that one, the
+  // handle is left without the buffer, not with the address of the old.
+  void replace(double*& p, long long count) {
+    dfree(p, stream);
+    p = nullptr;
+    p = dalloc<double>(count, stream);
   }
 
   void run_plan(ApplyPlan& plan, int nrhs) {
@@ -3993,8 +3999,8 @@ class Engine {
     if (!factored) throw Error{HIF_ERR_STATE, "solve before Factor"};
     if (nrhs <= 0 || ld < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ld"};
     if (pcg_nrhs < nrhs) {
-      dfree(d_pcg, stream);
-      d_pcg = dalloc<double>(5 * n3 * nrhs + 8 * nrhs + (size_t)kDotBlocks * nrhs, stream);
+      pcg_nrhs = 0;
+      replace(d_pcg, 5 * n3 * nrhs + 8 * nrhs + (long long)kDotBlocks * nrhs);
       pcg_nrhs = nrhs;
     }
     double* r = d_pcg;
