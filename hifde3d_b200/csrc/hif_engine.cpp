@@ -3950,6 +3950,19 @@ class Engine {
     }
   }
 
+  // No apply inside a caller's stream capture: its graph would keep the addresses of
+  // the work vectors, which a later apply with more right-hand sides gives back, and
+  // tables or vectors made meanwhile would exist in that graph only. The legacy default
+  // stream cannot be captured, so the sweeps' own graphs are not made there.
+  void refuse_capture() {
+    if (stream == cudaStreamLegacy && !profile)
+      throw Error{HIF_ERR_CUDA, "no apply on the legacy default stream (it cannot be captured)"};
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    HIF_CK(cudaStreamIsCapturing(stream, &st));
+    if (st != cudaStreamCaptureStatusNone)
+      throw Error{HIF_ERR_CUDA, "no apply inside a stream capture"};
+  }
+
   void apply_device(double* du, int nrhs, long long ldu, bool inverse) {
     apply_device(du, ldu, du, ldu, nrhs, inverse);
   }
@@ -3958,6 +3971,7 @@ class Engine {
                     bool inverse) {
     if (!factored) throw Error{HIF_ERR_STATE, "Apply before Factor"};
     if (nrhs <= 0 || lds < n3 || ldd < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ldu"};
+    refuse_capture();
     ensure_workspace(nrhs);
     ApplyPlan& plan = inverse ? plan_inv : plan_fwd;
     if (nrhs > 1) ensure_multi(plan, stream);
