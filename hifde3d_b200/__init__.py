@@ -32,6 +32,7 @@ PARTITION_REFERENCE, PARTITION_CLIPPED = 0, 1
 OPT_KEEP_SCHUR, OPT_VERBOSE, OPT_MEM_BUDGET_MB, OPT_PROFILE, OPT_ID_GROUP_MIN_N = 1, 2, 3, 4, 5
 OPT_PRECISION, OPT_AUTOTUNE, OPT_SCHUR_SLICES, OPT_X_SLICES = 6, 7, 8, 9
 OPT_ELIMINATION, OPT_Y_SLICES, OPT_GRAM_MIN_N, OPT_GRAM_SLICES, OPT_CHOL_SLICES = 10, 11, 12, 13, 14
+OPT_ID_MAX_PHASES = 15
 PRECISION_FP64, PRECISION_MIXED = 0, 1
 ELIM_AUTO, ELIM_GAUSS_JORDAN, ELIM_CHOLESKY = 0, 1, 2
 KCLASS_NAMES = ["gather", "gemm", "sweep_small", "sweep_panel", "id", "gemv", "copy", "vector",
@@ -80,6 +81,7 @@ _SIGNATURES = {
     "hif_set_option": [_p, _i, _ll],
     "hif_set_replay_pivots": [_p, _i, _i, _ip, _ip],
     "hif_factor_stats": [_p, _dp, _dp, _dp, _dp, _dp, _llp],
+    "hif_id_stats": [_p, _ip, _ip, _ip],
     "hif_kernel_stats": [_p, _i, _llp, _dp, _dp, _dp],
     "hif_autotune_stats": [_p, _ip, _ip, _ip],
     "hif_autotune_elimination": [_p, _ip, _ip, _ip],
@@ -368,6 +370,13 @@ class HIFFactor:
                                           ctypes.byref(fl), ctypes.byref(by)))
             out[name] = {"launches": n.value, "ms": ms.value, "flops": fl.value, "bytes": by.value}
         return out
+
+    def id_stats(self) -> dict:
+        """Decompositions by phases of the last Factor: phases run, faces given to them,
+        and how many of these went column by column after all."""
+        p, n, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        _check(lib().hif_id_stats(self._h, ctypes.byref(p), ctypes.byref(n), ctypes.byref(b)))
+        return {"phases": p.value, "faces": n.value, "column_by_column": b.value}
 
     def autotune_stats(self) -> dict:
         """OPT_AUTOTUNE tuner: batch signatures seen, decided, and how many chose 128 x 128."""

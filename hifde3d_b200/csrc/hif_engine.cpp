@@ -2432,18 +2432,24 @@ class Engine {
       idfl = 0;
     }
     if (!chol_id.empty()) id_cholesky(chol_id, tmp);
-    // by phases, unless the order is prescribed or the grouped QR was asked for:
-    // n = 128 FP64, the three wide levels 758 ms column by column, 218 ms by
+    // by phases, unless the order is prescribed or the column-by-column QR was asked
+    // for: n = 128 FP64, the three wide levels 758 ms column by column, 218 ms by
     // phases; n = 32, 12 faces of 225 columns, 11.0 ms against 2.4 ms
-    if (!wide_id.empty() && (d_ord || group_asked)) {
+    if (!wide_id.empty() && (d_ord || id_max_phases == 0)) {
       id_householder(wide_id, tmp);
-    } else if (!wide_id.empty() && !id_phases(wide_id, tmp)) {
-      // a face the phases do not take: the wide faces are assembled again and all
-      // of them decomposed column by column
-      std::vector<GatherTarget> tw;
-      for (int f : wide_f) tw.push_back(tg[f]);
-      gather(tw, cells, d_own, d_sd, d_dof, tmp);
-      id_householder(wide_id, tmp);
+    } else if (!wide_id.empty()) {
+      const std::vector<int> back = id_phases(wide_id, tmp);
+      if (!back.empty()) {
+        // faces the phases do not take: assembled again, then column by column
+        std::vector<GatherTarget> tw;
+        std::vector<IdDesc> vw;
+        for (int q : back) {
+          tw.push_back(tg[wide_f[q]]);
+          vw.push_back(wide_id[q]);
+        }
+        gather(tw, cells, d_own, d_sd, d_dof, tmp);
+        id_householder(vw, tmp);
+      }
     }
     HIF_CK(cudaGetLastError());
     // pivots, kept flags and |R_ii| read back into pinned staging: the copies
@@ -2733,13 +2739,14 @@ class Engine {
   // Column-pivoted QR of wide tall faces by phases (see PqrDesc). Per phase: the
   // Gram matrices of what is left, pivoted Cholesky panels on them, one read-back of
   // the pivot counts (they set the shapes of the phase's products), then the
-  // products. Returns false, with the faces' M overwritten, when a face is outside
-  // what the scheme holds for: |E| above kPqrMaxE (picked columns far worse
-  // conditioned than their pivots), kept columns that are not a prefix of the
-  // order, or more than kPqrMaxPhases phases (norms spread over hundreds of
-  // decades).
+  // products. Returns the faces (their M overwritten) outside what the scheme holds
+  // for: |E| above kPqrMaxE (picked columns far worse conditioned than their pivots),
+  // kept columns that are not a prefix of the order, or more than id_max_phases phases
+  // (by default norms spread over more than a hundred decades).
   static constexpr int kPqrMaxPhases = 40;
-  bool id_phases(const std::vector<IdDesc>& v, BufList& tmp) {
+  int id_max_phases = kPqrMaxPhases;  // 0: wide faces column by column
+  int id_phase_count = 0, id_wide = 0, id_back = 0;  // of the last factorization
+  std::vector<int> id_phases(const std::vector<IdDesc>& v, BufList& tmp) {
     Arena& work = *cur_work;
     const Arena::Mark mk = work.mark();
     const int nd = (int)v.size();
@@ -2777,23 +2784,26 @@ class Engine {
     int* chosen = work.alloc<int>(isz);
     int* piv = work.alloc<int>(isz);
     int* perm = work.alloc<int>(isz);
-    int* info = work.alloc<int>(2LL * nd + 1);  // steps, done flag per face; *flag last
-    int* flag = info + 2LL * nd;
-    HIF_CK(cudaMemsetAsync(flag, 0, sizeof(int), stream));
+    int* info = work.alloc<int>(3LL * nd);  // steps and done flag of the active faces
+    int* flag = info + 2LL * nd;            // per face: what put it outside the scheme
+    HIF_CK(cudaMemsetAsync(flag, 0, nd * sizeof(int), stream));
     int* h_perm = static_cast<int*>(stage.get(isz * sizeof(int)));
     for (int f = 0; f < nd; ++f)
       for (int j = 0; j < v[f].n; ++j) h_perm[fc[f].i + j] = j;
     HIF_CK(cudaMemcpyAsync(perm, h_perm, isz * sizeof(int), cudaMemcpyHostToDevice, stream));
-    int* h_info = static_cast<int*>(stage.get((2LL * nd + 1) * sizeof(int)));
+    int* h_info = static_cast<int*>(stage.get(3LL * nd * sizeof(int)));
+    const int* h_flag = h_info + 2LL * nd;
+    std::vector<int> back;
     auto tm = [&](int cls, double fl, double by, auto&& f, int n) { timed(cls, fl, by, f, n); };
     std::vector<int> act(nd);
     for (int f = 0; f < nd; ++f) act[f] = f;
-    bool ok = true;
-    for (int phase = 0; !act.empty() && ok; ++phase) {
-      if (phase == kPqrMaxPhases) {
-        ok = false;
+    id_wide += nd;
+    for (int phase = 0; !act.empty(); ++phase) {
+      if (phase == id_max_phases) {
+        back = act;
         break;
       }
+      ++id_phase_count;
       BufList step;
       const int na = (int)act.size();
       std::vector<PcholDesc> pd(na);
@@ -2859,13 +2869,9 @@ class Engine {
         gemm_batch(upd, step, stream, HIF_KCLASS_ID, tm);
       }
       HIF_CK(cudaMemcpyAsync(h_info, info, 2LL * na * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      HIF_CK(cudaMemcpyAsync(h_info + 2LL * nd, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+      HIF_CK(cudaMemcpyAsync(h_info + 2LL * nd, flag, nd * sizeof(int), cudaMemcpyDeviceToHost,
+                             stream));
       sync();
-      if (h_info[2LL * nd]) {
-        ok = false;
-        step.release(stream);
-        break;
-      }
       std::vector<PqrDesc> qd;
       std::vector<GemmDesc> gq, gz, gu;
       std::vector<int> next;
@@ -2874,6 +2880,7 @@ class Engine {
         const IdDesc& d = v[act[q]];
         Face& c = fc[act[q]];
         const int k = h_info[2 * q], w = d.n - c.o;
+        if (h_flag[act[q]]) continue;  // no further phase of it
         if (k == 0) {
           // nothing of the face is left: rows of zeros, the columns in their order
           HIF_CK(cudaMemset2DAsync(Rr + c.g + c.o, d.n * sizeof(double), 0, w * sizeof(double),
@@ -2891,6 +2898,7 @@ class Engine {
         p.perm = perm + c.i;
         p.Rsel = pd[q].R;
         p.piv = pd[q].piv;
+        p.flag = flag + act[q];
         p.m = d.m;
         p.n = d.n;
         p.o = c.o;
@@ -2951,42 +2959,50 @@ class Engine {
         HIF_CK(cudaGetLastError());
         gemm_batch(gq, step, stream, HIF_KCLASS_QR, tm);
         gemm_batch(gz, step, stream, HIF_KCLASS_QR, tm);
-        timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mk_, mc, flag, stream); }, 1);
+        timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mk_, mc, stream); }, 1);
         HIF_CK(cudaGetLastError());
         gemm_batch(gu, step, stream, HIF_KCLASS_QR, tm);
       }
       act.swap(next);
       step.release(stream);
     }
-    if (ok) {
-      std::vector<PqrOut> po(nd);
-      for (int f = 0; f < nd; ++f)
-        po[f] = PqrOut{Rr + fc[f].g, perm + fc[f].i, G + fc[f].g, v[f]};
+    std::vector<int> fin;  // every column picked
+    for (int f = 0; f < nd; ++f)
+      if (fc[f].o == v[f].n) fin.push_back(f);
+    const int nfin = (int)fin.size();
+    int* h_rank = static_cast<int*>(stage.get((nd + 1) * sizeof(int)));
+    if (nfin > 0) {
+      std::vector<PqrOut> po;
+      for (int f : fin) po.push_back(PqrOut{Rr + fc[f].g, perm + fc[f].i, G + fc[f].g, flag + f, v[f]});
       PqrOut* dpo = tmp.add(upload(po, stream));
       timed(HIF_KCLASS_ID, 0, 0, [&] {
-        launch_pqr_finish(dpo, nd, eps, max_n, flag, d_status, stream);
+        launch_pqr_finish(dpo, nfin, eps, max_n, d_status, stream);
       });
       HIF_CK(cudaGetLastError());
       // ranks of consecutive faces lie side by side: one copy per run of them
-      int* h_rank = static_cast<int*>(stage.get((nd + 1) * sizeof(int)));
-      for (int f = 0; f < nd;) {
-        int e = f + 1;
-        while (e < nd && v[e].rank == v[e - 1].rank + 1) ++e;
-        HIF_CK(cudaMemcpyAsync(h_rank + f, v[f].rank, (e - f) * sizeof(int),
+      for (int q = 0; q < nfin;) {
+        int e = q + 1;
+        while (e < nfin && v[fin[e]].rank == v[fin[e - 1]].rank + 1) ++e;
+        HIF_CK(cudaMemcpyAsync(h_rank + q, v[fin[q]].rank, (e - q) * sizeof(int),
                                cudaMemcpyDeviceToHost, stream));
-        f = e;
-      }
-      HIF_CK(cudaMemcpyAsync(h_rank + nd, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
-      sync();
-      ok = h_rank[nd] == 0;
-      if (ok) {
-        std::vector<TriSolve> ts;
-        for (int f = 0; f < nd; ++f) ts.push_back(TriSolve{G + fc[f].g, v[f].W, h_rank[f], v[f].n});
-        solve_w(ts, tmp);
+        q = e;
       }
     }
+    HIF_CK(cudaMemcpyAsync(h_info + 2LL * nd, flag, nd * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    sync();
+    std::vector<TriSolve> ts;
+    for (int q = 0; q < nfin; ++q) {
+      const int f = fin[q];
+      if (!h_flag[f]) ts.push_back(TriSolve{G + fc[f].g, v[f].W, h_rank[q], v[f].n});
+    }
+    solve_w(ts, tmp);
+    for (int f = 0; f < nd; ++f)
+      if (h_flag[f]) back.push_back(f);
+    std::sort(back.begin(), back.end());
+    back.erase(std::unique(back.begin(), back.end()), back.end());
+    id_back += (int)back.size();
     work.rewind(mk);
-    return ok;
+    return back;
   }
 
   // W := R11^{-1} R12 of every face (R11 k x k, ld k; W k x (n - k), ld k): diagonal
@@ -3037,10 +3053,10 @@ class Engine {
   }
 
   // Column-by-column pivoted QR of wide tall faces, for replayed pivot orders, for
-  // faces the phases do not take and where HIF_OPT_ID_GROUP_MIN_N was set: row compression to R0 (n x n), whose pivoted
-  // QR makes the same pivot choices and yields the same R as that of M in exact
-  // arithmetic (both depend on M only through M^T M = R0^T R0); several CTAs per
-  // face for the widest.
+  // faces the phases do not take and where it was asked for: row compression to R0
+  // (n x n), whose pivoted QR makes the same pivot choices and yields the same R as
+  // that of M in exact arithmetic (both depend on M only through M^T M = R0^T R0);
+  // several CTAs per face for the widest.
   void id_householder(std::vector<IdDesc>& v, BufList& tmp) {
     compress_faces(v, tmp);
     mark("skel row compression", -1);
@@ -3098,7 +3114,6 @@ class Engine {
   // of its kQrNB2 reflectors (T from V^T V).
   static constexpr int kCompressMinN = 64;  // wider faces (and m > n) are "wide"
   int kGroupMinN = 512;  // faces this wide get a CTA group (HIF_OPT_ID_GROUP_MIN_N)
-  bool group_asked = false;  // that option was set: wide faces column by column
   void compress_faces(std::vector<IdDesc>& v, BufList& tmp) {
     long long vsz = 0, wsz = 0, rsz = 0;
     int maxn = 0;
@@ -3444,6 +3459,7 @@ class Engine {
                              (elimination == HIF_ELIM_AUTO && precision == HIF_PRECISION_MIXED));
     t_total = t_gather = t_elim = t_id = t_host = 0;
     cur_bytes = peak_bytes = 0;
+    id_phase_count = id_wide = id_back = 0;
     HIF_CK(cudaMemsetAsync(d_status, 0, 4 * sizeof(int), stream));
     const double t0 = wall();
     mark_t = 0;
@@ -4504,7 +4520,11 @@ int hif_set_option(hif_handle h, int option, long long value) {
     case HIF_OPT_ID_GROUP_MIN_N:
       if (value < 2) return HIF_ERR_ARG;
       h->e->kGroupMinN = (int)value;
-      h->e->group_asked = true;
+      h->e->id_max_phases = 0;
+      return HIF_OK;
+    case HIF_OPT_ID_MAX_PHASES:
+      if (value < 0 || value > INT_MAX) return HIF_ERR_ARG;
+      h->e->id_max_phases = (int)value;
       return HIF_OK;
     case HIF_OPT_PROFILE:
       return guarded([&] {
@@ -4542,6 +4562,14 @@ int hif_factor_stats(hif_handle h, double* total_s, double* gather_s, double* el
     *device_bytes = (long long)(e.arena_factor.reserved() + e.arena_work[0].reserved() +
                                 e.arena_work[1].reserved()) +
                     7LL * e.n3 * 8;
+  return HIF_OK;
+}
+
+int hif_id_stats(hif_handle h, int* phases, int* faces, int* back) {
+  if (!h) return HIF_ERR_ARG;
+  if (phases) *phases = h->e->id_phase_count;
+  if (faces) *faces = h->e->id_wide;
+  if (back) *back = h->e->id_back;
   return HIF_OK;
 }
 

@@ -3492,8 +3492,7 @@ void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s) 
 // at every l, bound by that latency: 3.0 ms a launch over 1344 faces of 224 columns,
 // 2.0 ms now.)
 constexpr int kPqrFc = 32;
-__global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ descs,
-                                                    int* __restrict__ flag) {
+__global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ descs) {
   const PqrDesc d = descs[blockIdx.y];
   const int k = d.k, cols = d.n - d.o, c0 = blockIdx.x * kPqrFc, tid = threadIdx.x;
   if (c0 >= cols) return;
@@ -3582,19 +3581,17 @@ __global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ 
       }
     }
   }
-  if (bad) atomicOr(flag, 1);
+  if (bad) atomicOr(d.flag, 1);
 }
 
-void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, int* flag,
-                    cudaStream_t s) {
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, cudaStream_t s) {
   if (nd <= 0) return;
   const int smem = kPqrFc * max_k * (int)sizeof(double);
   ensure_smem((const void*)k_pqr_fix, kPqrFc * kPqrCap * sizeof(double));
-  k_pqr_fix<<<dim3((max_cols + kPqrFc - 1) / kPqrFc, nd), 256, smem, s>>>(d_desc, flag);
+  k_pqr_fix<<<dim3((max_cols + kPqrFc - 1) / kPqrFc, nd), 256, smem, s>>>(d_desc);
 }
 
 __global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ outs, double eps,
-                                                    int* __restrict__ flag,
                                                     int* __restrict__ status) {
   const PqrOut o = outs[blockIdx.x];
   const int n = o.id.n, tid = threadIdx.x, nthr = blockDim.x;
@@ -3621,7 +3618,7 @@ __global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ o
   const int k = s_k;
   if (tid == 0 && blockIdx.y == 0) {
     *o.id.rank = k;
-    if (s_last != k) atomicOr(flag, 2);
+    if (s_last != k) atomicOr(o.flag, 2);
     if (r00 == 0.0) atomicOr(status, kStatusIdZero);
   }
   // R by position: R11 (ld k, upper) and R12, split over the face's CTAs
@@ -3634,12 +3631,12 @@ __global__ void __launch_bounds__(512) k_pqr_finish(const PqrOut* __restrict__ o
   }
 }
 
-void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* flag, int* status,
+void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* status,
                        cudaStream_t s) {
   if (nd <= 0) return;
   const size_t smem = (size_t)max_n * sizeof(int);
   if (smem > 48 * 1024) ensure_smem((const void*)k_pqr_finish, smem);
-  k_pqr_finish<<<dim3(nd, nd < 148 ? 16 : 2), 512, smem, s>>>(d_out, eps, flag, status);
+  k_pqr_finish<<<dim3(nd, nd < 148 ? 16 : 2), 512, smem, s>>>(d_out, eps, status);
 }
 
 // ===========================================================================

@@ -150,24 +150,26 @@ struct PqrDesc {
   int* perm;      // n: column of the face at each position of T
   const double* Rsel;  // the phase's Cholesky rows (row-major, n - o wide)
   const int* piv;      // the phase's pivots as positions relative to o
+  int* flag;           // the face's: see launch_pqr_fix, launch_pqr_finish
   int m, n, o, k;
 };
 // Picked columns to S, the columns they displace into the holes, perm, R1.
 void launch_pqr_extract(const PqrDesc* d_desc, int nd, int max_m, cudaStream_t s);
 void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s);
-// R11 and B into Rr, (I - E) Q1^T T over Z; *flag |= 1 where |E| exceeds kPqrMaxE.
-void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, int* flag,
-                    cudaStream_t s);
+// R11 and B into Rr, (I - E) Q1^T T over Z; the face's *flag |= 1 where |E| exceeds
+// kPqrMaxE.
+void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, cudaStream_t s);
 // After the last phase: jpvt, rdiag, keep, rank; R11 (k x k, ld k) into G and R12
-// into W for the triangular solve. *flag |= 2 where the kept columns are not a
-// prefix of the pivot order.
+// into W for the triangular solve. The face's *flag |= 2 where the kept columns are
+// not a prefix of the pivot order.
 struct PqrOut {
   const double* Rr;
   const int* perm;
   double* R11;
+  int* flag;
   IdDesc id;
 };
-void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* flag, int* status,
+void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* status,
                        cudaStream_t s);
 
 // Source membership of the DOFs (the 6 x NC^3 arrays read by k_gather), built

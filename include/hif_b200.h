@@ -193,9 +193,10 @@ enum hif_option {
   HIF_OPT_PROFILE = 4,       /* time every launch with CUDA events (resets the counters) */
   HIF_OPT_ID_GROUP_MIN_N = 5, /* column-by-column pivoted QR of the faces wider than 64 columns:
                                  faces with at least this many columns get a CTA group (default
-                                 512). Setting it selects that QR for these faces; otherwise
-                                 they are decomposed by phases (the same pivots and R up to
-                                 rounding; R's diagonal is positive there) */
+                                 512). Setting it selects that QR for these faces (as
+                                 HIF_OPT_ID_MAX_PHASES 0); otherwise they are decomposed by
+                                 phases (the same pivots and R up to rounding; R's diagonal
+                                 is positive there) */
   HIF_OPT_PRECISION = 6,      /* HIF_PRECISION_FP64 (default) or HIF_PRECISION_MIXED */
   HIF_OPT_AUTOTUNE = 7,       /* 1: tune online: the tile shape of the batched FP64
                                  products per batch signature, and in mixed precision on
@@ -214,6 +215,10 @@ enum hif_option {
                                  than columns) take the Gram-matrix ID (default 32) */
   HIF_OPT_GRAM_SLICES = 13,   /* MIXED: the Gram matrices M^T M of that ID from int8 slices
                                  (2..8); 0 (default): FP64 products */
+  HIF_OPT_ID_MAX_PHASES = 15, /* phases of a wide face's decomposition (default 40): a face
+                                 that needs more is decomposed column by column, as all are
+                                 with 0. Set after HIF_OPT_ID_GROUP_MIN_N it selects the
+                                 phases again */
   HIF_OPT_CHOL_SLICES = 14    /* MIXED, Cholesky elimination: int8 slices (2..8) of the
                                  products forming L^{-1} (default 7); 0: FP64. The
                                  rank-128 updates of the pivot-block factorization stay
@@ -247,6 +252,12 @@ int hif_set_replay_pivots(hif_handle h, int level, int nfaces, const int* offset
  * elimination, ID, host partition). */
 int hif_factor_stats(hif_handle h, double* total_s, double* gather_s, double* elim_s,
                      double* id_s, double* host_s, long long* device_bytes);
+
+/* The interpolative decompositions by phases of the last hif_factor (faces wider than 64
+ * columns, HIF_OPT_ID_MAX_PHASES): phases run, summed over the levels; faces given to
+ * them; and how many of these were decomposed column by column after all. No reference
+ * counterpart. */
+int hif_id_stats(hif_handle h, int* phases, int* faces, int* back);
 
 /* ---- host-only test hooks of the partitioner (no GPU needed) ---------------------
  * Index data over a caller-given remaining-DOF mask (NC^3 bytes, DOF order).
