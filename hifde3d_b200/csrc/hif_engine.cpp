@@ -344,15 +344,17 @@ struct Arena {
   // skeleton ranks) can end with chunks none of which fits a later request.
   // At a point where nothing on the device uses the arena, consolidate():
   // when it holds several chunks, they are replaced by one of the largest
-  // total the arena was asked for in a cycle since the last consolidation.
-  size_t hw_cycle = 0;
+  // total the arena was asked for in a cycle since the last consolidation, with a
+  // sixteenth to spare that temporaries may take.
+  size_t hw_cycle = 0;  // kept to a cycle's end
+  size_t hw_peak = 0;   // with the temporaries rewound by then
   void consolidate() {
     size_t u = 0;
     for (const Chunk& c : chunks) u += c.used;
     hw_cycle = std::max(hw_cycle, u);
     if (chunks.size() > 1 && hw_cycle > 0) {
       release();
-      const size_t sz = ((hw_cycle + hw_cycle / 16) + 255) & ~size_t(255);
+      const size_t sz = (std::max(hw_cycle + hw_cycle / 16, hw_peak) + 255) & ~size_t(255);
       void* p = nullptr;
       const double t0 = wall();
       if (cudaMalloc(&p, sz) == cudaSuccess) {
@@ -364,7 +366,7 @@ struct Arena {
     }
     for (Chunk& c : chunks) c.used = 0;
     cur = 0;
-    hw_cycle = 0;
+    hw_cycle = hw_peak = 0;
   }
   // Stack discipline for temporaries: everything allocated after mark() is
   // given back by rewind(). Users are on one stream, so memory handed out
@@ -374,9 +376,9 @@ struct Arena {
   };
   Mark mark() const { return Mark{cur, chunks.empty() ? 0 : chunks[cur].used}; }
   void rewind(const Mark& m) {
-    size_t u = 0;  // the temporaries count towards what consolidate() asks for
+    size_t u = 0;
     for (const Chunk& c : chunks) u += c.used;
-    hw_cycle = std::max(hw_cycle, u);
+    hw_peak = std::max(hw_peak, u);
     for (size_t q = m.cur + 1; q < chunks.size(); ++q) chunks[q].used = 0;
     if (!chunks.empty()) chunks[m.cur].used = m.used;
     cur = m.cur;
@@ -2750,20 +2752,28 @@ class Engine {
     Arena& work = *cur_work;
     const Arena::Mark mk = work.mark();
     const int nd = (int)v.size();
+    // A face's buffers: R; a phase's G (at the end R11); the Cholesky rows, then Z over
+    // them; R1 and R1^{-1}. The picked columns S of as many faces as fit lie over the Gs,
+    // which have no reader left by then. That buffer is as large as lets the level's peak
+    // stay where the row compression had it, whose buffers (`was`) the elimination's
+    // blocks come beside: n = 128 FP64 75.8 GB with those, 81.2 GB with every S at once.
     struct Face {
-      long long g = 0, s = 0, z = 0, q = 0, i = 0;  // offsets of its buffers
-      int o = 0;                                     // columns already picked
+      long long g = 0, z = 0, q = 0, i = 0;  // offsets of its buffers
+      int o = 0;                              // columns already picked
     };
     std::vector<Face> fc(nd);
-    long long gsz = 0, ssz = 0, zsz = 0, qsz = 0, isz = 0;
+    long long gsz = 0, zsz = 0, qsz = 0, isz = 0, ssz = 0, smax = 0, parts = 0, was = 0;
     int max_m = 0, max_n = 0;
     for (int f = 0; f < nd; ++f) {
       const IdDesc& d = v[f];
       const long long cap = std::min(kPqrCap, d.n);
       fc[f].g = gsz;
       gsz += (long long)d.n * d.n;
-      fc[f].s = ssz;
       ssz += d.m * cap;
+      smax = std::max(smax, d.m * cap);
+      if (d.m >= 2048)  // the products' partial sums (gemm_batch)
+        parts += std::min(cap, (long long)d.m / 8) * std::min(d.n, d.m / 8) * ((d.m + 1023) / 1024);
+      was += compress_doubles(d.m, d.n) + (long long)d.n * d.n;
       fc[f].z = zsz;
       zsz += cap * d.n;
       fc[f].q = qsz;
@@ -2773,11 +2783,11 @@ class Engine {
       max_m = std::max(max_m, d.m);
       max_n = std::max(max_n, d.n);
     }
-    double* G = work.alloc<double>(gsz);
+    const long long scap =
+        std::max({gsz, smax, std::min(ssz, was - gsz - zsz - 2 * qsz - parts)});
     double* Rr = work.alloc<double>(gsz);
-    double* S = work.alloc<double>(ssz);
+    double* G = work.alloc<double>(scap);
     double* Z = work.alloc<double>(zsz);
-    double* Rsel = work.alloc<double>(zsz);
     double* R1 = work.alloc<double>(qsz);
     double* R1i = work.alloc<double>(qsz);
     double* d0 = work.alloc<double>(nd);
@@ -2816,7 +2826,7 @@ class Engine {
         max_w = std::max(max_w, w);
         PcholDesc& p = pd[q];
         p.G = G + c.g;
-        p.R = Rsel + c.z;
+        p.R = Z + c.z;
         p.chosen = chosen + c.i;
         p.piv = piv + c.i;
         p.info = info + 2 * q;
@@ -2890,7 +2900,6 @@ class Engine {
         }
         PqrDesc p{};
         p.T = d.M;
-        p.S = S + c.s;
         p.R1 = R1 + c.q;
         p.R1inv = R1i + c.q;
         p.Z = Z + c.z;
@@ -2911,7 +2920,6 @@ class Engine {
         GemmDesc a{};  // Q1 = S R1^{-1}, over the picked columns' place in T
         a.C = To;
         a.ldc = d.m;
-        a.A = p.S;
         a.lda = d.m;
         a.B = p.R1inv;
         a.ldb = k;
@@ -2950,14 +2958,31 @@ class Engine {
         c.o += k;
       }
       if (!qd.empty()) {
-        PqrDesc* dq = step.add(upload(qd, stream));
         const int nq = (int)qd.size();
-        timed(HIF_KCLASS_QR, 0, 0, [&] {
-          launch_pqr_extract(dq, nq, mm, stream);
-          launch_pqr_trinv(dq, nq, mk_, stream);
-        }, 2);
-        HIF_CK(cudaGetLastError());
-        gemm_batch(gq, step, stream, HIF_KCLASS_QR, tm);
+        std::vector<int> cut(1, 0);  // faces whose S fit together
+        long long used = 0;
+        for (int q = 0; q < nq; ++q) {
+          const long long sz = (long long)qd[q].m * qd[q].k;
+          if (used + sz > scap) {
+            cut.push_back(q);
+            used = 0;
+          }
+          qd[q].S = G + used;
+          gq[q].A = qd[q].S;
+          used += sz;
+        }
+        cut.push_back(nq);
+        PqrDesc* dq = step.add(upload(qd, stream));
+        for (size_t c = 0; c + 1 < cut.size(); ++c) {
+          const int q0 = cut[c], q1 = cut[c + 1];
+          timed(HIF_KCLASS_QR, 0, 0, [&] {
+            launch_pqr_extract(dq + q0, q1 - q0, mm, stream);
+            launch_pqr_trinv(dq + q0, q1 - q0, mk_, stream);
+          }, 2);
+          HIF_CK(cudaGetLastError());
+          gemm_batch(std::vector<GemmDesc>(gq.begin() + q0, gq.begin() + q1), step, stream,
+                     HIF_KCLASS_QR, tm);
+        }
         gemm_batch(gz, step, stream, HIF_KCLASS_QR, tm);
         timed(HIF_KCLASS_QR, 0, 0, [&] { launch_pqr_fix(dq, nq, mk_, mc, stream); }, 1);
         HIF_CK(cudaGetLastError());
@@ -3114,6 +3139,10 @@ class Engine {
   // of its kQrNB2 reflectors (T from V^T V).
   static constexpr int kCompressMinN = 64;  // wider faces (and m > n) are "wide"
   int kGroupMinN = 512;  // faces this wide get a CTA group (HIF_OPT_ID_GROUP_MIN_N)
+  // doubles that it holds for a face of m x n
+  static long long compress_doubles(int m, int n) {
+    return (long long)kQrNB2 * (m + 2LL * n + 2 * kQrNB2 + 1) + kQrNB * kQrNB + (long long)n * n;
+  }
   void compress_faces(std::vector<IdDesc>& v, BufList& tmp) {
     long long vsz = 0, wsz = 0, rsz = 0;
     int maxn = 0;

@@ -148,7 +148,7 @@ struct PqrDesc {
   double* Z;      // k x (n - o), ld k: [Q1^T Q1 | Q1^T T]; the second part ends as (I - E) Q1^T T
   double* Rr;     // n x n, ld n: R by column of the face
   int* perm;      // n: column of the face at each position of T
-  const double* Rsel;  // the phase's Cholesky rows (row-major, n - o wide)
+  const double* Rsel;  // the phase's Cholesky rows (row-major, n - o wide); may be Z's place
   const int* piv;      // the phase's pivots as positions relative to o
   int* flag;           // the face's: see launch_pqr_fix, launch_pqr_finish
   int m, n, o, k;
