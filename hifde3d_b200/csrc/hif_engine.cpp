@@ -2742,7 +2742,7 @@ class Engine {
   // Gram matrices of what is left, pivoted Cholesky panels on them, one read-back of
   // the pivot counts (they set the shapes of the phase's products), then the
   // products. Returns the faces (their M overwritten) outside what the scheme holds
-  // for: |E| above kPqrMaxE (picked columns far worse conditioned than their pivots),
+  // for: |E| above its limit (picked columns far worse conditioned than their pivots),
   // kept columns that are not a prefix of the order, or more than id_max_phases phases
   // (by default norms spread over more than a hundred decades).
   static constexpr int kPqrMaxPhases = 40;

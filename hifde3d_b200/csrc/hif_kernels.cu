@@ -3506,6 +3506,8 @@ __global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ 
   }
   const int tx = tid & 31, ty = tid >> 5;  // row within 32, group of 4 columns
   const double* E = d.Z;                   // Q1^T Q1 (symmetric), ld k
+  const double r00 = d.o == 0 ? d.R1[0] : d.Rr[(long long)d.perm[0] * d.n];
+  const double lim = fmin(kPqrMaxE * sqrt(fabs(r00) / d.R1[0]), kPqrCapE);
   bool bad = false;
   for (int a0 = 0; a0 < k; a0 += 128) {
     double lo[4][4] = {}, acc[4][4] = {}, ed[4] = {};
@@ -3518,7 +3520,7 @@ __global__ void __launch_bounds__(256, 2) k_pqr_fix(const PqrDesc* __restrict__ 
         const int e = tid + 256 * q, r = e & 127, l = e >> 7, a = a0 + r;
         double v = (l < nl && a < k) ? E[a + (long long)(l0 + l) * k] : 0.0;
         if (l < nl && a == l0 + l) v -= 1.0;
-        bad |= !(fabs(v) <= kPqrMaxE);
+        bad |= !(fabs(v) <= lim);
         Es[l][r] = v;
       }
       __syncthreads();

@@ -139,7 +139,10 @@ void launch_trsm_block(const TrsmBlockDesc* d_desc, int nd, int max_cols, cudaSt
 // downdating of a pivoted QR lets it reach sqrt(u).
 constexpr int kPqrCap = 256;        // pivots of one phase, at most
 constexpr double kPqrDrop = 1e-3;   // end of a phase: remaining norm / first norm
-constexpr double kPqrMaxE = 1e-6;   // largest |E| accepted (E^2 is dropped)
+// Largest |E| accepted in a phase whose first pivot is p: E^2, which is dropped, moves the
+// phase's rows by p E^2, and that stays below u |R_00|, as a Householder QR's error does:
+// kPqrMaxE sqrt(|R_00| / p), at most kPqrCapE.
+constexpr double kPqrMaxE = 1e-8, kPqrCapE = 1e-6;
 struct PqrDesc {
   double* T;      // m x n, ld m; columns o.. are active, o + k.. remain after this phase
   double* S;      // m x kPqrCap, ld m: the picked columns
@@ -157,7 +160,7 @@ struct PqrDesc {
 void launch_pqr_extract(const PqrDesc* d_desc, int nd, int max_m, cudaStream_t s);
 void launch_pqr_trinv(const PqrDesc* d_desc, int nd, int max_k, cudaStream_t s);
 // R11 and B into Rr, (I - E) Q1^T T over Z; the face's *flag |= 1 where |E| exceeds
-// kPqrMaxE.
+// its limit.
 void launch_pqr_fix(const PqrDesc* d_desc, int nd, int max_k, int max_cols, cudaStream_t s);
 // After the last phase: jpvt, rdiag, keep, rank; R11 (k x k, ld k) into G and R12
 // into W for the triangular solve. The face's *flag |= 2 where the kept columns are
