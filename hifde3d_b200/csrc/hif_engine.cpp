@@ -2418,8 +2418,6 @@ class Engine {
         small_n = std::max(small_n, n);
       }
     }
-    double idfl = 0;
-    for (const IdDesc& d : idd) idfl += 4.0 * d.m * d.n * d.n - 4.0 / 3.0 * d.n * d.n * (double)d.n;
     if (!small_id.empty()) {
       IdDesc* d_idd = tmp.add(upload(small_id, stream));
       long long max_mn = 0;
@@ -2428,10 +2426,9 @@ class Engine {
         max_mn = std::max(max_mn, (long long)d.m * d.n);
         max_m = std::max(max_m, d.m);
       }
-      timed(HIF_KCLASS_ID, idfl, 0, [&] {
+      timed(HIF_KCLASS_ID, qr_flops(small_id), 0, [&] {
         launch_id(d_idd, (int)small_id.size(), small_n, eps, d_status, stream, max_mn, max_m);
       });
-      idfl = 0;
     }
     if (!chol_id.empty()) id_cholesky(chol_id, tmp);
     // by phases, unless the order is prescribed or the column-by-column QR was asked
@@ -2756,7 +2753,7 @@ class Engine {
     // them; R1 and R1^{-1}. The picked columns S of as many faces as fit lie over the Gs,
     // which have no reader left by then. That buffer is as large as lets the level's peak
     // stay where the row compression had it, whose buffers (`was`) the elimination's
-    // blocks come beside: n = 128 FP64 75.8 GB with those, 81.2 GB with every S at once.
+    // blocks come beside: n = 128 FP64 74.1 GiB with those, 79.3 GiB with every S at once.
     struct Face {
       long long g = 0, z = 0, q = 0, i = 0;  // offsets of its buffers
       int o = 0;                              // columns already picked
@@ -3082,15 +3079,22 @@ class Engine {
   // (n x n), whose pivoted QR makes the same pivot choices and yields the same R as
   // that of M in exact arithmetic (both depend on M only through M^T M = R0^T R0);
   // several CTAs per face for the widest.
+  static double qr_flops(const std::vector<IdDesc>& v) {
+    double fl = 0;
+    for (const IdDesc& d : v) fl += 4.0 * d.m * d.n * d.n - 4.0 / 3.0 * d.n * d.n * (double)d.n;
+    return fl;
+  }
   void id_householder(std::vector<IdDesc>& v, BufList& tmp) {
     compress_faces(v, tmp);
     mark("skel row compression", -1);
+    double fl[2] = {0, 0};
     std::vector<IdGroupDesc> g1, gbig;
     int g1_m = 0, g1_n = 0, big_m = 0, big_n = 0;
     for (const IdDesc& d : v) {
       IdGroupDesc gd{};
       gd.id = d;
       (d.n >= kGroupMinN ? gbig : g1).push_back(gd);
+      fl[d.n >= kGroupMinN] += qr_flops({d});
       if (d.n >= kGroupMinN) {
         big_m = std::max(big_m, d.m);
         big_n = std::max(big_n, d.n);
@@ -3123,7 +3127,7 @@ class Engine {
       scratch_for(w, grp);
       IdGroupDesc* dg = tmp.add(upload(w, stream));
       cudaError_t le = cudaSuccess;
-      timed(HIF_KCLASS_ID, 0, 0, [&] {
+      timed(HIF_KCLASS_ID, fl[pass], 0, [&] {
         le = launch_id_group(dg, (int)w.size(), grp, eps, d_status, stream,
                              pass == 0 ? g1_m : big_m, pass == 0 ? g1_n : big_n);
       });
