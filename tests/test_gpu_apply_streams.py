@@ -2,7 +2,9 @@
 
 Inside a caller's stream capture every apply is refused, whether the sweep has a graph by
 then or not, and on the legacy default stream, which cannot be captured, from the first
-call on; the handle goes on as before.
+call on; the handle goes on as before. A sweep's graph is made at the 17th use of a count of
+right-hand sides: results stay bit for bit those of the plain launches, after the work
+vectors have grown and after new coefficients too.
 """
 import numpy as np
 import pytest
@@ -44,6 +46,7 @@ def apply(f, u, inverse=True):
     return v
 
 
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
 @pytest.mark.parametrize("nrhs", [1, 3])
 @pytest.mark.parametrize("uses", [0, 1, 20])
 def test_refused_inside_capture(factor, nrhs, uses):
@@ -83,3 +86,25 @@ def test_refused_on_legacy_stream(factor):
         assert e.value.code == hb.HIF_ERR_CUDA
     hb.set_stream(f, 0)
     assert torch.equal(apply(f, vectors(1)), x)
+
+
+@pytest.mark.parametrize("inverse", [True, False])
+@pytest.mark.parametrize("nrhs", [1, 3, 20])
+def test_graph_repeats_plain_launches(factor, nrhs, inverse):
+    f = factor
+    ref = hb.HIFFactor(N, 4, 1e-6)  # applied too seldom to make a graph
+    operator(ref, 3)
+    u = vectors(nrhs)
+    x = apply(ref, u, inverse)
+    for _ in range(20):
+        assert torch.equal(apply(f, u, inverse), x)
+    apply(f, vectors(40), inverse)  # larger work vectors: the graphs are dropped
+    for _ in range(20):
+        assert torch.equal(apply(f, u, inverse), x)
+    operator(f, 4)
+    operator(ref, 4)
+    y = apply(ref, u, inverse)
+    assert not torch.equal(y, x)
+    for _ in range(20):
+        assert torch.equal(apply(f, u, inverse), y)
+    ref.close()
