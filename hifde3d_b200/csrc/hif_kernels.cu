@@ -231,9 +231,9 @@ void launch_gather(const GatherTarget* d_tg, const int* d_tile_off, int ntg, int
                    const SourceDesc* d_src, const int* d_src_owner, const int* d_dof_src,
                    const double* d_band, long long ncell3, int NC, cudaStream_t s) {
   if (total_tiles <= 0) return;
-  // 8 resident CTAs of 256 threads per SM, 148 SMs, several waves' worth of
+  // 8 resident CTAs of 256 threads per SM, several waves' worth of
   // chunks so that uneven tiles even out
-  const int grid = std::min(total_tiles, 148 * 8 * 4);
+  const int grid = std::min(total_tiles, sm_count() * 8 * 4);
   k_gather<<<grid, 256, 0, s>>>(d_tg, d_tile_off, ntg, total_tiles, d_src, d_src_owner,
                                 d_dof_src, d_band, ncell3, NC);
 }
@@ -3638,7 +3638,7 @@ void launch_pqr_finish(const PqrOut* d_out, int nd, double eps, int max_n, int* 
   if (nd <= 0) return;
   const size_t smem = (size_t)max_n * sizeof(int);
   if (smem > 48 * 1024) ensure_smem((const void*)k_pqr_finish, smem);
-  k_pqr_finish<<<dim3(nd, nd < 148 ? 16 : 2), 512, smem, s>>>(d_out, eps, status);
+  k_pqr_finish<<<dim3(nd, nd < sm_count() ? 16 : 2), 512, smem, s>>>(d_out, eps, status);
 }
 
 // ===========================================================================
