@@ -797,8 +797,8 @@ void gemm_batch_int8(const std::vector<GemmDesc>& gin, BufList& tmp, cudaStream_
 
 // Dense elimination of a batch of blocks: descs[b].B holds [A22 A21; A12 A11]
 // (ld n); on return the compact A22^{-1}, X are written and B's trailing block
-// holds A11 - A12 X. Blocks up to kSmallSweepN are eliminated whole in shared
-// memory; larger ones by 64-wide pivot blocks with batched GEMM updates.
+// holds A11 - A12 X. Blocks up to kSmallSweepN are eliminated whole in
+// registers; larger ones by 128-wide pivot blocks with batched GEMM updates.
 // `timed(kernel class, flops, bytes, launch, launches)` wraps every launch.
 // Arithmetic of the products of an elimination. schur: S = A11 - A12 X in FP64
 // (-1), split TF32 (0) or from `schur` int8 slices; x: X = A22^{-1} A21 in FP64
@@ -1596,9 +1596,9 @@ class Engine {
     ws_nrhs = pcg_nrhs = 0;
   }
 
-  // CUDA graphs of the apply sweep (boundary zeroing, output clearing and every
-  // launch of the plan), one per (direction, right-hand-side count); valid
-  // while the plans and the apply workspace stay as they were captured
+  // CUDA graphs of the apply sweep (every launch of the plan; the copies into the work
+  // vectors and out of them stay outside), one per (direction, right-hand-side count);
+  // valid while the plans and the apply workspace stay as they were captured.
   // A graph is made once a pair has been applied kGraphAfter times: making one takes as
   // long as about 15 applies by single launches (n = 16: 0.19 ms, against 30 us of
   // launches), which a factor used for one solve does not give back.

@@ -10,9 +10,11 @@
 //   sweep       in-place Gauss-Jordan elimination of the redundant DOFs of a
 //               block [A22 A21; A12 A11]: yields A22^{-1}, X = A22^{-1} A21 and
 //               A11 - A12 X in one pass (Schur.hpp:72-100);
-//   dgemm       batched FP64 GEMM (rank-64 sweep updates, ID rotations);
-//   id          column-pivoted Householder QR, rank test and interpolation
-//               matrix (InterpDecomp.cpp:86-138);
+//   dgemm       batched FP64 GEMM (rank-128 sweep updates, the QR by phases, ID
+//               rotations);
+//   id          column-pivoted QR (narrow faces Householder, wide ones by phases of
+//               pivoted Cholesky), rank test and interpolation matrix
+//               (InterpDecomp.cpp:86-138);
 //   gemv        gather / multiply / scatter sweeps of Apply (Factor.cpp:992-1081).
 #include "hif_kernels.cuh"
 
@@ -37,8 +39,6 @@ namespace {
 std::mutex g_attr_mu;
 std::map<std::pair<int, const void*>, size_t> g_attr_smem;
 
-// Raises `fn`'s dynamic shared-memory limit on the current device to at least
-// `bytes` (never lowers it).
 // Multiprocessor count of the current device (cached per device).
 int sm_count() {
   int dev = 0;
@@ -54,6 +54,8 @@ int sm_count() {
   return n;
 }
 
+// Raises `fn`'s dynamic shared-memory limit on the current device to at least
+// `bytes` (never lowers it).
 void ensure_smem(const void* fn, size_t bytes) {
   int dev = 0;
   cudaGetDevice(&dev);

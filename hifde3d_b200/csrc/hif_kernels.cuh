@@ -195,7 +195,8 @@ struct GemvDesc {
   long long cslot;      // mode 1: first contribution slot of the block
   int m, n;             // M is m x n
   int trans;            // 0: y = M x (len m), 1: y = M^T x (len n)
-  int tri;              // 1: M is lower triangular (square); entries above the diagonal are not used
+  int tri;              // 1: M is lower triangular (square): what lies above the tiles of its
+                        // diagonal is not read, and the rest above it must be stored as zeros
   double alpha;
   int mode;             // 0: u_out[out] += alpha y; 1: contrib = y; 2: u_out[out] = alpha y
   // Optional per-descriptor vectors (batched solves of several operators in one
@@ -346,7 +347,7 @@ int oz_tile_n(int slices);
 void launch_gemm_oz(const OzGemm* d_desc, const int* d_tile_off, int nd, int total_tiles,
                     int slices, int* d_status, cudaStream_t s);
 
-// In-shared-memory Gauss-Jordan sweep of the first r pivots (n <= kSmallSweepN).
+// Gauss-Jordan sweep of the first r pivots, the block in registers (n <= kSmallSweepN).
 constexpr int kSmallSweepN = 160;
 void launch_sweep_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
                         cudaStream_t s);
@@ -356,7 +357,7 @@ constexpr int kSweepNB = 128;
 void launch_sweep_diag(const SweepDesc* d_desc, const int* d_active, int nact, int k0,
                        double* d_dinv, int* d_status, cudaStream_t s, int sym = 0);
 // Cholesky elimination of symmetric positive definite interiors (lower
-// triangles only). Small blocks whole in shared memory: L, L^{-1}, Y and the
+// triangles only). Small blocks whole in registers: L, L^{-1}, Y and the
 // Schur complement in one launch.
 void launch_chol_small(const SweepDesc* d_desc, int nd, int max_n, int* d_status,
                        cudaStream_t s);

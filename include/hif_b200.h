@@ -85,7 +85,13 @@ int hif_factor(hif_handle h);
 int hif_save_factor(hif_handle h, const char* path);
 int hif_load_factor(hif_handle h, const char* path);
 
-/* HIFFactor::Apply(u, apply_inverse) -- src/Factor.cpp:992-1081, in place. */
+/* HIFFactor::Apply(u, apply_inverse) -- src/Factor.cpp:992-1081, in place. The same call
+ * gives the same bits; a column of a call with several right-hand sides agrees with the
+ * call on that column alone to rounding (below 1e-12 relative), not bit for bit, for the two
+ * sum in different orders, and so may the iterates of hif_solve_pcg and hif_solve_gmres.
+ * The first apply with several right-hand sides, or with more of them than before,
+ * allocates device memory. Not inside a stream capture, nor on the legacy default stream
+ * (HIF_ERR_CUDA). */
 int hif_apply(hif_handle h, double* u, int nrhs, long long ldu, int apply_inverse);
 int hif_apply_device(hif_handle h, double* du, int nrhs, long long ldu, int apply_inverse);
 
@@ -215,14 +221,14 @@ enum hif_option {
                                  than columns) take the Gram-matrix ID (default 32) */
   HIF_OPT_GRAM_SLICES = 13,   /* MIXED: the Gram matrices M^T M of that ID from int8 slices
                                  (2..8); 0 (default): FP64 products */
-  HIF_OPT_ID_MAX_PHASES = 15, /* phases of a wide face's decomposition (default 40): a face
-                                 that needs more is decomposed column by column, as all are
-                                 with 0. Set after HIF_OPT_ID_GROUP_MIN_N it selects the
-                                 phases again */
-  HIF_OPT_CHOL_SLICES = 14    /* MIXED, Cholesky elimination: int8 slices (2..8) of the
+  HIF_OPT_CHOL_SLICES = 14,   /* MIXED, Cholesky elimination: int8 slices (2..8) of the
                                  products forming L^{-1} (default 7); 0: FP64. The
                                  rank-128 updates of the pivot-block factorization stay
                                  FP64 (too short a k for the slices) */
+  HIF_OPT_ID_MAX_PHASES = 15  /* phases of a wide face's decomposition (default 40): a face
+                                 that needs more is decomposed column by column, as all are
+                                 with 0. Set after HIF_OPT_ID_GROUP_MIN_N it selects the
+                                 phases again */
 };
 /* Arithmetic of the factorization. MIXED: the long-K products of the eliminations
  * (S = A11 - A12 X, and X or Y) are FP64 products formed from exact int8 slice
@@ -275,13 +281,14 @@ int hif_partition_face(int N, int P, int level, int ci, int cj, int ck, int face
 enum hif_kernel_class {
   HIF_KCLASS_GATHER = 0,      /* block assembly from the stencil + Schur complement blocks */
   HIF_KCLASS_GEMM = 1,        /* batched FP64 GEMM (elimination updates, ID rotations) */
-  HIF_KCLASS_SWEEP_SMALL = 2, /* whole-block elimination in shared memory */
+  HIF_KCLASS_SWEEP_SMALL = 2, /* whole-block elimination, the block in registers */
   HIF_KCLASS_SWEEP_PANEL = 3, /* pivot-block inverse and panels of the blocked elimination */
   HIF_KCLASS_ID = 4,          /* pivoted-QR interpolative decomposition */
   HIF_KCLASS_GEMV = 5,        /* apply sweeps */
   HIF_KCLASS_COPY = 6,        /* compact copies of factor blocks */
   HIF_KCLASS_VECTOR = 7,      /* reductions / vector updates of the apply */
-  HIF_KCLASS_QR = 8,          /* blocked Householder row compression of face blocks */
+  HIF_KCLASS_QR = 8,          /* wide faces: products of the QR by phases, or the row
+                                 compression of the column-by-column one */
   HIF_KCLASS_GEMM_MIXED = 9,  /* split-TF32 tensor-core Schur-complement updates */
   HIF_KCLASS_GEMM_INT8 = 10,  /* FP64 products from int8 slices on the tensor cores (flops:
                                  the int8 operations of the slice products) */
