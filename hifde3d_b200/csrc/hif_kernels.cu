@@ -890,7 +890,8 @@ __device__ __forceinline__ bool oz_unread(const OzOperand& o, int rt, int kt) {
 // trans = 0, two threads per row (lanes over consecutive rows), 32 k each;
 // trans = 1, a warp per row (lanes over consecutive k), 16 rows per warp. The
 // 32 loads of a thread are issued before the first maximum, which is taken over the
-// high words (an exponent needs no more; rows of subnormals take the exact way).
+// high words (an exponent needs no more). Rows of subnormals take the exact way, and rows
+// that hold a NaN, which is left out of the maximum and has no digits.
 __device__ __forceinline__ int oz_exponent(int hi) {  // m < 2^e, m >= 2^(e - 1)
   return (hi >> 20) - 1022;
 }
@@ -917,7 +918,7 @@ __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ op
     int h = 0;
 #pragma unroll
     for (int e = 0; e < 32; ++e) h = max(h, __double2hiint(v[e]) & 0x7fffffff);
-    if (h >= 0x00100000) {
+    if (h >= 0x00100000 && h < 0x7ff00000) {
       atomicMax(&o.rexp[gi], oz_exponent(h));
     } else {
       double m = 0.0;
@@ -944,7 +945,7 @@ __global__ void __launch_bounds__(256) k_oz_exp(const OzOperand* __restrict__ op
           0xffffffffu, max(__double2hiint(v[2 * j]) & 0x7fffffff,
                            __double2hiint(v[2 * j + 1]) & 0x7fffffff));
       if (gi >= o.rows) continue;
-      if (h >= 0x00100000) {
+      if (h >= 0x00100000 && h < 0x7ff00000) {
         if (lane == 0) atomicMax(&o.rexp[gi], oz_exponent(h));
       } else {
         double m = fmax(fabs(v[2 * j]), fabs(v[2 * j + 1]));
