@@ -3999,17 +3999,14 @@ class Engine {
     }
   }
 
-  // No apply inside a caller's stream capture: its graph would keep the addresses of
-  // the work vectors, which a later apply with more right-hand sides gives back, and
-  // tables or vectors made meanwhile would exist in that graph only. The legacy default
-  // stream cannot be captured, so the sweeps' own graphs are not made there.
+  // No apply and no solve inside a caller's stream capture: its graph would keep the
+  // addresses of the work vectors, which a later call with more right-hand sides gives
+  // back, and tables or vectors made meanwhile would exist in that graph only.
   void refuse_capture() {
-    if (stream == cudaStreamLegacy && !profile)
-      throw Error{HIF_ERR_CUDA, "no apply on the legacy default stream (it cannot be captured)"};
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     HIF_CK(cudaStreamIsCapturing(stream, &st));
     if (st != cudaStreamCaptureStatusNone)
-      throw Error{HIF_ERR_CUDA, "no apply inside a stream capture"};
+      throw Error{HIF_ERR_CUDA, "no apply or solve inside a stream capture"};
   }
 
   void apply_device(double* du, int nrhs, long long ldu, bool inverse) {
@@ -4021,6 +4018,8 @@ class Engine {
     if (!factored) throw Error{HIF_ERR_STATE, "Apply before Factor"};
     if (nrhs <= 0 || lds < n3 || ldd < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ldu"};
     refuse_capture();
+    if (stream == cudaStreamLegacy && !profile)  // the sweeps' own graphs are not made there
+      throw Error{HIF_ERR_CUDA, "no apply on the legacy default stream (it cannot be captured)"};
     ensure_workspace(nrhs);
     ApplyPlan& plan = inverse ? plan_inv : plan_fwd;
     if (nrhs > 1) ensure_multi(plan, stream);
@@ -4061,6 +4060,7 @@ class Engine {
                         int maxit, int* iters, double* relres) {
     if (!factored) throw Error{HIF_ERR_STATE, "solve before Factor"};
     if (nrhs <= 0 || ld < n3) throw Error{HIF_ERR_ARG, "bad nrhs / ld"};
+    refuse_capture();
     if (pcg_nrhs < nrhs) {
       pcg_nrhs = 0;
       replace(d_pcg, 5 * n3 * nrhs + 8 * nrhs + (long long)kDotBlocks * nrhs);

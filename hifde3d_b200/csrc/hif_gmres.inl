@@ -26,6 +26,7 @@ void solve_gmres_device(Engine& e, const double* db, double* dx, int nrhs, long 
   if (nrhs <= 0 || ld < e.n3) throw Error{HIF_ERR_ARG, "bad nrhs / ld"};
   if (restart < 1 || restart > kGmresMaxRestart)
     throw Error{HIF_ERR_ARG, "restart must be in 1.." + std::to_string(kGmresMaxRestart)};
+  e.refuse_capture();
   const long long n = e.n3;
   const int m = restart;
   cudaStream_t s = e.stream;

@@ -1,6 +1,6 @@
 """The apply on streams that it cannot use, and its own CUDA graphs.
 
-Inside a caller's stream capture every apply is refused, whether the sweep has a graph by
+Inside a caller's stream capture every apply and every solve is refused, whether the sweep has a graph by
 then or not, and on the legacy default stream, which cannot be captured, from the first
 call on; the handle goes on as before. A sweep's graph is made at the 17th use of a count of
 right-hand sides: results stay bit for bit those of the plain launches, after the work
@@ -72,6 +72,36 @@ def test_refused_inside_capture(factor, nrhs, uses):
     ref = hb.HIFFactor(N, 4, 1e-6)
     operator(ref, 3)
     assert torch.equal(apply(f, u), apply(ref, u))
+    ref.close()
+
+
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+@pytest.mark.parametrize("solver", ["solve_pcg_device", "solve_gmres_device"])
+def test_solve_refused_inside_capture(factor, solver):
+    f = factor
+    b, x = vectors(2), torch.zeros(2, N3, dtype=torch.float64, device="cuda")
+    s = torch.cuda.Stream()
+    hb.set_stream(f, s.cuda_stream)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode="relaxed")
+        try:
+            with pytest.raises(hb.HIFError) as e:
+                getattr(f, solver)(b.data_ptr(), x.data_ptr(), 2, N3, 1e-10, 50)
+        finally:
+            g.capture_end()
+    assert e.value.code == hb.HIF_ERR_CUDA
+    del g
+    hb.set_stream(f, 0)
+    ref = hb.HIFFactor(N, 4, 1e-6)
+    operator(ref, 3)
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    its = [getattr(q, solver)(b.data_ptr(), v.data_ptr(), 2, N3, 1e-10, 50)[0].tolist()
+           for q, v in ((f, x), (ref, y))]
+    torch.cuda.synchronize()
+    assert its[0] == its[1] and torch.equal(x, y)
     ref.close()
 
 
