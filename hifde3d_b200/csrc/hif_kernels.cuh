@@ -145,7 +145,7 @@ constexpr double kPqrDrop = 1e-3;   // end of a phase: remaining norm / first no
 constexpr double kPqrMaxE = 1e-8, kPqrCapE = 1e-6;
 struct PqrDesc {
   double* T;      // m x n, ld m; columns o.. are active, o + k.. remain after this phase
-  double* S;      // m x kPqrCap, ld m: the picked columns
+  double* S;      // m x k, ld m: the picked columns
   double* R1;     // k x k, ld k, upper
   double* R1inv;  // k x k, ld k, upper
   double* Z;      // k x (n - o), ld k: [Q1^T Q1 | Q1^T T]; the second part ends as (I - E) Q1^T T
